@@ -13,13 +13,14 @@ ROOT = os.path.dirname(PKG_DIR)
 BUILD_DIR = os.path.join(PKG_DIR, "_build")
 LIB_PATH = os.path.join(BUILD_DIR, "libfdtd_b200.so")
 SOURCES = [os.path.join(PKG_DIR, "csrc", f) for f in
-           ("fdtd_b200.cu", "es_net.cu", "fdtd_common.cuh", "fdtd_step.cuh", "fdtd_material.cuh",
-            "fdtd_batch.cuh", "fdtd_internal.h", "fdtd_ffpost.cuh")]
+           ("fdtd_b200.cu", "fdtd_fused.cu", "fdtd_half_f64.cu", "fdtd_half_f32.cu",
+            "fdtd_half_table.cu", "es_net.cu", "fdtd_common.cuh", "fdtd_step.cuh", "fdtd_material.cuh",
+            "fdtd_batch.cuh", "fdtd_internal.h", "fdtd_ffpost.cuh", "fdtd_fused.cuh", "fdtd_half.cuh")]
 CU_SOURCES = [p for p in SOURCES if p.endswith(".cu")]
 HEADER = os.path.join(ROOT, "include", "fdtd_b200.h")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-              "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off", "-shared"]
+              "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off", "-shared", "--threads", "0"]
 
 FDTD_OK, FDTD_ERR, FDTD_ERR_BADARG, FDTD_ERR_OOM, FDTD_ERR_CUDA, FDTD_ERR_NONFINITE, FDTD_ERR_STATE = range(7)
 PREC_F64, PREC_F32, PREC_F32_TABLE = 0, 1, 2

@@ -20,6 +20,8 @@
 #include "fdtd_step.cuh"
 #include "fdtd_batch.cuh"
 #include "fdtd_ffpost.cuh"
+#include "fdtd_fused.cuh"
+#include "fdtd_half.cuh"
 #include "fdtd_internal.h"
 
 #include <map>
@@ -69,6 +71,7 @@ struct HostVProbe {
   int comp, count;
   int* idx;
   double csvf;
+  std::vector<int> cells;   // idx on the host
 };
 
 struct HostIProbe {
@@ -76,6 +79,7 @@ struct HostIProbe {
   int* comp;
   int* idx;
   double* w;
+  std::vector<int> comps, cells;  // comp and idx on the host
 };
 
 }  // namespace
@@ -87,11 +91,31 @@ struct HostIProbe {
 // timed region.  A handful of counts is kept (early-stop runs advance in
 // checkpoints of a few different lengths).
 struct RunGraphs {
-  std::vector<std::pair<int, cudaGraphExec_t>> g;
+  std::vector<std::pair<long long, cudaGraphExec_t>> g;  // key: steps, and a tag of the state it starts from
   void clear() {
     for (auto& e : g) cudaGraphExecDestroy(e.second);
     g.clear();
   }
+};
+
+// The padded state of the one-pass step (fdtd_fused.cuh): allocated at the
+// first run that can use it, dropped when the set-up changes.
+struct FusedState {
+  bool tried = false, ok = false;  // built (or found unusable) for the present set-up
+  bool valid = false;              // holds the current fields and Psi, in copy `cur`
+  int cur = 0;
+  int ts_at = -1;                  // step index in d_ts[cur]
+  void* f[2][6] = {};
+  void* ph[3][2][2] = {};          // H Psi by axis, copy, slot
+  void* pe[3][2] = {};
+  void* prof[2][3][2] = {};
+  unsigned short* cls = nullptr;
+  void* tab = nullptr;             // class table
+  ClassLayout layout = {};         // of the table's rows, and the z slabs
+  int* d_ts = nullptr;
+  int* v_idx[kMaxProbes] = {};
+  int* i_idx[kMaxProbes] = {};
+  std::vector<void*> owned;
 };
 
 struct fdtd_ctx {
@@ -143,6 +167,9 @@ struct fdtd_ctx {
   // launch shape of the step kernels: x planes per thread, thread rows per block
   int ichunk = 1, block_rows = 8, prefetch = 1;
   int block_w = 32;   // threads of a block along k (32: a warp is one row; 16: a warp spans two rows)
+  bool chunk_set = false;   // x planes per thread chosen by the caller
+  FusedState fs;
+  bool dense_valid = true;  // `fields` and the faces' Psi hold the current state
   // graph cache
   RunGraphs graphs;
   bool dirty = true;
@@ -399,19 +426,6 @@ StepParams<T, C> step_params(const fdtd_ctx* c, const C& coef) {
   return p;
 }
 
-// Step kernels for a prefetch depth: 1, 2 = planes prefetched in registers;
-// 3, 4 = planes staged through shared memory (material-table problems only).
-template <typename T, class C, bool EXACT>
-void (*step_kernel(bool electric, int pf))(StepParams<T, C>) {
-  if constexpr (C::kTable) {
-    if (pf == 3) return electric ? k_step_e<T, C, EXACT, 3> : k_step_h<T, C, EXACT, 3>;
-    if (pf == 4) return electric ? k_step_e<T, C, EXACT, 4> : k_step_h<T, C, EXACT, 4>;
-    if (pf == 5) return electric ? k_step_e<T, C, EXACT, 5> : k_step_h<T, C, EXACT, 5>;
-  }
-  if (pf == 2) return electric ? k_step_e<T, C, EXACT, 2> : k_step_h<T, C, EXACT, 2>;
-  return electric ? k_step_e<T, C, EXACT, 1> : k_step_h<T, C, EXACT, 1>;
-}
-
 // Dynamic shared memory of a step launch; raises the kernel's limit when the
 // stages need more than the default 48 KB.
 template <class K>
@@ -437,6 +451,14 @@ int check_block(int w, int rows) {
   return FDTD_OK;
 }
 
+// The launch shape the caller set, whichever path the run takes.
+int check_shape(const fdtd_ctx* c) {
+  int rc = check_block(c->block_w, c->block_rows);
+  if (!rc && c->prefetch == 5 && c->block_w != 32)
+    return fail(FDTD_ERR_BADARG, "prefetch mode 5 (bulk-copied stages) needs 32-wide blocks, got %d", c->block_w);
+  return rc;
+}
+
 // Enqueue `count` steps on stream `st` (default: the handle's stream; with
 // `tm`, one step at a time, timing each kernel).
 template <typename T, class C, bool EXACT>
@@ -446,10 +468,8 @@ int enqueue_steps(fdtd_ctx* c, const C& coef, int count, KernelTimer* tm = nullp
   Probes pr = dev_probes(c);
   FarField ff = dev_ff(c);
   // a thread per (j, k) column walks `ichunk` x planes
-  int rc0 = check_block(c->block_w, c->block_rows);
+  int rc0 = check_shape(c);
   if (rc0) return rc0;
-  if (c->prefetch == 5 && c->block_w != 32)
-    return fail(FDTD_ERR_BADARG, "prefetch mode 5 (bulk-copied stages) needs 32-wide blocks, got %d", c->block_w);
   const dim3 blk(c->block_w, c->block_rows);
   const dim3 grd((c->nz + c->block_w) / c->block_w, (c->ny + c->block_rows) / c->block_rows,
                  (c->nx + 1 + c->ichunk - 1) / c->ichunk);
@@ -545,6 +565,513 @@ int prepare_table(fdtd_ctx* c, TableCoef* out) {
   return FDTD_OK;
 }
 
+// ---------------------------------------------------------------------------
+// One-pass step: state, set-up and launches (fdtd_fused.cuh).
+// ---------------------------------------------------------------------------
+int fused_pitch(const fdtd_ctx* c) {
+  // whole 32-byte sectors per row; eight values, so that a row of 16-bit classes
+  // is whole 16-byte units
+  const int a = 8;
+  return (c->nz + 1 + a - 1) / a * a;
+}
+long long fused_plane(const fdtd_ctx* c) { return (long long)(c->ny + 1) * fused_pitch(c); }
+
+int fused_alloc(fdtd_ctx* c, void** p, size_t bytes) {
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // no room: the caller takes the half-step path
+    *p = nullptr;
+    return FDTD_ERR_OOM;
+  }
+  c->fs.owned.push_back(*p);
+  CK(cudaMemsetAsync(*p, 0, bytes, c->stream));
+  return FDTD_OK;
+}
+
+// Every field and present Psi slot between the dense arrays and copy `cur`.
+template <typename T>
+int fused_copy(fdtd_ctx* c, int to_pad) {
+  FusedState& fs = c->fs;
+  const int nx = c->nx, ny = c->ny, nz = c->nz, P = fused_pitch(c);
+  const long long S = fused_plane(c);
+  for (int q = 0; q < 6; q++) {
+    const int ni = (q == 1 || q == 2 || q == 3) ? nx : nx + 1, nj = (q == 0 || q == 2 || q == 4) ? ny : ny + 1,
+              nk = (q == 0 || q == 1 || q == 5) ? nz : nz + 1;
+    CK(fused_repack<T>((T*)fs.f[fs.cur][q], S, P, (T*)field_ptr(c, q), ni, nj, nk, to_pad, c->stream));
+  }
+  for (int f = 0; f < 6; f++) {
+    const HostFace& h = c->face[f];
+    if (!h.present) continue;
+    for (int s = 0; s < 4; s++) {
+      const int ax = f / 2, el = s >= 2, nb = fs.layout.row.n[ax];
+      const int c0 = ax == 2 ? (f % 2 ? fs.layout.zw[el][0] : 0) + (el ? h.e_start : h.m_start) - fs.layout.z0[el][f % 2]
+                             : (f % 2 ? c->face[2 * ax].nc : 0);
+      T* pad = (T*)(s < 2 ? fs.ph[ax][fs.cur][s] : fs.pe[ax][s - 2]);
+      // extents of the slot's component, the band along the face axis (cpml.js:147-448)
+      const bool first = s == 0 || s == 3;
+      int n[3] = {nx, ny, nz};
+      if (f / 2 == 0) n[first ? 1 : 2]++;
+      if (f / 2 == 1) n[s % 2 == 0 ? 0 : 2]++;
+      if (f / 2 == 2) n[first ? 0 : 1]++;
+      n[f / 2] = h.nc;
+      long long si, sj;
+      if (ax == 0) {
+        si = S;
+        sj = P;
+        pad += c0 * S;
+      } else if (ax == 1) {
+        si = (long long)nb * P;
+        sj = P;
+        pad += (long long)c0 * P;
+      } else {
+        si = (long long)(ny + 1) * nb;
+        sj = nb;
+        pad += c0;
+      }
+      CK(fused_repack<T>(pad, si, sj, (T*)h.psi[s], n[0], n[1], n[2], to_pad, c->stream));
+    }
+  }
+  return FDTD_OK;
+}
+
+int fused_copy_any(fdtd_ctx* c, int to_pad) {
+  return c->esz == 8 ? fused_copy<double>(c, to_pad) : fused_copy<float>(c, to_pad);
+}
+
+// Brings the dense arrays and the half-step path's counter up to date.
+int to_dense(fdtd_ctx* c) {
+  if (c->dense_valid) return FDTD_OK;
+  CK(cudaSetDevice(c->device));
+  int rc = fused_copy_any(c, 0);
+  if (rc) return rc;
+  const int dts = c->ts - 1;
+  CK(xfer(c, c->d_ts, &dts, sizeof(int), cudaMemcpyHostToDevice));
+  c->dense_valid = true;
+  return FDTD_OK;
+}
+
+// The half-step path, or a load, is about to change the dense arrays.
+int claim_dense(fdtd_ctx* c) {
+  int rc = to_dense(c);
+  if (!rc) c->fs.valid = false;
+  return rc;
+}
+
+void fused_free(fdtd_ctx* c) {
+  for (void* p : c->fs.owned) cudaFree(p);
+  c->fs = FusedState();
+}
+
+// Frees the padded state (after saving what it holds): the set-up changes.
+int fused_drop(fdtd_ctx* c) {
+  int rc = to_dense(c);
+  c->graphs.clear();
+  if (c->stream) cudaStreamSynchronize(c->stream);
+  fused_free(c);
+  return rc;
+}
+
+// Layout of a class row for the problem's bands, and the z bands widened to
+// whole groups.  *ok = false: the slabs of the two z faces meet.
+ClassLayout class_layout(const fdtd_ctx* c, bool* ok) {
+  ClassLayout L{};
+  const int V = 8 / (int)c->esz;
+  int nbz = 0;
+  *ok = true;
+  for (int el = 0; el < 2; el++) {
+    for (int side = 0; side < 2; side++) {
+      const HostFace& h = c->face[4 + side];
+      const int st = el ? h.e_start : h.m_start;
+      L.z0[el][side] = st / V * V;
+      L.zw[el][side] = h.nc ? (st + h.nc + V - 1) / V * V - st / V * V : 0;
+    }
+    nbz = std::max(nbz, L.zw[el][0] + L.zw[el][1]);
+    if (L.zw[el][0] && L.zw[el][1] && L.z0[el][0] + L.zw[el][0] > L.z0[el][1] &&
+        L.z0[el][1] + L.zw[el][1] > L.z0[el][0])
+      *ok = false;
+  }
+  int o = kRowBands;
+  for (int a = 0; a < 3; a++) {
+    L.row.o[a] = o;
+    L.row.n[a] = a == 2 ? nbz : c->face[2 * a].nc + c->face[2 * a + 1].nc;
+    o += 4 * L.row.n[a];  // stays a multiple of 4
+  }
+  L.row.stride = o;
+  return L;
+}
+
+constexpr size_t kMaxClassTable = (size_t)256 << 20;  // bytes
+
+template <typename T, class C>
+int fused_classes(fdtd_ctx* c, const C& coef, bool* ok) {
+  FusedState& fs = c->fs;
+  const StepParams<T, C> sp = step_params<T, C>(c, coef);
+  const unsigned n = (unsigned)((c->nx + 1) * fused_plane(c));
+  ClassTable tb{};
+  void* scratch = nullptr;
+  const size_t kb = kClassSlots * sizeof(unsigned long long), ib = kClassSlots * sizeof(unsigned);
+  if (cudaMalloc(&scratch, kb + ib + 16) != cudaSuccess) {
+    cudaGetLastError();
+    return FDTD_OK;  // no room: not usable
+  }
+  tb.key = (unsigned long long*)scratch;
+  tb.id = (unsigned*)((char*)scratch + kb);
+  tb.count = (int*)(tb.id + kClassSlots);
+  int cnt[2] = {0, 0};
+  int rc = FDTD_OK;
+  const ClassLayout& L = fs.layout;
+  cudaError_t e = cudaMemsetAsync(scratch, 0, kb + ib + 16, c->stream);
+  if (e == cudaSuccess) e = fused_class_find<T, C>(sp, fused_pitch(c), n, tb, c->stream);
+  if (e == cudaSuccess) e = xfer(c, cnt, tb.count, sizeof(cnt), cudaMemcpyDeviceToHost);
+  const size_t bytes = (size_t)cnt[0] * L.row.stride * sizeof(T);
+  if (e == cudaSuccess && !cnt[1] && bytes <= kMaxClassTable) {
+    rc = fused_alloc(c, &fs.tab, bytes);
+    if (!rc) {
+      e = fused_class_rows<T, C>(sp, fused_pitch(c), n, tb, L, (T*)fs.tab, fs.cls, c->stream);
+      if (e == cudaSuccess) e = xfer(c, cnt, tb.count, sizeof(cnt), cudaMemcpyDeviceToHost);
+      *ok = e == cudaSuccess && !cnt[1];
+    }
+  }
+  cudaFree(scratch);
+  if (e != cudaSuccess) return fail(FDTD_ERR_CUDA, "cell classes: %s", cudaGetErrorString(e));
+  return rc == FDTD_ERR_OOM ? FDTD_OK : rc;
+}
+
+// Profiles b, a over a whole axis, zero outside the bands.
+template <typename T>
+int fused_profiles(fdtd_ctx* c) {
+  const int n_axis[3] = {c->nx + 1, c->ny + 1, fused_pitch(c)};
+  for (int el = 0; el < 2; el++)
+    for (int a = 0; a < 3; a++)
+      for (int w = 0; w < 2; w++) {
+        std::vector<T> v(n_axis[a] + 8, T(0));
+        for (int side = 0; side < 2; side++) {
+          const HostFace& h = c->face[2 * a + side];
+          if (!h.present) continue;
+          const int st = el ? h.e_start : h.m_start;
+          CK(xfer(c, v.data() + st, h.prof[(el ? 0 : 2) + w], h.nc * sizeof(T), cudaMemcpyDeviceToHost));
+        }
+        int rc = fused_alloc(c, &c->fs.prof[el][a][w], v.size() * sizeof(T));
+        if (rc) return rc;
+        CK(xfer(c, c->fs.prof[el][a][w], v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+      }
+  return FDTD_OK;
+}
+
+// Probe cells in the padded layout.
+int fused_probes(fdtd_ctx* c) {
+  const int P = fused_pitch(c);
+  const long long S = fused_plane(c);
+  auto at = [&](int comp, int idx) {
+    const int nj = (comp == 0 || comp == 2 || comp == 4) ? c->ny : c->ny + 1,
+              nk = (comp == 0 || comp == 1 || comp == 5) ? c->nz : c->nz + 1;
+    return (int)((idx / (nj * nk)) * S + (long long)((idx / nk) % nj) * P + idx % nk);
+  };
+  auto put = [&](int** dst, const std::vector<int>& v) {
+    int rc = fused_alloc(c, (void**)dst, std::max<size_t>(v.size(), 1) * sizeof(int));
+    if (rc) return rc;
+    CK(xfer(c, *dst, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice));
+    return (int)FDTD_OK;
+  };
+  for (size_t q = 0; q < c->vprobe.size(); q++) {
+    std::vector<int> v;
+    for (int x : c->vprobe[q].cells) v.push_back(at(3 + c->vprobe[q].comp, x));
+    int rc = put(&c->fs.v_idx[q], v);
+    if (rc) return rc;
+  }
+  for (size_t q = 0; q < c->iprobe.size(); q++) {
+    std::vector<int> v;
+    for (size_t m = 0; m < c->iprobe[q].cells.size(); m++) v.push_back(at(c->iprobe[q].comps[m], c->iprobe[q].cells[m]));
+    int rc = put(&c->fs.i_idx[q], v);
+    if (rc) return rc;
+  }
+  return FDTD_OK;
+}
+
+// Builds the padded state.  It serves problems whose CPML bands are disjoint
+// per axis (along z as whole groups), whose padded arrays have 32-bit indices,
+// with at most 65,536 cell classes, and whose padded state takes at most half
+// of the device memory that is free; others keep the half-step path.
+int fused_build(fdtd_ctx* c) {
+  FusedState& fs = c->fs;
+  const int P = fused_pitch(c);
+  const long long S = fused_plane(c);
+  const long long elems = (long long)(c->nx + 1) * S;
+  if (!bands_disjoint(c) || elems + 2 * S > (1LL << 31) - 1) return FDTD_OK;
+  bool slabs = false;
+  fs.layout = class_layout(c, &slabs);
+  if (!slabs) return FDTD_OK;
+  const size_t comp = (size_t)elems * c->esz;
+  long long psi[3] = {};
+  size_t need = 12 * comp + (size_t)elems * 2;
+  for (int a = 0; a < 3; a++) {
+    const int nb = fs.layout.row.n[a];
+    psi[a] = nb * (a == 0 ? S : (long long)(c->nx + 1) * (a == 1 ? P : c->ny + 1));
+    if (psi[a] > (1LL << 31) - 1) return FDTD_OK;
+    need += 6 * (size_t)psi[a] * c->esz;
+  }
+  size_t free_b = 0, total_b = 0;
+  CK(cudaMemGetInfo(&free_b, &total_b));
+  if (need > free_b / 2) return FDTD_OK;
+  int rc = FDTD_OK;
+  for (int w = 0; w < 2 && !rc; w++)
+    for (int q = 0; q < 6 && !rc; q++) rc = fused_alloc(c, &fs.f[w][q], comp);
+  for (int a = 0; a < 3 && !rc; a++)
+    if (psi[a])
+      for (int s = 0; s < 2 && !rc; s++) {
+        for (int w = 0; w < 2 && !rc; w++) rc = fused_alloc(c, &fs.ph[a][w][s], (size_t)psi[a] * c->esz);
+        if (!rc) rc = fused_alloc(c, &fs.pe[a][s], (size_t)psi[a] * c->esz);
+      }
+  if (!rc) rc = fused_alloc(c, (void**)&fs.cls, (size_t)elems * 2);
+  if (!rc) rc = fused_alloc(c, (void**)&fs.d_ts, 2 * sizeof(int));
+  if (!rc) rc = c->esz == 8 ? fused_profiles<double>(c) : fused_profiles<float>(c);
+  if (!rc) rc = fused_probes(c);
+  bool ok = false;
+  if (!rc) {
+    if (c->prec == FDTD_PREC_F64)
+      rc = fused_classes<double, ArrayCoef<double>>(c, array_coef<double>(c), &ok);
+    else if (c->prec == FDTD_PREC_F32)
+      rc = fused_classes<float, ArrayCoef<float>>(c, array_coef<float>(c), &ok);
+    else
+      rc = fused_classes<float, TableCoef>(c, c->tcoef, &ok);
+  }
+  if (rc == FDTD_ERR_OOM) rc = FDTD_OK;  // no room after all
+  fs.ok = !rc && ok;
+  return rc;
+}
+
+// Makes the padded state hold the current step; *use = false: half-step path.
+int fused_ready(fdtd_ctx* c, bool* use) {
+  FusedState& fs = c->fs;
+  *use = false;
+  if (!fs.tried) {
+    int rc = fused_build(c);
+    if (rc || !fs.ok) {
+      fused_free(c);
+      fs.tried = rc == FDTD_OK;
+      if (rc) return rc;
+    } else {
+      fs.tried = true;
+    }
+  }
+  if (!fs.ok) return FDTD_OK;
+  if (!fs.valid) {
+    int rc = fused_copy_any(c, 1);
+    if (rc) return rc;
+    fs.valid = true;
+    fs.ts_at = -1;
+  }
+  if (fs.ts_at != c->ts) {
+    CK(xfer(c, fs.d_ts + fs.cur, &c->ts, sizeof(int), cudaMemcpyHostToDevice));
+    fs.ts_at = c->ts;
+  }
+  *use = true;
+  return FDTD_OK;
+}
+
+// cuTensorMapEncodeTiled, through the runtime (the library does not link the driver).
+using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled encode_tiled() {
+  static const EncodeTiled fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess) p = nullptr;
+    return (EncodeTiled)p;
+  }();
+  return fn;
+}
+
+// Tensor map of one padded array: (w, rows, 1) tiles of (k, j, i).
+template <typename T>
+bool fused_map(const fdtd_ctx* c, CUtensorMap* m, const T* base, int w, int rows) {
+  const cuuint64_t dim[3] = {(cuuint64_t)fused_pitch(c), (cuuint64_t)c->ny + 1, (cuuint64_t)c->nx + 1};
+  const cuuint64_t stride[2] = {dim[0] * sizeof(T), (cuuint64_t)fused_plane(c) * sizeof(T)};
+  const CUtensorMapDataType type = sizeof(T) == 8   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
+                                   : sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                                    : CU_TENSOR_MAP_DATA_TYPE_UINT16;
+  const cuuint32_t box[3] = {(cuuint32_t)w, (cuuint32_t)rows, 1}, one[3] = {1, 1, 1};
+  const EncodeTiled enc = encode_tiled();
+  return enc && enc(m, type, 3,
+                    (void*)base, dim, stride, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Tiles: a row as few k tiles of equal width as hold it, then the number of x
+// chunks (one tile of each per block): a chunk recomputes one H plane, sets up
+// and fills its pipeline, about kFusedFill planes' time, and a plane with Psi
+// takes about 1 + kFusedBand times that of one without (512 x 512 x 640,
+// material table, 8-cell CPML: 2.3 ms of 2.97 without the z bands' Psi, 2.6
+// without the y bands', 1.7 without any).
+constexpr double kFusedFill = 5, kFusedBand = 0.6;
+template <typename T>
+void fused_shape(const fdtd_ctx* c, FusedParams<T>& p) {
+  const int cols = c->nz + 1;
+  // owned columns: all of them, or a multiple of four (a tile starts on 16
+  // bytes) with room for the halo group
+  constexpr int V = FusedShape<T>::V;
+  p.halo_k = cols > kTileCols;
+  p.tk = p.halo_k ? (cols + kTileCols - 5) / (kTileCols - 4) : 1;
+  p.rk = (p.halo_k ? ((cols + p.tk - 1) / p.tk + 3) / 4 * 4 : (cols + V - 1) / V * V) / V + p.halo_k;
+  p.tj = (c->ny + kTileRows - 1) / (kTileRows - 1);
+  // tiles that meet a band, from the low and from the high end
+  auto slow = [](const FusedAxis<T>& x, int width, int n, int* out) {
+    int lo = 0, hi = n;
+    for (int e = 0; e < 2; e++) {
+      if (x.nc[e][0] > 0) lo = std::max(lo, (x.start[e][0] + x.nc[e][0] - 1) / width + 1);
+      if (x.nc[e][1] > 0) hi = std::min(hi, x.start[e][1] / width);
+    }
+    out[0] = std::min(lo, n);
+    out[1] = n - std::max(std::min(hi, n), out[0]);
+  };
+  slow(p.axis[1], kTileRows - 1, p.tj, p.slow_j);
+  slow(p.axis[2], (p.rk - p.halo_k) * V, p.tk, p.slow_k);
+  const int nxp = c->nx + 1;
+  if (c->chunk_set) {
+    p.tx = (nxp + c->ichunk - 1) / c->ichunk;
+    return;
+  }
+  // Blocks of the three kinds that fused_place orders, per x chunk, and their
+  // time per plane: the device takes them in that order, a free slot the next.
+  const int nj = p.slow_j[0] + p.slow_j[1], nk = p.slow_k[0] + p.slow_k[1];
+  const int kind[3] = {nj * p.tk, (p.tj - nj) * nk, (p.tj - nj) * (p.tk - nk)};
+  int xb[2] = {0, 0};  // planes in the x bands
+  for (int f = 0; f < 2; f++) xb[f] = std::max(p.axis[0].nc[0][f], p.axis[0].nc[1][f]);
+  double t_best = -1;
+  const int slots = 148 * FusedShape<T>::kBlocks, n_max = std::min(nxp, 64 + 4 * slots / (p.tk * p.tj));
+  for (int n = 1; n <= n_max; n++) {
+    std::map<double, int> free_at;  // time -> slots
+    free_at[0] = slots;
+    double end = 0;
+    const double planes = (nxp + n - 1) / n;
+    for (int q = 0; q < 3; q++)
+      for (int z = 0; z < 2; z++) {  // the chunks at the ends, the others
+        long long blocks = (long long)kind[q] * (z ? std::max(0, n - 2) : std::min(n, 2));
+        const double band = z ? 0 : std::min(planes, (double)std::max(xb[0], xb[1]) * (n == 1 ? 2 : 1));
+        const double t = (planes + kFusedFill + kFusedBand * band) * (q < 2 ? 1 + kFusedBand : 1.0);
+        while (blocks > 0) {
+          const auto it = free_at.begin();
+          const double at = it->first + t;
+          const int m = (int)std::min<long long>(blocks, it->second);
+          if (m == it->second) free_at.erase(it); else it->second -= m;
+          free_at[at] += m;
+          end = std::max(end, at);
+          blocks -= m;
+        }
+      }
+    if (t_best < 0 || end < t_best) {
+      t_best = end;
+      p.tx = n;
+    }
+  }
+}
+
+template <typename T>
+FusedParams<T> fused_params(const fdtd_ctx* c, int flip) {
+  const FusedState& fs = c->fs;
+  FusedParams<T> p{};
+  p.nx = c->nx; p.ny = c->ny; p.nz = c->nz;
+  p.pitch = fused_pitch(c);
+  p.plane = (unsigned)fused_plane(c);
+  for (int q = 0; q < 6; q++) {
+    p.fi[q] = (const T*)fs.f[flip][q];
+    p.fo[q] = (T*)fs.f[flip ^ 1][q];
+  }
+  p.cls = fs.cls;
+  p.tab = (const T*)fs.tab;
+  p.row = fs.layout.row;
+  for (int a = 0; a < 3; a++) {
+    FusedAxis<T>& x = p.axis[a];
+    for (int el = 0; el < 2; el++)
+      for (int f = 0; f < 2; f++) {
+        const HostFace& h = c->face[2 * a + f];
+        x.nc[el][f] = a == 2 ? fs.layout.zw[el][f] : h.nc;
+        x.start[el][f] = a == 2 ? fs.layout.z0[el][f] : el ? h.e_start : h.m_start;
+      }
+    x.nb = fs.layout.row.n[a];
+    for (int s = 0; s < 2; s++) {
+      x.phi[s] = (const T*)fs.ph[a][flip][s];
+      x.pho[s] = (T*)fs.ph[a][flip ^ 1][s];
+      x.pe[s] = (T*)fs.pe[a][s];
+      for (int w = 0; w < 2; w++) x.prof[s][w] = (const T*)fs.prof[s][a][w];
+    }
+  }
+  p.ts = fs.d_ts + flip;
+  p.ts_next = fs.d_ts + (flip ^ 1);
+  p.src = dev_sources<T>(c);
+  p.x_wall = c->x_wall;
+  p.fault = c->d_status;
+  fused_shape(c, p);
+  for (int q = 0; q < 6; q++) {
+    if (!fused_map(c, &p.map[q], p.fi[q], kTileW, q < 3 ? kTileRows : kTileRows + 1)) p.tx = 0;  // no maps: no launch
+  }
+  if (!fused_map(c, &p.map[6], p.cls, kTileC, kTileRows)) p.tx = 0;
+  return p;
+}
+
+Probes fused_dev_probes(const fdtd_ctx* c) {
+  Probes p = dev_probes(c);
+  for (int q = 0; q < p.n_v; q++) p.v_idx[q] = c->fs.v_idx[q];
+  for (int q = 0; q < p.n_i; q++) p.i_idx[q] = c->fs.i_idx[q];
+  return p;
+}
+
+long long surface_points(const fdtd_ctx* c) { return c->nFreq > 0 ? c->ffsz[0] + c->ffsz[1] + c->ffsz[2] : 0; }
+
+// `count` steps from copy `flip` and step `ts` on the handle's stream.  A step's
+// epilogue is queued after the next step's launch, and runs beside it; the last
+// one's after its own.
+template <typename T, bool EXACT>
+int fused_enqueue_steps(fdtd_ctx* c, int count, int flip, int ts, KernelTimer* tm) {
+  const FusedParams<T> pf[2] = {fused_params<T>(c, 0), fused_params<T>(c, 1)};  // by the copy read
+  if (pf[0].tx == 0 || pf[1].tx == 0) return fail(FDTD_ERR_CUDA, "cannot encode the step's tensor maps");
+  const Probes pr = fused_dev_probes(c);
+  const FarField ff = dev_ff(c);
+  cudaStream_t st = c->stream;
+  const int probes = pr.n_v + pr.n_i;
+  const long long pts = surface_points(c);
+  const unsigned epi = pts + probes ? (unsigned)((epilogue_threads(pts, probes) + 255) / 256) : 0;
+  // the epilogue of step `step`, under the parameters of the step after it or its own
+  auto epilogue = [&](const FusedParams<T>& p, int step, bool late) -> cudaError_t {
+    if (!epi) return cudaSuccess;
+    const cudaError_t e = fused_epilogue<T>(p, ff, pr, epi, late, st);
+    if (e == cudaSuccess && c->dft_block > 0 && (step + 1) % c->dft_block == 0)
+      k_dft_flush<<<(unsigned)((pts * c->nFreq + 255) / 256), 256, 0, st>>>(ff, late ? p.ts : p.ts_next, -2);
+    return e;
+  };
+  for (int s = 0; s < count; s++, flip ^= 1) {
+    const FusedParams<T>& p = pf[flip];
+    if (tm) CK(cudaEventRecord(tm->ev[0], st));
+    CK((fused_step<T, EXACT>(p, st)));
+    if (tm) CK(cudaEventRecord(tm->ev[1], st));
+    if (!p.x_wall) CK((fused_wall<T, EXACT>(p, st)));
+    if (tm) {
+      CK(cudaEventRecord(tm->ev[2], st));
+      CK(cudaEventRecord(tm->ev[3], st));
+    }
+    if (!tm && s > 0) CK(epilogue(p, ts + s - 1, true));
+    if (tm || s + 1 == count) CK(epilogue(p, ts + s, false));
+    if (tm) {
+      CK(cudaEventRecord(tm->ev[4], st));
+      CK(cudaEventSynchronize(tm->ev[4]));
+      for (int q = 0; q < 4; q++) {
+        float ms = 0;
+        CK(cudaEventElapsedTime(&ms, tm->ev[q], tm->ev[q + 1]));
+        tm->ms[q] += ms;
+      }
+    }
+  }
+  CK(cudaGetLastError());
+  return FDTD_OK;
+}
+
+int fused_enqueue(fdtd_ctx* c, int count, int ts, KernelTimer* tm = nullptr) {
+  if (c->prec == FDTD_PREC_F64) return fused_enqueue_steps<double, true>(c, count, c->fs.cur, ts, tm);
+  if (c->prec == FDTD_PREC_F32) return fused_enqueue_steps<float, true>(c, count, c->fs.cur, ts, tm);
+  return fused_enqueue_steps<float, false>(c, count, c->fs.cur, ts, tm);
+}
+
 int enqueue(fdtd_ctx* c, int count, KernelTimer* tm = nullptr, cudaStream_t st = nullptr) {
   if (c->prec == FDTD_PREC_F64)
     return enqueue_steps<double, ArrayCoef<double>, true>(c, array_coef<double>(c), count, tm, st);
@@ -574,9 +1101,10 @@ constexpr size_t kMaxCachedGraphs = 6;
 // The graph of `steps` steps from the cache, captured on `st` through `enq`
 // (which enqueues that many steps) when missing.
 template <class Enq>
-int graph_for(RunGraphs& rg, cudaStream_t st, int steps, Enq enq, cudaGraphExec_t* out) {
+int graph_for(RunGraphs& rg, cudaStream_t st, int steps, int tag, Enq enq, cudaGraphExec_t* out) {
+  const long long key = (long long)steps << 16 | tag;
   for (auto& e : rg.g)
-    if (e.first == steps) {
+    if (e.first == key) {
       *out = e.second;
       return FDTD_OK;
     }
@@ -594,26 +1122,29 @@ int graph_for(RunGraphs& rg, cudaStream_t st, int steps, Enq enq, cudaGraphExec_
   ce = cudaGraphInstantiate(&ge, g, 0);
   cudaGraphDestroy(g);
   if (ce != cudaSuccess) return fail(FDTD_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(ce));
-  rg.g.push_back({steps, ge});
+  rg.g.push_back({key, ge});
   *out = ge;
   return FDTD_OK;
 }
 
 // The graph launches of a run of `count` steps: full graphs of `cap` steps
-// and one of the remainder, each captured (if missing) now.
+// and one of the remainder, each captured (if missing) now.  `period` and
+// `tag`: what a graph's steps depend on beyond their number repeats every
+// `period` steps, and `tag` is where in it the run starts.
 template <class Enq>
 int run_plan(RunGraphs& rg, cudaStream_t st, int count, int launches_per_step, Enq enq,
-             std::vector<cudaGraphExec_t>* plan) {
-  const int cap = std::max(kGraphSteps, kMaxGraphNodes / std::max(1, launches_per_step));
+             std::vector<cudaGraphExec_t>* plan, int period = 1, int tag = 0) {
+  int cap = std::max(kGraphSteps, kMaxGraphNodes / std::max(1, launches_per_step));
+  cap = std::max(cap / period, 1) * period;
   plan->clear();
   if (count <= 0) return FDTD_OK;
   cudaGraphExec_t full = nullptr, rest = nullptr;
   if (count >= cap) {
-    int rc = graph_for(rg, st, cap, enq, &full);
+    int rc = graph_for(rg, st, cap, tag, enq, &full);
     if (rc) return rc;
   }
   if (count % cap) {
-    int rc = graph_for(rg, st, count % cap, enq, &rest);
+    int rc = graph_for(rg, st, count % cap, tag, enq, &rest);
     if (rc) return rc;
   }
   for (int q = 0; q < count / cap; q++) plan->push_back(full);
@@ -637,13 +1168,29 @@ int run_steps(fdtd_ctx* c, int count, float* elapsed_ms = nullptr, KernelTimer* 
     rc = prepare_table(c, &c->tcoef);
     if (rc) return rc;
   }
+  if (count > 0) {
+    rc = check_shape(c);
+    if (rc) return rc;
+  }
+  bool fused = false;
+  if (count > 0) {
+    rc = fused_ready(c, &fused);
+    if (!rc && !fused) rc = claim_dense(c);
+    if (rc) return rc;
+  }
   // the whole run as cached graphs, captured before the first launch
   if (c->dirty) {
     c->graphs.clear();
     c->dirty = false;
   }
   std::vector<cudaGraphExec_t> plan;
-  if (!tm) {
+  if (!tm && fused) {
+    // a graph depends on the copy it starts from and on where DFT blocks close
+    const int per = c->dft_block > 0 ? c->dft_block : 1;
+    rc = run_plan(c->graphs, c->stream, count, 3, [c](int n) { return fused_enqueue(c, n, c->ts); }, &plan, 2 * per,
+                  2 * (c->ts % per) + c->fs.cur);
+    if (rc) return rc;
+  } else if (!tm) {
     rc = run_plan(c->graphs, c->stream, count, c->dft_block > 0 ? 5 : 4,
                   [c](int n) { return enqueue(c, n); }, &plan);
     if (rc) return rc;
@@ -654,11 +1201,20 @@ int run_steps(fdtd_ctx* c, int count, float* elapsed_ms = nullptr, KernelTimer* 
     CK(cudaEventCreate(&ev1));
     CK(cudaEventRecord(ev0, c->stream));
   }
+  if (fused) {
+    // from here the padded state runs ahead of the dense one
+    c->dense_valid = false;
+    c->fs.valid = true;
+  }
   if (tm) {
-    rc = enqueue(c, count, tm);
+    rc = fused ? fused_enqueue(c, count, c->ts, tm) : enqueue(c, count, tm);
     if (rc) return rc;
   }
   for (cudaGraphExec_t ge : plan) CK(cudaGraphLaunch(ge, c->stream));
+  if (fused) {
+    c->fs.cur ^= count & 1;
+    c->fs.ts_at = c->ts + count;
+  }
   if (elapsed_ms) {
     CK(cudaEventRecord(ev1, c->stream));
     CK(cudaEventSynchronize(ev1));
@@ -831,6 +1387,7 @@ void fdtd_free(fdtd_ctx* c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   c->graphs.clear();
+  fused_free(c);
   for (void* p : c->owned) cudaFree(p);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
@@ -844,7 +1401,8 @@ int fdtd_ctx_upload_coeff(fdtd_ctx* c, int which, const double* host, long n) {
   digest_vals(c, 2, {(double)which});
   digest(c, 2, host, (size_t)n * sizeof(double));
   CK(cudaSetDevice(c->device));
-  int rc = upload_real(c, c->coef[which], host, n);
+  int rc = fused_drop(c);
+  if (!rc) rc = upload_real(c, c->coef[which], host, n);
   if (!rc) c->coef_set[which] = true;
   c->coef_device = false;  // host arrays carry their own kappa division and come with CPsi
   return rc;
@@ -925,6 +1483,7 @@ int fdtd_ctx_upload_cpml(fdtd_ctx* c, int f, int nc, const double* b_e, const do
       return fail(FDTD_ERR_BADARG, "face %d slot %d: got %ld CPsi values, expected %lld", f, s, got[s], want[s]);
   }
   CK(cudaSetDevice(c->device));
+  if (int rc0 = fused_drop(c)) return rc0;
   HostFace& h = c->face[f];
   for (int s = 0; s < 4; s++) { dfree(c, h.prof[s]); dfree(c, h.psi[s]); dfree(c, h.cpsi[s]); }
   dfree(c, h.inv_k[0]); dfree(c, h.inv_k[1]);
@@ -998,6 +1557,7 @@ int fdtd_ctx_add_vsource(fdtd_ctx* c, int dir, const int* idx, const double* coe
   for (int q2 = 0; q2 < count; q2++)
     if (!std::isfinite(coef[q2])) return fail(FDTD_ERR_BADARG, "non-finite source coefficient");
   CK(cudaSetDevice(c->device));
+  if (int rc0 = fused_drop(c)) return rc0;
   HostSource s;
   s.box = SourceBox{dir, bi0, bi1, bj0, bj1, bk0, bk1};
   s.count = count;
@@ -1022,7 +1582,8 @@ int fdtd_ctx_add_svoltage(fdtd_ctx* c, int dir, const int* idx, int count, doubl
   digest_vals(c, 5, {(double)dir, (double)count, Csvf});
   digest(c, 5, idx, (size_t)count * sizeof(int));
   CK(cudaSetDevice(c->device));
-  HostVProbe p{dir, count, nullptr, Csvf};
+  if (int rc0 = fused_drop(c)) return rc0;
+  HostVProbe p{dir, count, nullptr, Csvf, std::vector<int>(idx, idx + count)};
   int rc = dalloc(c, (void**)&p.idx, count * sizeof(int));
   if (rc) return rc;
   CK(xfer(c, p.idx, idx, count * sizeof(int), cudaMemcpyHostToDevice));
@@ -1044,7 +1605,9 @@ int fdtd_ctx_add_scurrent(fdtd_ctx* c, const int* comp, const int* idx, const do
   digest(c, 6, idx, (size_t)count * sizeof(int));
   digest(c, 6, w, (size_t)count * sizeof(double));
   CK(cudaSetDevice(c->device));
-  HostIProbe p{count, nullptr, nullptr, nullptr};
+  if (int rc0 = fused_drop(c)) return rc0;
+  HostIProbe p{count, nullptr, nullptr, nullptr, std::vector<int>(comp, comp + count),
+               std::vector<int>(idx, idx + count)};
   int rc = dalloc(c, (void**)&p.comp, count * sizeof(int));
   if (!rc) rc = dalloc(c, (void**)&p.idx, count * sizeof(int));
   if (!rc) rc = dalloc(c, (void**)&p.w, count * sizeof(double));
@@ -1116,6 +1679,7 @@ int fdtd_ctx_upload_material(fdtd_ctx* c, int comp, const unsigned char* ids, lo
   digest(c, 8, ids, (size_t)n);
   digest(c, 8, table, (size_t)rows * 3 * sizeof(double));
   CK(cudaSetDevice(c->device));
+  if (int rc0 = fused_drop(c)) return rc0;
   CK(xfer(c, c->ids[comp], ids, n, cudaMemcpyHostToDevice));
   int rc = set_rows(c, comp, std::vector<double>(table, table + 3 * rows));
   if (rc) return rc;
@@ -1189,6 +1753,7 @@ int fdtd_ctx_build_material(fdtd_ctx* c, const unsigned char* mat, long ncells, 
     b.plate[q] = PlateBox{P[0], P[1], P[2], P[3], P[4], P[5], P[6], sid};
   }
   CK(cudaSetDevice(c->device));
+  if (int rc0 = fused_drop(c)) return rc0;
   unsigned char* d_mat = nullptr;
   uint8_t *d_present = nullptr, *d_map = nullptr;
   int* d_map64 = nullptr;     // FP64: code -> row
@@ -1311,6 +1876,7 @@ static int override_coef64(fdtd_ctx* c, int comp, const int* idx, const double* 
       if (!std::isfinite(triples[3 * q + w])) return fail(FDTD_ERR_BADARG, "non-finite coefficient");
   }
   CK(cudaSetDevice(c->device));
+  if (int rc0 = fused_drop(c)) return rc0;
   int* d_idx = nullptr;
   double* d_trip = nullptr;
   int rc = FDTD_OK;
@@ -1345,6 +1911,7 @@ int fdtd_ctx_override_material(fdtd_ctx* c, int comp, const int* idx, const doub
   const long long n = c->ncomp[(comp + 3) % 6];
   std::vector<double> rows = c->rows64[comp];
   CK(cudaSetDevice(c->device));
+  if (int rc0 = fused_drop(c)) return rc0;
   for (int q = 0; q < count; q++) {
     if (idx[q] < 0 || idx[q] >= n) return fail(FDTD_ERR_BADARG, "cell index %d out of range", idx[q]);
     int r = -1;
@@ -1397,6 +1964,7 @@ int fdtd_ctx_set_tiling(fdtd_ctx* c, int x_planes_per_thread, int block_rows) {
     return fail(FDTD_ERR_BADARG, "block rows %d not in {1,2,4,8,16}", block_rows);
   c->ichunk = x_planes_per_thread;
   c->block_rows = block_rows;
+  c->chunk_set = true;
   invalidate(c);
   return FDTD_OK;
 }
@@ -1468,6 +2036,7 @@ int fdtd_ctx_read_field(fdtd_ctx* c, int which, double* host, long n) {
   if (which < 0 || which > 5) return fail(FDTD_ERR_BADARG, "field id %d not in 0..5", which);
   if (n != c->ncomp[which]) return fail(FDTD_ERR_BADARG, "field %d: buffer of %ld, need %lld", which, n, c->ncomp[which]);
   CK(cudaSetDevice(c->device));
+  if (int rc = to_dense(c)) return rc;
   return read_real(c, field_ptr(c, which), host, n);
 }
 
@@ -1476,6 +2045,7 @@ int fdtd_ctx_read_psi(fdtd_ctx* c, int f, int slot, double* host, long n) {
   if (f < 0 || f > 5 || slot < 0 || slot > 3 || !c->face[f].present) return fail(FDTD_ERR_BADARG, "no Psi slot %d on face %d", slot, f);
   if (n != c->face[f].n[slot]) return fail(FDTD_ERR_BADARG, "Psi buffer of %ld, need %lld", n, c->face[f].n[slot]);
   CK(cudaSetDevice(c->device));
+  if (int rc = to_dense(c)) return rc;
   return read_real(c, c->face[f].psi[slot], host, n);
 }
 
@@ -1565,6 +2135,8 @@ int fdtd_ctx_save_state(fdtd_ctx* c, void* buf, long long bytes) {
   if (rc) return rc;
   const StateHeader h = state_header(c);
   if (bytes != h.bytes) return fail(FDTD_ERR_BADARG, "state buffer of %lld bytes, need %lld", bytes, h.bytes);
+  rc = to_dense(c);
+  if (rc) return rc;
   char* p = (char*)buf;
   memcpy(p, &h, sizeof(h));
   p += sizeof(h);
@@ -1593,6 +2165,8 @@ int fdtd_ctx_load_state(fdtd_ctx* c, const void* buf, long long bytes) {
     return fail(FDTD_ERR_BADARG, "state was saved from a problem of another shape, precision or probe set");
   if (theirs.ts < 0 || theirs.ts > c->nsteps) return fail(FDTD_ERR_BADARG, "state step %d out of range", theirs.ts);
   const char* p = (const char*)buf + sizeof(StateHeader);
+  c->dense_valid = true;   // every value of the state is replaced
+  c->fs.valid = false;
   for (auto& q : state_ranges(c)) {
     CK(cudaMemcpyAsync(q.first, p, q.second, cudaMemcpyHostToDevice, c->stream));
     p += q.second;
@@ -1885,35 +2459,6 @@ int upload_vec(fdtd_batch* b, V** dst, const std::vector<V>& v) {
   if (!v.empty()) CK(cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice, b->stream));
   CK(cudaStreamSynchronize(b->stream));
   return FDTD_OK;
-}
-
-// Batched H/E kernel for a prefetch depth (as step_kernel) and grid kind.
-template <typename T, class C, bool EXACT>
-void (*batch_kernel(bool electric, int pf, bool persist))(const Instance<T, C>*, const BatchTile*, int, BatchCtl*,
-                                                           int) {
-#define FDTD_BK(PF)                                                                                           \
-  (electric ? (persist ? k_batch_half<T, C, EXACT, PF, true, true> : k_batch_half<T, C, EXACT, PF, true, false>) \
-            : (persist ? k_batch_half<T, C, EXACT, PF, false, true> : k_batch_half<T, C, EXACT, PF, false, false>))
-  if constexpr (C::kTable) {
-    if (pf == 3) return FDTD_BK(3);
-    if (pf == 4) return FDTD_BK(4);
-  }
-  if (pf == 2) return FDTD_BK(2);
-  return FDTD_BK(1);
-#undef FDTD_BK
-}
-
-// Grouped H/E kernel for a prefetch depth (as step_kernel).
-template <typename T, class C, bool EXACT>
-void (*batch_group_kernel(bool electric, int pf))(const BatchGroup<T, C>) {
-#define FDTD_GK(PF) (electric ? k_batch_group<T, C, EXACT, PF, true> : k_batch_group<T, C, EXACT, PF, false>)
-  if constexpr (C::kTable) {
-    if (pf == 3) return FDTD_GK(3);
-    if (pf == 4) return FDTD_GK(4);
-  }
-  if (pf == 2) return FDTD_GK(2);
-  return FDTD_GK(1);
-#undef FDTD_GK
 }
 
 int batch_worker_streams(fdtd_batch* b, int count);
@@ -2263,6 +2808,7 @@ int batch_run(fdtd_batch* b, int count, float* elapsed_ms = nullptr, KernelTimer
     int rc = check_ready(c);
     if (!rc) rc = ensure_traces(c);
     if (!rc && c->prec == FDTD_PREC_F32_TABLE && c->table_dirty) rc = prepare_table(c, &c->tcoef);
+    if (!rc && count > 0) rc = claim_dense(c);
     if (rc) {
       std::string msg = g_err;
       return fail(rc, "batch member %zu: %s", q, msg.c_str());

@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(256)
     k_batch_epilogue(const Instance<T, C>* __restrict__ inst, const BatchBlock* __restrict__ blocks) {
   const BatchBlock b = blocks[blockIdx.x];
   const Instance<T, C>& in = inst[b.inst];
-  epilogue_thread<T>(in.sp.f, in.sp.g, in.ff, in.pr, in.sp.ts, (long long)b.local * blockDim.x + threadIdx.x);
+  epilogue_thread<T>(in.sp.f, in.sp.g, in.ff, in.pr, *in.sp.ts, (long long)b.local * blockDim.x + threadIdx.x);
 }
 
 // Time-blocked DFT flush of every member (see k_dft_flush).
@@ -167,7 +167,8 @@ __global__ void __launch_bounds__(256)
     k_batch_flush(const Instance<T, C>* __restrict__ inst, const BatchBlock* __restrict__ blocks, int upto) {
   const BatchBlock b = blocks[blockIdx.x];
   const Instance<T, C>& in = inst[b.inst];
-  dft_flush_thread(in.ff, in.sp.ts, upto, (long long)b.local * blockDim.x + threadIdx.x);
+  if (flush_upto(in.ff, in.sp.ts, upto))
+    dft_flush_thread(in.ff, upto, (long long)b.local * blockDim.x + threadIdx.x);
 }
 
 }  // namespace fdtd

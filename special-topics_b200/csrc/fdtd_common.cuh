@@ -21,6 +21,20 @@ struct GridDims {
   int nx, ny, nz;
 };
 
+// The padded layout of fdtd_fused.cuh: one index for all six components.
+struct PaddedGrid {
+  int pitch, rows;
+};
+
+// Index of component c (0..5 = Hx Hy Hz Ex Ey Ez) at (i, j, k) in either layout.
+__device__ __forceinline__ long long field_index(const GridDims& g, int c, int i, int j, int k) {
+  const int rows = c == 1 || c == 3 || c == 5 ? g.ny + 1 : g.ny, cols = c >= 2 && c <= 4 ? g.nz + 1 : g.nz;
+  return ((long long)i * rows + j) * cols + k;
+}
+__device__ __forceinline__ long long field_index(const PaddedGrid& g, int, int i, int j, int k) {
+  return ((long long)i * g.rows + j) * g.pitch + k;
+}
+
 template <typename T>
 struct Fields {
   T *Hx, *Hy, *Hz, *Ex, *Ey, *Ez;
@@ -129,6 +143,35 @@ __device__ void voltage_probe(const Fields<T>& f, const Probes& pr, int q, int t
   }
 }
 
+// The same probes by a warp: the lanes fetch 32 samples at a time, every lane
+// then adds them in list order (one thread's chain of dependent loads, an index
+// and a sample per cell, took 15 us for a 15-cell port).
+template <typename T>
+__device__ void probe_warp(const Fields<T>& f, const Probes& pr, int q, int ts, int lane) {
+  const bool volt = q < pr.n_v;
+  const int u = volt ? q : q - pr.n_v, n = volt ? pr.v_count[u] : pr.i_count[u];
+  double sum = 0.0;
+  for (int m0 = 0; m0 < n; m0 += 32) {
+    const int m = m0 + lane;
+    double x = 0.0;
+    if (m < n)
+      x = volt ? (double)comp_ptr(f, 3 + pr.v_comp[u])[pr.v_idx[u][m]]
+               : mul(pr.i_w[u][m], (double)comp_ptr(f, pr.i_comp[u][m])[pr.i_idx[u][m]]);
+    for (int l = 0; l < min(32, n - m0); l++) sum = add(sum, __shfl_sync(0xffffffffu, x, l));
+  }
+  if (lane) return;
+  if (volt) {
+    const double v = mul(pr.v_csvf[u], sum);
+    pr.V[(long long)u * pr.nsteps + ts] = v;
+    if (!isfinite(v)) {
+      atomicExch(&pr.status[0], 5);
+      atomicMin(&pr.status[1], ts);
+    }
+  } else {
+    pr.I[(long long)u * pr.nsteps + ts] = sum;
+  }
+}
+
 // Names of the 24 accumulator arrays, in FarField::off order.
 enum {
   CJYXP, CJZXP, CJYXN, CJZXN, CJXYP, CJZYP, CJXYN, CJZYN, CJXZP, CJYZP, CJXZN, CJYZN,
@@ -148,9 +191,9 @@ __device__ __forceinline__ int sample_array(int group, int a) {
 // ts % block; this writes them into the running accumulators.
 __device__ __forceinline__ void store_samples(const FarField& ff, long long t, int ts, const double* v) {
   const long long npts = ff.sz[0] + ff.sz[1] + ff.sz[2];
-  float* s = ff.samples + ((long long)(ts % ff.block) * npts + t) * 8;
-#pragma unroll
-  for (int a = 0; a < 8; a++) s[a] = (float)v[a];
+  float4* s = reinterpret_cast<float4*>(ff.samples + ((long long)(ts % ff.block) * npts + t) * 8);
+  s[0] = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
+  s[1] = make_float4((float)v[4], (float)v[5], (float)v[6], (float)v[7]);
 }
 
 // One Kahan-compensated FP32 step: v = (sum, compensation), sum += x.
@@ -163,141 +206,135 @@ __device__ __forceinline__ void kahan_add(float2* v, float x) {
   *v = a;
 }
 
-__device__ __forceinline__ void acc2(const FarField& ff, int a, long long p, double c, double s, double t) {
-  double* re = ff.acc + ff.off[a] + p;
-  double* im = re + ff.nFreq * ff.sz[(a % 12) / 4];
-  if (ff.kahan) {
-    const float tf = (float)t;
-    kahan_add(reinterpret_cast<float2*>(re), __fmul_rn((float)c, tf));
-    kahan_add(reinterpret_cast<float2*>(im), __fmul_rn((float)s, tf));
-    return;
+// One step of the running DFT at a surface point: its 8 samples into the 8
+// arrays of its group.  Every accumulator is loaded before the first is stored:
+// in load-store pairs the chain of 8 memory latencies per frequency was the
+// epilogue's time (20 us for 15,000 points; 8 us this way).
+__device__ __forceinline__ void accumulate(const FarField& ff, int group, long long pt, int ts, const double* v) {
+  const long long sz = ff.sz[group], im = ff.nFreq * sz;
+  const double* ph = ff.ph + (long long)ts * ff.nFreq * 4;
+  double* re[8];
+#pragma unroll
+  for (int a = 0; a < 8; a++) re[a] = ff.acc + ff.off[sample_array(group, a)] + pt;
+  for (int m = 0; m < ff.nFreq; m++, ph += 4) {
+    const double c[2] = {ph[0], ph[2]}, s[2] = {ph[1], ph[3]};  // H-time, E-time
+    double r[8], i[8];
+#pragma unroll
+    for (int a = 0; a < 8; a++) {
+      r[a] = re[a][0];
+      i[a] = re[a][im];
+    }
+#pragma unroll
+    for (int a = 0; a < 8; a++) {
+      const int e = (a & 2) == 0;  // sample order: two magnetic (E-time), two electric (H-time), twice
+      if (ff.kahan) {
+        const float tf = (float)v[a];
+        kahan_add(reinterpret_cast<float2*>(&r[a]), __fmul_rn((float)c[e], tf));
+        kahan_add(reinterpret_cast<float2*>(&i[a]), __fmul_rn((float)s[e], tf));
+      } else if (group == 2 && a == 2) {
+        // zp Jx: the reference adds the Hx average (sample 3), then swaps it for
+        // the Hy average in a second statement (farfield.js:211-225); keep both
+        // roundings (with compensated FP32 only the net Hy term is added)
+        const double r1 = add(r[a], mul(c[0], v[3])), i1 = add(i[a], mul(s[0], v[3]));
+        r[a] = add(sub(r1, mul(c[0], v[3])), mul(c[0], v[2]));
+        i[a] = add(sub(i1, mul(s[0], v[3])), mul(s[0], v[2]));
+      } else {
+        r[a] = add(r[a], mul(c[e], v[a]));
+        i[a] = add(i[a], mul(s[e], v[a]));
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < 8; a++) {
+      re[a][0] = r[a];
+      re[a][im] = i[a];
+      re[a] += sz;
+    }
   }
-  *re = add(*re, mul(c, t));
-  *im = add(*im, mul(s, t));
 }
 
 // ---------------------------------------------------------------------------
 // Epilogue: running NF-FF DFT (farfield.js:90-248) on the six Huygens faces,
-// then the port voltages.  One thread per surface point (xp/xn, yp/yn and zp/zn
-// pairs share the point), looping over frequencies.
+// then the port voltages and, in the padded layout (whose step has no mid
+// launch), the port currents, a warp each.  One thread per surface point
+// (xp/xn, yp/yn and zp/zn pairs share the point), looping over frequencies.
 // ---------------------------------------------------------------------------
-template <typename T>
-__device__ __forceinline__ void epilogue_thread(const Fields<T>& f, const GridDims& g, const FarField& ff,
-                                                const Probes& probes, const int* ts_ptr, long long t) {
-  const int ts = *ts_ptr;
-  const int ny = g.ny, nz = g.nz, nyp1 = ny + 1, nzp1 = nz + 1;
+template <class G>
+constexpr bool kWarpProbes = false;
+template <>
+constexpr bool kWarpProbes<PaddedGrid> = true;
+
+// Threads of an epilogue in the padded layout.
+inline long long epilogue_threads(long long points, int probes) { return ((points + 31) / 32 + probes) * 32; }
+
+template <typename T, class G>
+__device__ __forceinline__ void epilogue_thread(const Fields<T>& f, const G& g, const FarField& ff,
+                                                const Probes& probes, int ts, long long t) {
   const long long nff = ff.nFreq > 0 ? ff.sz[0] + ff.sz[1] + ff.sz[2] : 0;
-  if (t >= nff) {
+  if constexpr (kWarpProbes<G>) {  // whole warps after the points' last one
+    const long long w = t / 32 - (nff + 31) / 32;
+    if (w >= 0) {
+      if (w < probes.n_v + probes.n_i) probe_warp(f, probes, (int)w, ts, (int)(t % 32));
+      return;
+    }
+    if (t >= nff) return;
+  } else if (t >= nff) {
     const long long q = t - nff;
     if (q < probes.n_v) voltage_probe(f, probes, (int)q, ts);
     return;
   }
-#define HX(i, j, k) (double)f.Hx[((long long)(i) * ny + (j)) * nz + (k)]
-#define HY(i, j, k) (double)f.Hy[((long long)(i) * nyp1 + (j)) * nz + (k)]
-#define HZ(i, j, k) (double)f.Hz[((long long)(i) * ny + (j)) * nzp1 + (k)]
-#define EX(i, j, k) (double)f.Ex[((long long)(i) * nyp1 + (j)) * nzp1 + (k)]
-#define EY(i, j, k) (double)f.Ey[((long long)(i) * ny + (j)) * nzp1 + (k)]
-#define EZ(i, j, k) (double)f.Ez[((long long)(i) * nyp1 + (j)) * nz + (k)]
-  const double* ph = ff.ph + (long long)ts * ff.nFreq * 4;
+#define HX(i, j, k) (double)f.Hx[field_index(g, 0, i, j, k)]
+#define HY(i, j, k) (double)f.Hy[field_index(g, 1, i, j, k)]
+#define HZ(i, j, k) (double)f.Hz[field_index(g, 2, i, j, k)]
+#define EX(i, j, k) (double)f.Ex[field_index(g, 3, i, j, k)]
+#define EY(i, j, k) (double)f.Ey[field_index(g, 4, i, j, k)]
+#define EZ(i, j, k) (double)f.Ez[field_index(g, 5, i, j, k)]
+  double v[8];
+  int group;
+  long long pt = t;
   if (t < ff.sz[0]) {
-    const int nj = (int)(t / ff.nk), nk = (int)(t % ff.nk);
+    group = 0;
+    const int nj = (int)pt / ff.nk, nk = (int)pt % ff.nk;
     const int j0 = ff.LJ + nj, k0 = ff.LK + nk, UI = ff.UI, LI = ff.LI;
-    const double tmyxp = mul(0.5, add(EZ(UI, j0, k0), EZ(UI, j0 + 1, k0)));
-    const double tmzxp = mul(-0.5, add(EY(UI, j0, k0), EY(UI, j0, k0 + 1)));
-    const double tjyxp = mul(-0.25, add(add(add(HZ(UI, j0, k0), HZ(UI, j0, k0 + 1)), HZ(UI - 1, j0, k0)), HZ(UI - 1, j0, k0 + 1)));
-    const double tjzxp = mul(0.25, add(add(add(HY(UI, j0, k0), HY(UI, j0 + 1, k0)), HY(UI - 1, j0, k0)), HY(UI - 1, j0 + 1, k0)));
-    const double tmyxn = mul(-0.5, add(EZ(LI, j0, k0), EZ(LI, j0 + 1, k0)));
-    const double tmzxn = mul(0.5, add(EY(LI, j0, k0), EY(LI, j0, k0 + 1)));
-    const double tjyxn = mul(0.25, add(add(add(HZ(LI, j0, k0), HZ(LI, j0, k0 + 1)), HZ(LI - 1, j0, k0)), HZ(LI - 1, j0, k0 + 1)));
-    const double tjzxn = mul(-0.25, add(add(add(HY(LI, j0, k0), HY(LI, j0 + 1, k0)), HY(LI - 1, j0, k0)), HY(LI - 1, j0 + 1, k0)));
-    if (ff.block) {  // time-blocked: buffer the samples, k_dft_flush accumulates them
-      const double v[8] = {tmyxp, tmzxp, tjyxp, tjzxp, tmyxn, tmzxn, tjyxn, tjzxn};
-      store_samples(ff, t, ts, v);
-      return;
-    }
-    for (int m = 0; m < ff.nFreq; m++) {
-      const long long p = (long long)m * ff.sz[0] + t;
-      const double ch = ph[4 * m], sh = ph[4 * m + 1], ce = ph[4 * m + 2], se = ph[4 * m + 3];
-      acc2(ff, CMYXP, p, ce, se, tmyxp);
-      acc2(ff, CMZXP, p, ce, se, tmzxp);
-      acc2(ff, CJYXP, p, ch, sh, tjyxp);
-      acc2(ff, CJZXP, p, ch, sh, tjzxp);
-      acc2(ff, CMYXN, p, ce, se, tmyxn);
-      acc2(ff, CMZXN, p, ce, se, tmzxn);
-      acc2(ff, CJYXN, p, ch, sh, tjyxn);
-      acc2(ff, CJZXN, p, ch, sh, tjzxn);
-    }
+    v[0] = mul(0.5, add(EZ(UI, j0, k0), EZ(UI, j0 + 1, k0)));
+    v[1] = mul(-0.5, add(EY(UI, j0, k0), EY(UI, j0, k0 + 1)));
+    v[2] = mul(-0.25, add(add(add(HZ(UI, j0, k0), HZ(UI, j0, k0 + 1)), HZ(UI - 1, j0, k0)), HZ(UI - 1, j0, k0 + 1)));
+    v[3] = mul(0.25, add(add(add(HY(UI, j0, k0), HY(UI, j0 + 1, k0)), HY(UI - 1, j0, k0)), HY(UI - 1, j0 + 1, k0)));
+    v[4] = mul(-0.5, add(EZ(LI, j0, k0), EZ(LI, j0 + 1, k0)));
+    v[5] = mul(0.5, add(EY(LI, j0, k0), EY(LI, j0, k0 + 1)));
+    v[6] = mul(0.25, add(add(add(HZ(LI, j0, k0), HZ(LI, j0, k0 + 1)), HZ(LI - 1, j0, k0)), HZ(LI - 1, j0, k0 + 1)));
+    v[7] = mul(-0.25, add(add(add(HY(LI, j0, k0), HY(LI, j0 + 1, k0)), HY(LI - 1, j0, k0)), HY(LI - 1, j0 + 1, k0)));
   } else if (t < ff.sz[0] + ff.sz[1]) {
-    const long long q = t - ff.sz[0];
-    const int ni = (int)(q / ff.nk), nk = (int)(q % ff.nk);
+    group = 1;
+    pt = t - ff.sz[0];
+    const int ni = (int)pt / ff.nk, nk = (int)pt % ff.nk;
     const int i0 = ff.LI + ni, k0 = ff.LK + nk, UJ = ff.UJ, LJ = ff.LJ;
-    const double tmxyp = mul(-0.5, add(EZ(i0, UJ, k0), EZ(i0 + 1, UJ, k0)));
-    const double tmzyp = mul(0.5, add(EX(i0, UJ, k0), EX(i0, UJ, k0 + 1)));
-    const double tjzyp = mul(-0.25, add(add(add(HX(i0, UJ, k0), HX(i0 + 1, UJ, k0)), HX(i0, UJ - 1, k0)), HX(i0 + 1, UJ - 1, k0)));
-    const double tjxyp = mul(0.25, add(add(add(HZ(i0, UJ, k0), HZ(i0, UJ, k0 + 1)), HZ(i0, UJ - 1, k0)), HZ(i0, UJ - 1, k0 + 1)));
-    const double tmxyn = mul(0.5, add(EZ(i0, LJ, k0), EZ(i0 + 1, LJ, k0)));
-    const double tmzyn = mul(-0.5, add(EX(i0, LJ, k0), EX(i0, LJ, k0 + 1)));
-    const double tjzyn = mul(0.25, add(add(add(HX(i0, LJ, k0), HX(i0 + 1, LJ, k0)), HX(i0, LJ - 1, k0)), HX(i0 + 1, LJ - 1, k0)));
-    const double tjxyn = mul(-0.25, add(add(add(HZ(i0, LJ, k0), HZ(i0, LJ, k0 + 1)), HZ(i0, LJ - 1, k0)), HZ(i0, LJ - 1, k0 + 1)));
-    if (ff.block) {  // time-blocked: buffer the samples, k_dft_flush accumulates them
-      const double v[8] = {tmxyp, tmzyp, tjzyp, tjxyp, tmxyn, tmzyn, tjzyn, tjxyn};
-      store_samples(ff, t, ts, v);
-      return;
-    }
-    for (int m = 0; m < ff.nFreq; m++) {
-      const long long p = (long long)m * ff.sz[1] + q;
-      const double ch = ph[4 * m], sh = ph[4 * m + 1], ce = ph[4 * m + 2], se = ph[4 * m + 3];
-      acc2(ff, CMXYP, p, ce, se, tmxyp);
-      acc2(ff, CMZYP, p, ce, se, tmzyp);
-      acc2(ff, CJZYP, p, ch, sh, tjzyp);
-      acc2(ff, CJXYP, p, ch, sh, tjxyp);
-      acc2(ff, CMXYN, p, ce, se, tmxyn);
-      acc2(ff, CMZYN, p, ce, se, tmzyn);
-      acc2(ff, CJZYN, p, ch, sh, tjzyn);
-      acc2(ff, CJXYN, p, ch, sh, tjxyn);
-    }
+    v[0] = mul(-0.5, add(EZ(i0, UJ, k0), EZ(i0 + 1, UJ, k0)));
+    v[1] = mul(0.5, add(EX(i0, UJ, k0), EX(i0, UJ, k0 + 1)));
+    v[2] = mul(-0.25, add(add(add(HX(i0, UJ, k0), HX(i0 + 1, UJ, k0)), HX(i0, UJ - 1, k0)), HX(i0 + 1, UJ - 1, k0)));
+    v[3] = mul(0.25, add(add(add(HZ(i0, UJ, k0), HZ(i0, UJ, k0 + 1)), HZ(i0, UJ - 1, k0)), HZ(i0, UJ - 1, k0 + 1)));
+    v[4] = mul(0.5, add(EZ(i0, LJ, k0), EZ(i0 + 1, LJ, k0)));
+    v[5] = mul(-0.5, add(EX(i0, LJ, k0), EX(i0, LJ, k0 + 1)));
+    v[6] = mul(0.25, add(add(add(HX(i0, LJ, k0), HX(i0 + 1, LJ, k0)), HX(i0, LJ - 1, k0)), HX(i0 + 1, LJ - 1, k0)));
+    v[7] = mul(-0.25, add(add(add(HZ(i0, LJ, k0), HZ(i0, LJ, k0 + 1)), HZ(i0, LJ - 1, k0)), HZ(i0, LJ - 1, k0 + 1)));
   } else {
-    const long long q = t - ff.sz[0] - ff.sz[1];
-    const int ni = (int)(q / ff.nj), nj = (int)(q % ff.nj);
+    group = 2;
+    pt = t - ff.sz[0] - ff.sz[1];
+    const int ni = (int)pt / ff.nj, nj = (int)pt % ff.nj;
     const int i0 = ff.LI + ni, j0 = ff.LJ + nj, UK = ff.UK, LK = ff.LK;
-    const double tmxzp = mul(0.5, add(EY(i0, j0, UK), EY(i0 + 1, j0, UK)));
-    const double tmyzp = mul(-0.5, add(EX(i0, j0, UK), EX(i0, j0 + 1, UK)));
-    const double tjxzp = mul(0.25, add(add(add(HX(i0, j0, UK), HX(i0 + 1, j0, UK)), HX(i0, j0, UK - 1)), HX(i0 + 1, j0, UK - 1)));
-    const double tjxzp2 = mul(-0.25, add(add(add(HY(i0, j0, UK), HY(i0, j0 + 1, UK)), HY(i0, j0, UK - 1)), HY(i0, j0 + 1, UK - 1)));
-    const double tmxzn = mul(-0.5, add(EY(i0, j0, LK), EY(i0 + 1, j0, LK)));
-    const double tmyzn = mul(0.5, add(EX(i0, j0, LK), EX(i0, j0 + 1, LK)));
-    const double tjxzn = mul(0.25, add(add(add(HY(i0, j0, LK), HY(i0, j0 + 1, LK)), HY(i0, j0, LK - 1)), HY(i0, j0 + 1, LK - 1)));
-    const double tjyzn = mul(-0.25, add(add(add(HX(i0, j0, LK), HX(i0 + 1, j0, LK)), HX(i0, j0, LK - 1)), HX(i0 + 1, j0, LK - 1)));
-    if (ff.block) {  // time-blocked: buffer the samples, k_dft_flush accumulates them
-      const double v[8] = {tmxzp, tmyzp, tjxzp2, tjxzp, tmxzn, tmyzn, tjxzn, tjyzn};
-      store_samples(ff, t, ts, v);
-      return;
-    }
-    for (int m = 0; m < ff.nFreq; m++) {
-      const long long p = (long long)m * ff.sz[2] + q;
-      const double ch = ph[4 * m], sh = ph[4 * m + 1], ce = ph[4 * m + 2], se = ph[4 * m + 3];
-      acc2(ff, CMXZP, p, ce, se, tmxzp);
-      acc2(ff, CMYZP, p, ce, se, tmyzp);
-      // zp Jx: the reference adds the Hx average, then swaps it for the Hy
-      // average in a second statement (farfield.js:211-225); keep both roundings
-      // (with compensated FP32 accumulators only the net Hy term is added).
-      if (ff.kahan) {
-        acc2(ff, CJXZP, p, ch, sh, tjxzp2);
-      } else {
-        double* re = ff.acc + ff.off[CJXZP] + p;
-        double* im = re + ff.nFreq * ff.sz[2];
-        const double r1 = add(*re, mul(ch, tjxzp));
-        const double i1 = add(*im, mul(sh, tjxzp));
-        *re = add(sub(r1, mul(ch, tjxzp)), mul(ch, tjxzp2));
-        *im = add(sub(i1, mul(sh, tjxzp)), mul(sh, tjxzp2));
-      }
-      acc2(ff, CJYZP, p, ch, sh, tjxzp);  // the reference's zp Jy is the same Hx average
-      acc2(ff, CMXZN, p, ce, se, tmxzn);
-      acc2(ff, CMYZN, p, ce, se, tmyzn);
-      acc2(ff, CJXZN, p, ch, sh, tjxzn);
-      acc2(ff, CJYZN, p, ch, sh, tjyzn);
-    }
+    v[0] = mul(0.5, add(EY(i0, j0, UK), EY(i0 + 1, j0, UK)));
+    v[1] = mul(-0.5, add(EX(i0, j0, UK), EX(i0, j0 + 1, UK)));
+    // zp: the reference's Jx is the Hy average, its Jy the Hx average
+    v[3] = mul(0.25, add(add(add(HX(i0, j0, UK), HX(i0 + 1, j0, UK)), HX(i0, j0, UK - 1)), HX(i0 + 1, j0, UK - 1)));
+    v[2] = mul(-0.25, add(add(add(HY(i0, j0, UK), HY(i0, j0 + 1, UK)), HY(i0, j0, UK - 1)), HY(i0, j0 + 1, UK - 1)));
+    v[4] = mul(-0.5, add(EY(i0, j0, LK), EY(i0 + 1, j0, LK)));
+    v[5] = mul(0.5, add(EX(i0, j0, LK), EX(i0, j0 + 1, LK)));
+    v[6] = mul(0.25, add(add(add(HY(i0, j0, LK), HY(i0, j0 + 1, LK)), HY(i0, j0, LK - 1)), HY(i0, j0 + 1, LK - 1)));
+    v[7] = mul(-0.25, add(add(add(HX(i0, j0, LK), HX(i0 + 1, j0, LK)), HX(i0, j0, LK - 1)), HX(i0 + 1, j0, LK - 1)));
   }
+  if (ff.block)  // time-blocked: buffer the samples, k_dft_flush accumulates them
+    store_samples(ff, t, ts, v);
+  else
+    accumulate(ff, group, pt, ts, v);
 #undef HX
 #undef HY
 #undef HZ
@@ -309,23 +346,17 @@ __device__ __forceinline__ void epilogue_thread(const Fields<T>& f, const GridDi
 template <typename T>
 __global__ void __launch_bounds__(256) k_epilogue(Fields<T> f, GridDims g, FarField ff, Probes probes,
                                                   const int* ts_ptr) {
-  epilogue_thread<T>(f, g, ff, probes, ts_ptr, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+  epilogue_thread<T>(f, g, ff, probes, *ts_ptr, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// Accumulates the buffered samples of steps [*ff.done, upto) into the
-// running DFT: one thread per (surface point pair, frequency), steps in
-// order.  upto < 0: flush only when the step just finished closes a block
-// (upto = ts + 1 then), so the launch can sit in every step of a graph.
-__device__ __forceinline__ void dft_flush_thread(const FarField& ff, const int* ts_ptr, int upto, long long q) {
+// Accumulates the buffered samples of the steps before `upto` that are not in
+// the running DFT yet (from the block's first step, or *ff.done when a run
+// started inside the block): one thread per (surface point pair, frequency),
+// steps in order.
+__device__ __forceinline__ void dft_flush_thread(const FarField& ff, int upto, long long q) {
   const long long npts = ff.sz[0] + ff.sz[1] + ff.sz[2];
   if (ff.block <= 0 || q >= npts * ff.nFreq) return;
-  if (upto >= 0 && upto % ff.block == 0) return;  // closed by the flush inside its last step
-  if (upto < 0) {
-    const int ts = *ts_ptr;
-    if ((ts + 1) % ff.block != 0) return;
-    upto = ts + 1;
-  }
-  const int from = *ff.done;
+  const int from = max(*ff.done, (upto - 1) / ff.block * ff.block);
   const long long t = q % npts;
   const int m = (int)(q / npts);
   const int group = t < ff.sz[0] ? 0 : t < ff.sz[0] + ff.sz[1] ? 1 : 2;
@@ -356,8 +387,19 @@ __device__ __forceinline__ void dft_flush_thread(const FarField& ff, const int* 
   }
 }
 
-__global__ void __launch_bounds__(256) k_dft_flush(FarField ff, const int* ts_ptr, int upto) {
-  dft_flush_thread(ff, ts_ptr, upto, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+// The steps a flush covers: upto >= 0, the end of a run (nothing to do when a
+// block closed there); -1, a launch inside every step of a graph, which acts
+// only when the step just finished, *ts_ptr, closes a block; -2, the same where
+// *ts_ptr is the step after it.
+__device__ __forceinline__ bool flush_upto(const FarField& ff, const int* ts_ptr, int& upto) {
+  if (ff.block <= 0) return false;
+  if (upto >= 0) return upto % ff.block != 0;
+  upto = *ts_ptr + (upto == -1 ? 1 : 0);
+  return upto % ff.block == 0;
+}
+
+static __global__ void __launch_bounds__(256) k_dft_flush(FarField ff, const int* ts_ptr, int upto) {
+  if (flush_upto(ff, ts_ptr, upto)) dft_flush_thread(ff, upto, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 }  // namespace fdtd
