@@ -223,9 +223,12 @@ typedef struct fdtd_batch fdtd_batch;
 
 /* Groups `count` handles of one device and one precision.  The batch owns no
  * member: members stay valid handles (readbacks, fdtd_status, their own runs)
- * and must outlive the batch.  By default each step of fdtd_batch_run is four
- * launches for the whole batch: H over a tile list spanning every member, the
- * mid-step kernel, E over the tile list, and the far-field/port epilogue
+ * and must outlive the batch.  By default, where every member can run the
+ * one-pass step (csrc/fdtd_fused.cuh) and their DFT blocks are of one length,
+ * each member's steps are a chain of its own, side by side on worker streams;
+ * the launch shape then has no effect.  Otherwise each step of fdtd_batch_run is
+ * four launches for the whole batch: H over a tile list spanning every member,
+ * the mid-step kernel, E over the tile list, and the far-field/port epilogue
  * (fdtd_batch_set_streams selects the member-kernel mode instead). */
 int fdtd_batch_create(fdtd_ctx* const* members, int count, fdtd_batch** out);
 void fdtd_batch_free(fdtd_batch* batch);
@@ -245,8 +248,8 @@ int fdtd_batch_get_tiling(const fdtd_batch* batch, int* x_planes_per_thread, int
  * (those of fdtd_ctx_run, with the batch's launch shape), the members spread
  * over S worker streams inside one CUDA graph, all steps of a graph for one
  * member before the next member of its stream (so a member's arrays stay in L2
- * from one step to the next).  streams = 0 (default) is the tile-list mode.
- * Results are identical in both modes.  S <= 32. */
+ * from one step to the next).  streams = 0 (default) is the one-pass or the
+ * tile-list mode.  Results are identical in all modes.  S <= 32. */
 int fdtd_batch_set_streams(fdtd_batch* batch, int streams);
 /* Block width along k of the batch's step launches (16 or 32), as
  * fdtd_ctx_set_block_width. */
@@ -267,8 +270,8 @@ int fdtd_batch_get_members_per_launch(const fdtd_batch* batch, int* members);
 int fdtd_batch_run(fdtd_batch* batch, int count);
 int fdtd_batch_run_timed(fdtd_batch* batch, int count, float* ms);
 /* Per-kernel mean durations (ms) of the batch's H, mid-step, E and epilogue
- * launches per step (member-kernel mode: each member timed alone, summed over
- * the members). */
+ * launches per step (member-kernel and one-pass mode: each member timed alone,
+ * summed over the members). */
 int fdtd_batch_profile_kernels(fdtd_batch* batch, int count, double* avg_ms);
 
 /* Whole probe traces, FP64, one value per step (first `n` steps). kind 0 = voltage, 1 = current. */

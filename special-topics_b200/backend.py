@@ -262,8 +262,9 @@ class Engine:
 
 class Batch:
     """Engines of one precision on one device advanced together
-    (fdtd_batch_* in include/fdtd_b200.h).  streams = 0: every step is four
-    launches for the whole batch over a tile list, or, with per_launch = P > 0,
+    (fdtd_batch_* in include/fdtd_b200.h).  streams = 0: each engine's one-pass
+    steps as a chain of their own, side by side; where an engine cannot run
+    them, or the DFT blocks differ in length, every step is four launches for the whole batch over a tile list, or, with per_launch = P > 0,
     H and E launches that each carry P members' parameter blocks as their
     kernel parameter (grouped mode); streams = S > 0: each member's own step
     kernels on S worker streams in one graph.  The engines stay usable for

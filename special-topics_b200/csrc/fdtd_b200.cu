@@ -95,7 +95,9 @@ struct RunGraphs {
   void clear() {
     for (auto& e : g) cudaGraphExecDestroy(e.second);
     g.clear();
+    rev++;
   }
+  long long rev = 0;  // times cleared: what else captured the same set-up is stale then
 };
 
 // The padded state of the one-pass step (fdtd_fused.cuh): allocated at the
@@ -576,6 +578,7 @@ int fused_pitch(const fdtd_ctx* c) {
 }
 long long fused_plane(const fdtd_ctx* c) { return (long long)(c->ny + 1) * fused_pitch(c); }
 
+// One zeroed allocation of the padded state.
 int fused_alloc(fdtd_ctx* c, void** p, size_t bytes) {
   const cudaError_t e = cudaMalloc(p, bytes);
   if (e != cudaSuccess) {
@@ -587,6 +590,22 @@ int fused_alloc(fdtd_ctx* c, void** p, size_t bytes) {
   CK(cudaMemsetAsync(*p, 0, bytes, c->stream));
   return FDTD_OK;
 }
+
+// The arrays of the padded state, in one allocation: some 45 of them, one call
+// each, took most of the build of a small problem.
+struct FusedArena {
+  struct Part {
+    void** p;
+    size_t at;
+  };
+  std::vector<Part> parts;
+  size_t size = 0;
+  template <typename V>
+  void add(V** p, size_t bytes) {
+    parts.push_back({(void**)p, size});
+    size += (bytes + 255) / 256 * 256;
+  }
+};
 
 // Every field and present Psi slot between the dense arrays and copy `cur`.
 template <typename T>
@@ -738,54 +757,34 @@ int fused_classes(fdtd_ctx* c, const C& coef, bool* ok) {
 }
 
 // Profiles b, a over a whole axis, zero outside the bands.
-template <typename T>
+int fused_axis_values(const fdtd_ctx* c, int a) { return (a == 0 ? c->nx + 1 : a == 1 ? c->ny + 1 : fused_pitch(c)) + 8; }
+
 int fused_profiles(fdtd_ctx* c) {
-  const int n_axis[3] = {c->nx + 1, c->ny + 1, fused_pitch(c)};
   for (int el = 0; el < 2; el++)
-    for (int a = 0; a < 3; a++)
-      for (int w = 0; w < 2; w++) {
-        std::vector<T> v(n_axis[a] + 8, T(0));
-        for (int side = 0; side < 2; side++) {
-          const HostFace& h = c->face[2 * a + side];
-          if (!h.present) continue;
-          const int st = el ? h.e_start : h.m_start;
-          CK(xfer(c, v.data() + st, h.prof[(el ? 0 : 2) + w], h.nc * sizeof(T), cudaMemcpyDeviceToHost));
-        }
-        int rc = fused_alloc(c, &c->fs.prof[el][a][w], v.size() * sizeof(T));
-        if (rc) return rc;
-        CK(xfer(c, c->fs.prof[el][a][w], v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
-      }
+    for (int f = 0; f < 6; f++) {
+      const HostFace& h = c->face[f];
+      for (int w = 0; w < 2 && h.present; w++)
+        CK(cudaMemcpyAsync((char*)c->fs.prof[el][f / 2][w] + (el ? h.e_start : h.m_start) * c->esz,
+                           h.prof[(el ? 0 : 2) + w], h.nc * c->esz, cudaMemcpyDeviceToDevice, c->stream));
+    }
   return FDTD_OK;
 }
 
-// Probe cells in the padded layout.
-int fused_probes(fdtd_ctx* c) {
+// Probe cells in the padded layout, probe after probe.
+std::vector<int> fused_probe_cells(const fdtd_ctx* c) {
   const int P = fused_pitch(c);
   const long long S = fused_plane(c);
-  auto at = [&](int comp, int idx) {
+  std::vector<int> v;
+  auto put = [&](int comp, int idx) {
     const int nj = (comp == 0 || comp == 2 || comp == 4) ? c->ny : c->ny + 1,
               nk = (comp == 0 || comp == 1 || comp == 5) ? c->nz : c->nz + 1;
-    return (int)((idx / (nj * nk)) * S + (long long)((idx / nk) % nj) * P + idx % nk);
+    v.push_back((int)((idx / (nj * nk)) * S + (long long)((idx / nk) % nj) * P + idx % nk));
   };
-  auto put = [&](int** dst, const std::vector<int>& v) {
-    int rc = fused_alloc(c, (void**)dst, std::max<size_t>(v.size(), 1) * sizeof(int));
-    if (rc) return rc;
-    CK(xfer(c, *dst, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice));
-    return (int)FDTD_OK;
-  };
-  for (size_t q = 0; q < c->vprobe.size(); q++) {
-    std::vector<int> v;
-    for (int x : c->vprobe[q].cells) v.push_back(at(3 + c->vprobe[q].comp, x));
-    int rc = put(&c->fs.v_idx[q], v);
-    if (rc) return rc;
-  }
-  for (size_t q = 0; q < c->iprobe.size(); q++) {
-    std::vector<int> v;
-    for (size_t m = 0; m < c->iprobe[q].cells.size(); m++) v.push_back(at(c->iprobe[q].comps[m], c->iprobe[q].cells[m]));
-    int rc = put(&c->fs.i_idx[q], v);
-    if (rc) return rc;
-  }
-  return FDTD_OK;
+  for (const auto& pr : c->vprobe)
+    for (int x : pr.cells) put(3 + pr.comp, x);
+  for (const auto& pr : c->iprobe)
+    for (size_t m = 0; m < pr.cells.size(); m++) put(pr.comps[m], pr.cells[m]);
+  return v;
 }
 
 // Builds the padded state.  It serves problems whose CPML bands are disjoint
@@ -813,19 +812,34 @@ int fused_build(fdtd_ctx* c) {
   size_t free_b = 0, total_b = 0;
   CK(cudaMemGetInfo(&free_b, &total_b));
   if (need > free_b / 2) return FDTD_OK;
-  int rc = FDTD_OK;
-  for (int w = 0; w < 2 && !rc; w++)
-    for (int q = 0; q < 6 && !rc; q++) rc = fused_alloc(c, &fs.f[w][q], comp);
-  for (int a = 0; a < 3 && !rc; a++)
-    if (psi[a])
-      for (int s = 0; s < 2 && !rc; s++) {
-        for (int w = 0; w < 2 && !rc; w++) rc = fused_alloc(c, &fs.ph[a][w][s], (size_t)psi[a] * c->esz);
-        if (!rc) rc = fused_alloc(c, &fs.pe[a][s], (size_t)psi[a] * c->esz);
-      }
-  if (!rc) rc = fused_alloc(c, (void**)&fs.cls, (size_t)elems * 2);
-  if (!rc) rc = fused_alloc(c, (void**)&fs.d_ts, 2 * sizeof(int));
-  if (!rc) rc = c->esz == 8 ? fused_profiles<double>(c) : fused_profiles<float>(c);
-  if (!rc) rc = fused_probes(c);
+  FusedArena ar;
+  for (int w = 0; w < 2; w++)
+    for (int q = 0; q < 6; q++) ar.add(&fs.f[w][q], comp);
+  for (int a = 0; a < 3; a++)
+    for (int s = 0; s < 2 && psi[a]; s++) {
+      for (int w = 0; w < 2; w++) ar.add(&fs.ph[a][w][s], (size_t)psi[a] * c->esz);
+      ar.add(&fs.pe[a][s], (size_t)psi[a] * c->esz);
+    }
+  ar.add(&fs.cls, (size_t)elems * 2);
+  ar.add(&fs.d_ts, 2 * sizeof(int));
+  for (int el = 0; el < 2; el++)
+    for (int a = 0; a < 3; a++)
+      for (int w = 0; w < 2; w++) ar.add(&fs.prof[el][a][w], fused_axis_values(c, a) * c->esz);
+  const std::vector<int> cells = fused_probe_cells(c);
+  int* d_cells = nullptr;
+  ar.add(&d_cells, cells.size() * sizeof(int));
+  void* base = nullptr;
+  int rc = fused_alloc(c, &base, ar.size);
+  if (!rc) {
+    for (const FusedArena::Part& q : ar.parts) *q.p = (char*)base + q.at;
+    rc = fused_profiles(c);
+  }
+  if (!rc && !cells.empty()) {
+    CK(cudaMemcpyAsync(d_cells, cells.data(), cells.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    for (size_t q = 0; q < c->vprobe.size(); d_cells += c->vprobe[q++].cells.size()) fs.v_idx[q] = d_cells;
+    for (size_t q = 0; q < c->iprobe.size(); d_cells += c->iprobe[q++].cells.size()) fs.i_idx[q] = d_cells;
+  }
   bool ok = false;
   if (!rc) {
     if (c->prec == FDTD_PREC_F64)
@@ -841,7 +855,7 @@ int fused_build(fdtd_ctx* c) {
 }
 
 // Makes the padded state hold the current step; *use = false: half-step path.
-int fused_ready(fdtd_ctx* c, bool* use) {
+int fused_usable(fdtd_ctx* c, bool* use) {
   FusedState& fs = c->fs;
   *use = false;
   if (!fs.tried) {
@@ -854,9 +868,17 @@ int fused_ready(fdtd_ctx* c, bool* use) {
       fs.tried = true;
     }
   }
-  if (!fs.ok) return FDTD_OK;
+  *use = fs.ok;
+  return FDTD_OK;
+}
+
+// And makes it hold the current fields and step.
+int fused_ready(fdtd_ctx* c, bool* use) {
+  FusedState& fs = c->fs;
+  int rc = fused_usable(c, use);
+  if (rc || !*use) return rc;
   if (!fs.valid) {
-    int rc = fused_copy_any(c, 1);
+    rc = fused_copy_any(c, 1);
     if (rc) return rc;
     fs.valid = true;
     fs.ts_at = -1;
@@ -865,7 +887,6 @@ int fused_ready(fdtd_ctx* c, bool* use) {
     CK(xfer(c, fs.d_ts + fs.cur, &c->ts, sizeof(int), cudaMemcpyHostToDevice));
     fs.ts_at = c->ts;
   }
-  *use = true;
   return FDTD_OK;
 }
 
@@ -906,7 +927,7 @@ bool fused_map(const fdtd_ctx* c, CUtensorMap* m, const T* base, int w, int rows
 // without the y bands', 1.7 without any).
 constexpr double kFusedFill = 5, kFusedBand = 0.6;
 template <typename T>
-void fused_shape(const fdtd_ctx* c, FusedParams<T>& p) {
+void fused_shape(const fdtd_ctx* c, FusedParams<T>& p, double share) {
   const int cols = c->nz + 1;
   // owned columns: all of them, or a multiple of four (a tile starts on 16
   // bytes) with room for the halo group
@@ -928,7 +949,7 @@ void fused_shape(const fdtd_ctx* c, FusedParams<T>& p) {
   slow(p.axis[1], kTileRows - 1, p.tj, p.slow_j);
   slow(p.axis[2], (p.rk - p.halo_k) * V, p.tk, p.slow_k);
   const int nxp = c->nx + 1;
-  if (c->chunk_set) {
+  if (c->chunk_set && share == 1) {
     p.tx = (nxp + c->ichunk - 1) / c->ichunk;
     return;
   }
@@ -939,7 +960,8 @@ void fused_shape(const fdtd_ctx* c, FusedParams<T>& p) {
   int xb[2] = {0, 0};  // planes in the x bands
   for (int f = 0; f < 2; f++) xb[f] = std::max(p.axis[0].nc[0][f], p.axis[0].nc[1][f]);
   double t_best = -1;
-  const int slots = 148 * FusedShape<T>::kBlocks, n_max = std::min(nxp, 64 + 4 * slots / (p.tk * p.tj));
+  const int slots = std::max(1, (int)(148 * FusedShape<T>::kBlocks * share));
+  const int n_max = std::min(nxp, 64 + 4 * slots / (p.tk * p.tj));
   for (int n = 1; n <= n_max; n++) {
     std::map<double, int> free_at;  // time -> slots
     free_at[0] = slots;
@@ -968,7 +990,7 @@ void fused_shape(const fdtd_ctx* c, FusedParams<T>& p) {
 }
 
 template <typename T>
-FusedParams<T> fused_params(const fdtd_ctx* c, int flip) {
+FusedParams<T> fused_params(const fdtd_ctx* c, int flip, double share) {
   const FusedState& fs = c->fs;
   FusedParams<T> p{};
   p.nx = c->nx; p.ny = c->ny; p.nz = c->nz;
@@ -1002,7 +1024,7 @@ FusedParams<T> fused_params(const fdtd_ctx* c, int flip) {
   p.src = dev_sources<T>(c);
   p.x_wall = c->x_wall;
   p.fault = c->d_status;
-  fused_shape(c, p);
+  fused_shape(c, p, share);
   for (int q = 0; q < 6; q++) {
     if (!fused_map(c, &p.map[q], p.fi[q], kTileW, q < 3 ? kTileRows : kTileRows + 1)) p.tx = 0;  // no maps: no launch
   }
@@ -1019,23 +1041,25 @@ Probes fused_dev_probes(const fdtd_ctx* c) {
 
 long long surface_points(const fdtd_ctx* c) { return c->nFreq > 0 ? c->ffsz[0] + c->ffsz[1] + c->ffsz[2] : 0; }
 
-// `count` steps from copy `flip` and step `ts` on the handle's stream.  A step's
-// epilogue is queued after the next step's launch, and runs beside it; the last
-// one's after its own.
+// `count` steps from copy `flip` and step `ts` on stream `st`.  Alone on the
+// device (share 1), a step's epilogue is queued after the next step's launch and
+// runs beside it, the last one's after its own; with other problems' launches
+// around it (share < 1, its part of the device) a launch waits for the one ahead
+// instead of holding slots that they could use.
 template <typename T, bool EXACT>
-int fused_enqueue_steps(fdtd_ctx* c, int count, int flip, int ts, KernelTimer* tm) {
-  const FusedParams<T> pf[2] = {fused_params<T>(c, 0), fused_params<T>(c, 1)};  // by the copy read
+int fused_enqueue_steps(fdtd_ctx* c, int count, int flip, int ts, KernelTimer* tm, cudaStream_t st, double share) {
+  const bool alone = share == 1;
+  const FusedParams<T> pf[2] = {fused_params<T>(c, 0, share), fused_params<T>(c, 1, share)};  // by the copy read
   if (pf[0].tx == 0 || pf[1].tx == 0) return fail(FDTD_ERR_CUDA, "cannot encode the step's tensor maps");
   const Probes pr = fused_dev_probes(c);
   const FarField ff = dev_ff(c);
-  cudaStream_t st = c->stream;
   const int probes = pr.n_v + pr.n_i;
   const long long pts = surface_points(c);
   const unsigned epi = pts + probes ? (unsigned)((epilogue_threads(pts, probes) + 255) / 256) : 0;
   // the epilogue of step `step`, under the parameters of the step after it or its own
   auto epilogue = [&](const FusedParams<T>& p, int step, bool late) -> cudaError_t {
     if (!epi) return cudaSuccess;
-    const cudaError_t e = fused_epilogue<T>(p, ff, pr, epi, late, st);
+    const cudaError_t e = fused_epilogue<T>(p, ff, pr, epi, late, alone, st);
     if (e == cudaSuccess && c->dft_block > 0 && (step + 1) % c->dft_block == 0)
       k_dft_flush<<<(unsigned)((pts * c->nFreq + 255) / 256), 256, 0, st>>>(ff, late ? p.ts : p.ts_next, -2);
     return e;
@@ -1043,15 +1067,16 @@ int fused_enqueue_steps(fdtd_ctx* c, int count, int flip, int ts, KernelTimer* t
   for (int s = 0; s < count; s++, flip ^= 1) {
     const FusedParams<T>& p = pf[flip];
     if (tm) CK(cudaEventRecord(tm->ev[0], st));
-    CK((fused_step<T, EXACT>(p, st)));
+    CK((fused_step<T, EXACT>(p, alone, st)));
     if (tm) CK(cudaEventRecord(tm->ev[1], st));
     if (!p.x_wall) CK((fused_wall<T, EXACT>(p, st)));
     if (tm) {
       CK(cudaEventRecord(tm->ev[2], st));
       CK(cudaEventRecord(tm->ev[3], st));
     }
-    if (!tm && s > 0) CK(epilogue(p, ts + s - 1, true));
-    if (tm || s + 1 == count) CK(epilogue(p, ts + s, false));
+    const bool late = alone && !tm;
+    if (late && s > 0) CK(epilogue(p, ts + s - 1, true));
+    if (!late || s + 1 == count) CK(epilogue(p, ts + s, false));
     if (tm) {
       CK(cudaEventRecord(tm->ev[4], st));
       CK(cudaEventSynchronize(tm->ev[4]));
@@ -1066,10 +1091,12 @@ int fused_enqueue_steps(fdtd_ctx* c, int count, int flip, int ts, KernelTimer* t
   return FDTD_OK;
 }
 
-int fused_enqueue(fdtd_ctx* c, int count, int ts, KernelTimer* tm = nullptr) {
-  if (c->prec == FDTD_PREC_F64) return fused_enqueue_steps<double, true>(c, count, c->fs.cur, ts, tm);
-  if (c->prec == FDTD_PREC_F32) return fused_enqueue_steps<float, true>(c, count, c->fs.cur, ts, tm);
-  return fused_enqueue_steps<float, false>(c, count, c->fs.cur, ts, tm);
+int fused_enqueue(fdtd_ctx* c, int count, KernelTimer* tm = nullptr, cudaStream_t st = nullptr, double share = 1) {
+  if (!st) st = c->stream;
+  const int flip = c->fs.cur, ts = c->ts;
+  if (c->prec == FDTD_PREC_F64) return fused_enqueue_steps<double, true>(c, count, flip, ts, tm, st, share);
+  if (c->prec == FDTD_PREC_F32) return fused_enqueue_steps<float, true>(c, count, flip, ts, tm, st, share);
+  return fused_enqueue_steps<float, false>(c, count, flip, ts, tm, st, share);
 }
 
 int enqueue(fdtd_ctx* c, int count, KernelTimer* tm = nullptr, cudaStream_t st = nullptr) {
@@ -1133,8 +1160,8 @@ int graph_for(RunGraphs& rg, cudaStream_t st, int steps, int tag, Enq enq, cudaG
 // `period` steps, and `tag` is where in it the run starts.
 template <class Enq>
 int run_plan(RunGraphs& rg, cudaStream_t st, int count, int launches_per_step, Enq enq,
-             std::vector<cudaGraphExec_t>* plan, int period = 1, int tag = 0) {
-  int cap = std::max(kGraphSteps, kMaxGraphNodes / std::max(1, launches_per_step));
+             std::vector<cudaGraphExec_t>* plan, int period = 1, int tag = 0, int cap = 0) {
+  if (!cap) cap = std::max(kGraphSteps, kMaxGraphNodes / std::max(1, launches_per_step));
   cap = std::max(cap / period, 1) * period;
   plan->clear();
   if (count <= 0) return FDTD_OK;
@@ -1187,7 +1214,7 @@ int run_steps(fdtd_ctx* c, int count, float* elapsed_ms = nullptr, KernelTimer* 
   if (!tm && fused) {
     // a graph depends on the copy it starts from and on where DFT blocks close
     const int per = c->dft_block > 0 ? c->dft_block : 1;
-    rc = run_plan(c->graphs, c->stream, count, 3, [c](int n) { return fused_enqueue(c, n, c->ts); }, &plan, 2 * per,
+    rc = run_plan(c->graphs, c->stream, count, 3, [c](int n) { return fused_enqueue(c, n); }, &plan, 2 * per,
                   2 * (c->ts % per) + c->fs.cur);
     if (rc) return rc;
   } else if (!tm) {
@@ -1207,7 +1234,7 @@ int run_steps(fdtd_ctx* c, int count, float* elapsed_ms = nullptr, KernelTimer* 
     c->fs.valid = true;
   }
   if (tm) {
-    rc = fused ? fused_enqueue(c, count, c->ts, tm) : enqueue(c, count, tm);
+    rc = fused ? fused_enqueue(c, count, tm) : enqueue(c, count, tm);
     if (rc) return rc;
   }
   for (cudaGraphExec_t ge : plan) CK(cudaGraphLaunch(ge, c->stream));
@@ -2444,11 +2471,17 @@ struct fdtd_batch {
   std::vector<unsigned char> groups;  // host copies of the BatchGroup parameter structs
   int ngroups = 0;
   size_t group_size = 0;
+  // one-pass mode (streams == 0, every member can run the one-pass step): what
+  // the cached graphs were captured from, two numbers a member
+  std::vector<long long> chain_key;
 };
 
 namespace {
 
-void batch_drop_graph(fdtd_batch* b) { b->graphs.clear(); }
+void batch_drop_graph(fdtd_batch* b) {
+  b->graphs.clear();
+  b->chain_key.clear();
+}
 
 template <class V>
 int upload_vec(fdtd_batch* b, V** dst, const std::vector<V>& v) {
@@ -2747,16 +2780,86 @@ int batch_member_enqueue(fdtd_batch* b, int count) {
   return rc;
 }
 
-int batch_run_members(fdtd_batch* b, int count, float* elapsed_ms, KernelTimer* tm) {
+// One-pass mode.  A member's steps are a chain of launches that needs none of
+// the other members', so the chains run side by side, each on its worker stream
+// (member-major, as above), with blocks for its share of the device: no launch
+// waits for the slowest member, and a member's last blocks overlap the others'
+// first.  160 steps of 32 antennas of 1.1 M cells (material table), half-step
+// tile list 224.5 ms; chains on 2, 4, 8, 16, 32 streams 200, 161, 139, 133,
+// 132 ms.  6 FP64 antennas 53.9 ms; 34.0, 33.0, 29.3 ms on 2, 4, 6.
+// Launches of a chain graph: 32 members' graphs of 32 steps run as fast as of
+// 160 (132.3 ms), and the first run, which captures them, took 264 ms for 342.
+constexpr int kChainNodes = 4096;
+int batch_chain_streams(const fdtd_batch* b) { return std::min((int)b->m.size(), kMaxBatchStreams); }
+
+int batch_chain_enqueue(fdtd_batch* b, int count) {
+  const int S = batch_chain_streams(b);
+  CK(cudaEventRecord(b->fork_ev, b->stream));
+  for (int q = 0; q < S; q++) CK(cudaStreamWaitEvent(b->ws[q], b->fork_ev, 0));
+  int rc = FDTD_OK;
+  for (size_t q = 0; q < b->m.size() && !rc; q++)
+    rc = fused_enqueue(b->m[q], count, nullptr, b->ws[q % S], S > 1 ? 1.0 / S : 1);
+  for (int q = 0; q < S; q++) {
+    CK(cudaEventRecord(b->wev[q], b->ws[q]));
+    CK(cudaStreamWaitEvent(b->stream, b->wev[q], 0));
+  }
+  return rc;
+}
+
+// Whether every member can run the one-pass step (their DFT blocks closing
+// together); then makes them hold the current state in that form.
+int batch_chain_ready(fdtd_batch* b, bool* use) {
+  *use = b->streams == 0;
+  for (size_t q = 0; q < b->m.size() && *use; q++) {
+    *use = b->m[q]->dft_block == b->m[0]->dft_block;
+    if (!*use) break;
+    int rc = fused_usable(b->m[q], use);
+    if (rc) return rc;
+  }
+  for (size_t q = 0; q < b->m.size() && *use; q++) {
+    fdtd_ctx* c = b->m[q];
+    int rc = fused_ready(c, use);
+    if (rc) return rc;
+    CK(cudaStreamSynchronize(c->stream));
+    if (c->dirty) {
+      c->graphs.clear();
+      c->dirty = false;
+    }
+  }
+  return FDTD_OK;
+}
+
+// Runs the members: by their own step kernels on worker streams, or (chain) as
+// one-pass chains.
+int batch_run_members(fdtd_batch* b, int count, bool chain, float* elapsed_ms, KernelTimer* tm) {
   const int ts = b->m[0]->ts;
-  int rc = batch_worker_streams(b, b->streams);
+  int rc = batch_worker_streams(b, chain ? batch_chain_streams(b) : b->streams);
   if (rc) return rc;
+  if (chain) {
+    std::vector<long long> key;
+    for (fdtd_ctx* c : b->m) {
+      key.push_back(c->graphs.rev);
+      key.push_back(c->fs.cur ^ b->m[0]->fs.cur);
+    }
+    if (key != b->chain_key) {
+      batch_drop_graph(b);
+      b->chain_key = key;
+    }
+  } else if (!b->chain_key.empty()) {
+    batch_drop_graph(b);
+  }
   // the whole run as cached graphs, captured before the first launch
   std::vector<cudaGraphExec_t> plan;
   if (!tm) {
     int per_step = 0;
     for (fdtd_ctx* c : b->m) per_step += c->dft_block > 0 ? 5 : 4;
-    rc = run_plan(b->graphs, b->stream, count, per_step, [b](int n) { return batch_member_enqueue(b, n); }, &plan);
+    if (chain) {
+      const int per = b->m[0]->dft_block > 0 ? b->m[0]->dft_block : 1;
+      rc = run_plan(b->graphs, b->stream, count, per_step, [b](int n) { return batch_chain_enqueue(b, n); }, &plan,
+                    2 * per, 2 * (ts % per) + b->m[0]->fs.cur, std::max(1, kChainNodes / per_step));
+    } else {
+      rc = run_plan(b->graphs, b->stream, count, per_step, [b](int n) { return batch_member_enqueue(b, n); }, &plan);
+    }
     if (rc) return rc;
   }
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -2769,11 +2872,18 @@ int batch_run_members(fdtd_batch* b, int count, float* elapsed_ms, KernelTimer* 
     // one member at a time on the batch's stream: per-kernel times summed over members
     for (size_t q = 0; q < b->m.size() && !rc; q++) {
       MemberShape shape(b->m[q], b);
-      rc = enqueue(b->m[q], count, tm, b->stream);
+      rc = chain ? fused_enqueue(b->m[q], count, tm, b->stream) : enqueue(b->m[q], count, tm, b->stream);
     }
     if (rc) return rc;
   }
+  if (chain && count > 0)  // from here the padded states run ahead of the dense ones
+    for (fdtd_ctx* c : b->m) c->dense_valid = false;
   for (cudaGraphExec_t ge : plan) CK(cudaGraphLaunch(ge, b->stream));
+  if (chain)
+    for (fdtd_ctx* c : b->m) {
+      c->fs.cur ^= count & 1;
+      c->fs.ts_at = ts + count;
+    }
   if (elapsed_ms) {
     CK(cudaEventRecord(ev1, b->stream));
     CK(cudaEventSynchronize(ev1));
@@ -2808,15 +2918,23 @@ int batch_run(fdtd_batch* b, int count, float* elapsed_ms = nullptr, KernelTimer
     int rc = check_ready(c);
     if (!rc) rc = ensure_traces(c);
     if (!rc && c->prec == FDTD_PREC_F32_TABLE && c->table_dirty) rc = prepare_table(c, &c->tcoef);
-    if (!rc && count > 0) rc = claim_dense(c);
     if (rc) {
       std::string msg = g_err;
       return fail(rc, "batch member %zu: %s", q, msg.c_str());
     }
   }
   CK(cudaSetDevice(b->device));
-  if (b->streams > 0) return batch_run_members(b, count, elapsed_ms, tm);
-  int rc = batch_prepare_any(b);
+  bool chain = false;
+  int rc = count > 0 ? batch_chain_ready(b, &chain) : FDTD_OK;
+  if (rc) return rc;
+  if (chain) return batch_run_members(b, count, true, elapsed_ms, tm);
+  for (size_t q = 0; q < b->m.size() && count > 0; q++)
+    if ((rc = claim_dense(b->m[q]))) {
+      std::string msg = g_err;
+      return fail(rc, "batch member %zu: %s", q, msg.c_str());
+    }
+  if (b->streams > 0) return batch_run_members(b, count, false, elapsed_ms, tm);
+  rc = batch_prepare_any(b);
   if (rc) return rc;
   const int ctl_ts = ts - 1;
   CK(cudaMemcpyAsync(&b->d_ctl->ts, &ctl_ts, sizeof(int), cudaMemcpyHostToDevice, b->stream));

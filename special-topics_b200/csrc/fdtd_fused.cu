@@ -6,34 +6,34 @@ namespace fdtd {
 
 namespace {
 
-// A launch whose blocks may start before the launch ahead of it has ended.
+// A launch; `early`: its blocks may start before the launch ahead of it has ended.
 template <typename... P, typename... A>
-cudaError_t launch_early(void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st,
+cudaError_t launch(bool early, void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t st,
                          A... args) {
-  cudaLaunchAttribute early{};
-  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cfg.attrs = &early;
-  cfg.numAttrs = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 }  // namespace
 
 template <typename T, bool EXACT>
-cudaError_t fused_step(const FusedParams<T>& p, cudaStream_t st) {
+cudaError_t fused_step(const FusedParams<T>& p, bool early, cudaStream_t st) {
   const int smem = fused_smem_bytes<T>(), tiles = p.tk * p.tj * p.tx;
   if (smem > 48 * 1024) {
     const cudaError_t e =
         cudaFuncSetAttribute(k_fused<T, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
   }
-  return launch_early(k_fused<T, EXACT>, (unsigned)tiles, FusedShape<T>::kThreads, (size_t)smem, st, p);
+  return launch(early, k_fused<T, EXACT>, (unsigned)tiles, FusedShape<T>::kThreads, (size_t)smem, st, p);
 }
 
 template <typename T, bool EXACT>
@@ -45,8 +45,8 @@ cudaError_t fused_wall(const FusedParams<T>& p, cudaStream_t st) {
 
 template <typename T>
 cudaError_t fused_epilogue(const FusedParams<T>& p, const FarField& ff, const Probes& pr, unsigned blocks,
-                           bool late, cudaStream_t st) {
-  return launch_early(k_fused_epilogue<T>, blocks, 256, 0, st, p, ff, pr, (int)late);
+                           bool late, bool early, cudaStream_t st) {
+  return launch(early, k_fused_epilogue<T>, blocks, 256, 0, st, p, ff, pr, (int)late);
 }
 
 template <typename T, class C>
@@ -73,14 +73,14 @@ cudaError_t fused_repack(T* pad, long long si, long long sj, T* dense, int ni, i
 }
 
 #define FDTD_FUSED(T, EXACT)                                                                                       \
-  template cudaError_t fused_step<T, EXACT>(const FusedParams<T>&, cudaStream_t); \
+  template cudaError_t fused_step<T, EXACT>(const FusedParams<T>&, bool, cudaStream_t); \
   template cudaError_t fused_wall<T, EXACT>(const FusedParams<T>&, cudaStream_t);
 FDTD_FUSED(double, true)
 FDTD_FUSED(float, true)
 FDTD_FUSED(float, false)
 #define FDTD_FUSED_T(T)                                                                                            \
   template cudaError_t fused_epilogue<T>(const FusedParams<T>&, const FarField&, const Probes&, unsigned, bool,    \
-                                         cudaStream_t);                                                            \
+                                         bool, cudaStream_t);                                                            \
   template cudaError_t fused_repack<T>(T*, long long, long long, T*, int, int, int, int, cudaStream_t);
 FDTD_FUSED_T(double)
 FDTD_FUSED_T(float)

@@ -1048,12 +1048,12 @@ __global__ void __launch_bounds__(256) k_repack(T* pad, long long si, long long 
 // Launchers (fdtd_fused.cu).
 // ---------------------------------------------------------------------------
 template <typename T, bool EXACT>
-cudaError_t fused_step(const FusedParams<T>& p, cudaStream_t st);
+cudaError_t fused_step(const FusedParams<T>& p, bool early, cudaStream_t st);
 template <typename T, bool EXACT>
 cudaError_t fused_wall(const FusedParams<T>& p, cudaStream_t st);
 template <typename T>
 cudaError_t fused_epilogue(const FusedParams<T>& p, const FarField& ff, const Probes& pr, unsigned blocks,
-                           bool late, cudaStream_t st);
+                           bool late, bool early, cudaStream_t st);
 template <typename T, class C>
 cudaError_t fused_class_find(const StepParams<T, C>& s, int pitch, unsigned n, const ClassTable& tb, cudaStream_t st);
 template <typename T, class C>

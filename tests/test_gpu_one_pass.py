@@ -119,3 +119,34 @@ def test_chunks_of_any_length_match(planes):
             eng.run(STEPS)
             states.append(_state(eng))
     _assert_same(*states)
+
+
+@pytest.mark.parametrize("blocks", [(0, 0, 0), (4, 4, 4), (0, 4, 3)], ids=str)
+@pytest.mark.parametrize("group,per_launch", [(0, 0), (2, 0), (0, 2)])
+def test_batch_chains_match_members_alone(blocks, group, per_launch):
+    """Members at different copies of their state; DFT blocks of one length
+    (chains) and of several (tile list, persistent grid, grouped launches)."""
+    probs = [_problem(SHAPES[q])[1] for q in (0, 3, 6)]
+    want = []
+    for p, d in zip(probs, blocks):
+        with Engine(p, "f32-table", dft_block=d) as eng:
+            eng.run(STEPS)
+            want.append(_state(eng))
+    engs = [Engine(p, "f32-table", dft_block=d) for p, d in zip(probs, blocks)]
+    try:
+        engs[1].run(1)
+        engs[0].run(1)
+        with Batch([engs[2]]) as b:
+            b.run(1)
+        engs[0].load_state(engs[0].save_state())
+        with Batch(engs, group=group) as b:
+            b.set_tiling(8, 4, 1, group, per_launch=per_launch)
+            b.run(6)
+            b.run(5)
+            engs[1].field("Hx")
+            b.run(STEPS - 12)
+        for w, e in zip(want, engs):
+            _assert_same(w, _state(e))
+    finally:
+        for e in engs:
+            e.close()
