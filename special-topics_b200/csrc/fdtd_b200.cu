@@ -479,7 +479,6 @@ int enqueue_steps(fdtd_ctx* c, const C& coef, int count, KernelTimer* tm = nullp
   const unsigned mid_blocks = (unsigned)((plane + pr.n_i + 255) / 256);
   const long long nff = (c->nFreq > 0) ? c->ffsz[0] + c->ffsz[1] + c->ffsz[2] : 0;
   const unsigned epi_blocks = (unsigned)((nff + pr.n_v + 255) / 256);
-  const unsigned flush_blocks = (unsigned)((nff * std::max(c->nFreq, 1) + 255) / 256);
   auto kh = step_kernel<T, C, EXACT>(false, c->prefetch);
   auto ke = step_kernel<T, C, EXACT>(true, c->prefetch);
   size_t smem = 0;
@@ -495,7 +494,7 @@ int enqueue_steps(fdtd_ctx* c, const C& coef, int count, KernelTimer* tm = nullp
     ke<<<grd, blk, smem, st>>>(p);
     if (tm) CK(cudaEventRecord(tm->ev[3], st));
     if (epi_blocks) k_epilogue<T><<<epi_blocks, 256, 0, st>>>(p.f, p.g, ff, pr, c->d_ts);
-    if (c->dft_block > 0) k_dft_flush<<<flush_blocks, 256, 0, st>>>(ff, c->d_ts, -1);
+    if (c->dft_block > 0) CK(dft_flush(ff, c->d_ts, -1, st));
     if (tm) {
       CK(cudaEventRecord(tm->ev[4], st));
       CK(cudaEventSynchronize(tm->ev[4]));
@@ -1059,9 +1058,9 @@ int fused_enqueue_steps(fdtd_ctx* c, int count, int flip, int ts, KernelTimer* t
   // the epilogue of step `step`, under the parameters of the step after it or its own
   auto epilogue = [&](const FusedParams<T>& p, int step, bool late) -> cudaError_t {
     if (!epi) return cudaSuccess;
-    const cudaError_t e = fused_epilogue<T>(p, ff, pr, epi, late, alone, st);
+    cudaError_t e = fused_epilogue<T>(p, ff, pr, epi, late, alone, st);
     if (e == cudaSuccess && c->dft_block > 0 && (step + 1) % c->dft_block == 0)
-      k_dft_flush<<<(unsigned)((pts * c->nFreq + 255) / 256), 256, 0, st>>>(ff, late ? p.ts : p.ts_next, -2);
+      e = dft_flush(ff, late ? p.ts : p.ts_next, -2, st);
     return e;
   };
   for (int s = 0; s < count; s++, flip ^= 1) {
@@ -1111,11 +1110,7 @@ int enqueue(fdtd_ctx* c, int count, KernelTimer* tm = nullptr, cudaStream_t st =
 // what the run left buffered (the open block) and mark it done.
 int close_dft_block(fdtd_ctx* c, int upto, cudaStream_t st) {
   if (c->dft_block <= 0) return FDTD_OK;
-  if (upto % c->dft_block != 0) {
-    const long long n = (c->ffsz[0] + c->ffsz[1] + c->ffsz[2]) * (long long)c->nFreq;
-    k_dft_flush<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(dev_ff(c), c->d_ts, upto);
-    CK(cudaGetLastError());
-  }
+  if (upto % c->dft_block != 0) CK(dft_flush(dev_ff(c), c->d_ts, upto, st));
   CK(cudaMemcpyAsync(c->d_dft_done, &upto, sizeof(int), cudaMemcpyHostToDevice, st));
   CK(cudaStreamSynchronize(st));  // `upto` is read from this frame
   return FDTD_OK;
@@ -2550,7 +2545,7 @@ int batch_prepare(fdtd_batch* b, C (*coef_of)(fdtd_ctx*)) {
     const long long nff = (c->nFreq > 0) ? c->ffsz[0] + c->ffsz[1] + c->ffsz[2] : 0;
     for (long long s = 0; s < (nff + in.pr.n_v + 255) / 256; s++) epi.push_back(BatchBlock{q, (int)s});
     if (c->dft_block > 0)
-      for (long long s = 0; s < (nff * c->nFreq + 255) / 256; s++) flush.push_back(BatchBlock{q, (int)s});
+      for (long long s = 0; s < flush_blocks(nff, c->nFreq); s++) flush.push_back(BatchBlock{q, (int)s});
   }
   if (tiles.size() > (size_t)INT32_MAX) return fail(FDTD_ERR_BADARG, "batch has too many tiles");
   if (b->members_per_launch > 0) {

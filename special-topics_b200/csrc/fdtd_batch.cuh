@@ -161,14 +161,17 @@ __global__ void __launch_bounds__(256)
   epilogue_thread<T>(in.sp.f, in.sp.g, in.ff, in.pr, *in.sp.ts, (long long)b.local * blockDim.x + threadIdx.x);
 }
 
-// Time-blocked DFT flush of every member (see k_dft_flush).
+// Time-blocked DFT flush of every member (see dft_flush).
 template <typename T, class C>
 __global__ void __launch_bounds__(256)
     k_batch_flush(const Instance<T, C>* __restrict__ inst, const BatchBlock* __restrict__ blocks, int upto) {
   const BatchBlock b = blocks[blockIdx.x];
   const Instance<T, C>& in = inst[b.inst];
-  if (flush_upto(in.ff, in.sp.ts, upto))
-    dft_flush_thread(in.ff, upto, (long long)b.local * blockDim.x + threadIdx.x);
+  if (!flush_upto(in.ff, in.sp.ts, upto)) return;
+  if (in.ff.kahan)
+    dft_flush_any<true>(in.ff, upto, b.local);
+  else
+    dft_flush_any<false>(in.ff, upto, b.local);
 }
 
 }  // namespace fdtd

@@ -1,6 +1,7 @@
 // fdtd_common.cuh -- shared device types and the per-step epilogue (port
 // voltages + running far-field DFT) used by every field layout.
 #pragma once
+#include <type_traits>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -91,8 +92,8 @@ struct FarField {
   long long off[24];
   long long sz[3];             // x-, y-, z-face point counts
   int kahan;                   // accumulators are FP32 (sum, compensation) pairs, not FP64
-  int block;                   // > 0: steps per time block (samples buffered, accumulated by k_dft_flush)
-  float* samples;              // [block][points][8] surface samples of the open block
+  int block;                   // > 0: steps per time block (samples buffered, accumulated by dft_flush)
+  float* samples;              // [block][8][points] surface samples of the open block
   const int* done;             // steps already accumulated
 };
 
@@ -191,9 +192,9 @@ __device__ __forceinline__ int sample_array(int group, int a) {
 // ts % block; this writes them into the running accumulators.
 __device__ __forceinline__ void store_samples(const FarField& ff, long long t, int ts, const double* v) {
   const long long npts = ff.sz[0] + ff.sz[1] + ff.sz[2];
-  float4* s = reinterpret_cast<float4*>(ff.samples + ((long long)(ts % ff.block) * npts + t) * 8);
-  s[0] = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
-  s[1] = make_float4((float)v[4], (float)v[5], (float)v[6], (float)v[7]);
+  float* s = ff.samples + (long long)(ts % ff.block) * 8 * npts + t;
+#pragma unroll
+  for (int a = 0; a < 8; a++) s[a * npts] = (float)v[a];
 }
 
 // One Kahan-compensated FP32 step: v = (sum, compensation), sum += x.
@@ -331,7 +332,7 @@ __device__ __forceinline__ void epilogue_thread(const Fields<T>& f, const G& g, 
     v[6] = mul(0.25, add(add(add(HY(i0, j0, LK), HY(i0, j0 + 1, LK)), HY(i0, j0, LK - 1)), HY(i0, j0 + 1, LK - 1)));
     v[7] = mul(-0.25, add(add(add(HX(i0, j0, LK), HX(i0 + 1, j0, LK)), HX(i0, j0, LK - 1)), HX(i0 + 1, j0, LK - 1)));
   }
-  if (ff.block)  // time-blocked: buffer the samples, k_dft_flush accumulates them
+  if (ff.block)  // time-blocked: buffer the samples, dft_flush accumulates them
     store_samples(ff, t, ts, v);
   else
     accumulate(ff, group, pt, ts, v);
@@ -351,40 +352,97 @@ __global__ void __launch_bounds__(256) k_epilogue(Fields<T> f, GridDims g, FarFi
 
 // Accumulates the buffered samples of the steps before `upto` that are not in
 // the running DFT yet (from the block's first step, or *ff.done when a run
-// started inside the block): one thread per (surface point pair, frequency),
-// steps in order.
-__device__ __forceinline__ void dft_flush_thread(const FarField& ff, int upto, long long q) {
+// started inside the block), steps in order.
+//
+// A block holds the accumulators of 32 surface points and NF frequencies in
+// registers over all those steps (a warp per sample array, a point a thread), so
+// an accumulator is read and written once and a sample is read once per NF
+// frequencies; the phasors of kFlushSteps steps wait in shared memory.  One
+// thread per (point, frequency), which read every sample and phasor again for
+// each frequency, was bound by those loads: 16 steps of 93 k point pairs at 64
+// frequencies took 888 us, now 341 us (of which the accumulators' own traffic is
+// 235 us).  Two points a thread, or 4 or 16 frequencies, leave too few warps or
+// loads in flight (484, 460, 371 us); few frequencies take a smaller NF, whose
+// blocks need fewer registers.
+constexpr int kFlushPoints = 32, kFlushSteps = 32;
+__host__ __device__ inline int flush_freqs(int freqs) { return freqs <= 2 ? 2 : freqs <= 4 ? 4 : 8; }  // NF
+__host__ __device__ inline long long flush_blocks(long long points, int freqs) {
+  const int nf = flush_freqs(freqs);
+  return (points + kFlushPoints - 1) / kFlushPoints * ((freqs + nf - 1) / nf);
+}
+
+template <bool KAHAN, int NF>
+__device__ __forceinline__ void dft_flush_block(const FarField& ff, int upto, long long b) {
+  using A = std::conditional_t<KAHAN, float2, double>;   // an accumulator
+  using P = std::conditional_t<KAHAN, float2, double2>;  // a phasor
+  __shared__ P ph[kFlushSteps][NF][2];          // H-time, E-time
   const long long npts = ff.sz[0] + ff.sz[1] + ff.sz[2];
-  if (ff.block <= 0 || q >= npts * ff.nFreq) return;
-  const int from = max(*ff.done, (upto - 1) / ff.block * ff.block);
-  const long long t = q % npts;
-  const int m = (int)(q / npts);
+  const int chunks = (ff.nFreq + NF - 1) / NF;
+  const int m0 = (int)(b % chunks) * NF, nf = min(NF, ff.nFreq - m0);
+  const int a = threadIdx.x / 32;
+  const int first = (upto - 1) / ff.block * ff.block, from = max(*ff.done, first);
+  const long long t = b / chunks * kFlushPoints + threadIdx.x % 32;
+  const bool has = t < npts;
   const int group = t < ff.sz[0] ? 0 : t < ff.sz[0] + ff.sz[1] ? 1 : 2;
-  const long long p = (long long)m * ff.sz[group] + (group == 0 ? t : group == 1 ? t - ff.sz[0] : t - ff.sz[0] - ff.sz[1]);
-  for (int a = 0; a < 8; a++) {
-    const int arr = sample_array(group, a);
-    const int e = arr >= CMYXP ? 2 : 0;  // magnetic currents take the E-time phasor
-    double* re = ff.acc + ff.off[arr] + p;
-    double* im = re + ff.nFreq * ff.sz[group];
-    if (ff.kahan) {
-      for (int s = from; s < upto; s++) {
-        const double* ph = ff.ph + ((long long)s * ff.nFreq + m) * 4 + e;
-        const float v = ff.samples[((long long)(s % ff.block) * npts + t) * 8 + a];
-        kahan_add(reinterpret_cast<float2*>(re), __fmul_rn((float)ph[0], v));
-        kahan_add(reinterpret_cast<float2*>(im), __fmul_rn((float)ph[1], v));
+  const long long sz = ff.sz[group];
+  A* const acc = reinterpret_cast<A*>(ff.acc + ff.off[sample_array(group, a)]) + m0 * sz +
+                 (group == 0 ? t : group == 1 ? t - ff.sz[0] : t - ff.sz[0] - ff.sz[1]);
+  A re[NF], im[NF];
+#pragma unroll
+  for (int f = 0; f < NF; f++)
+    if (has && f < nf) {
+      re[f] = acc[f * sz];
+      im[f] = acc[(ff.nFreq + f) * sz];
+    }
+  const int e = (a & 2) == 0;  // magnetic currents take the E-time phasor
+  for (int s0 = from; s0 < upto; s0 += kFlushSteps) {
+    const int ns = min(kFlushSteps, upto - s0);
+    __syncthreads();
+    for (int w = threadIdx.x; w < ns * NF * 2; w += 256) {
+      const int s = w / (2 * NF), f = w / 2 % NF;
+      if (f < nf) {
+        const double* src = ff.ph + ((long long)(s0 + s) * ff.nFreq + m0 + f) * 4 + w % 2 * 2;
+        ph[s][f][w % 2].x = src[0];
+        ph[s][f][w % 2].y = src[1];
       }
-    } else {
-      double r = *re, i = *im;
-      for (int s = from; s < upto; s++) {
-        const double* ph = ff.ph + ((long long)s * ff.nFreq + m) * 4 + e;
-        const double v = ff.samples[((long long)(s % ff.block) * npts + t) * 8 + a];
-        r += ph[0] * v;
-        i += ph[1] * v;
-      }
-      *re = r;
-      *im = i;
+    }
+    __syncthreads();
+    const float* smp = ff.samples + ((long long)(s0 - first) * 8 + a) * npts + t;
+#pragma unroll 8
+    for (int s = 0; s < ns; s++) {
+      const float v = has ? smp[s * 8 * npts] : 0.0f;
+#pragma unroll
+      for (int f = 0; f < NF; f++)
+        if (f < nf) {
+          const P c = ph[s][f][e];
+          if constexpr (KAHAN) {
+            kahan_add(&re[f], __fmul_rn(c.x, v));
+            kahan_add(&im[f], __fmul_rn(c.y, v));
+          } else {
+            re[f] += c.x * v;
+            im[f] += c.y * v;
+          }
+        }
     }
   }
+#pragma unroll
+  for (int f = 0; f < NF; f++)
+    if (has && f < nf) {
+      acc[f * sz] = re[f];
+      acc[(ff.nFreq + f) * sz] = im[f];
+    }
+}
+
+// With NF as flush_blocks counts the blocks.
+template <bool KAHAN>
+__device__ __forceinline__ void dft_flush_any(const FarField& ff, int upto, long long b) {
+  const int nf = flush_freqs(ff.nFreq);
+  if (nf == 2)
+    dft_flush_block<KAHAN, 2>(ff, upto, b);
+  else if (nf == 4)
+    dft_flush_block<KAHAN, 4>(ff, upto, b);
+  else
+    dft_flush_block<KAHAN, 8>(ff, upto, b);
 }
 
 // The steps a flush covers: upto >= 0, the end of a run (nothing to do when a
@@ -398,8 +456,25 @@ __device__ __forceinline__ bool flush_upto(const FarField& ff, const int* ts_ptr
   return upto % ff.block == 0;
 }
 
+// 256 threads; flush_blocks() of them.
+template <bool KAHAN, int NF>
 static __global__ void __launch_bounds__(256) k_dft_flush(FarField ff, const int* ts_ptr, int upto) {
-  if (flush_upto(ff, ts_ptr, upto)) dft_flush_thread(ff, upto, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+  if (flush_upto(ff, ts_ptr, upto)) dft_flush_block<KAHAN, NF>(ff, upto, blockIdx.x);
+}
+template <int NF>
+cudaError_t dft_flush_launch(const FarField& ff, const int* ts_ptr, int upto, cudaStream_t st) {
+  const unsigned n = (unsigned)flush_blocks(ff.sz[0] + ff.sz[1] + ff.sz[2], ff.nFreq);
+  if (ff.kahan)
+    k_dft_flush<true, NF><<<n, 256, 0, st>>>(ff, ts_ptr, upto);
+  else
+    k_dft_flush<false, NF><<<n, 256, 0, st>>>(ff, ts_ptr, upto);
+  return cudaGetLastError();
+}
+inline cudaError_t dft_flush(const FarField& ff, const int* ts_ptr, int upto, cudaStream_t st) {
+  const int nf = flush_freqs(ff.nFreq);
+  return nf == 2 ? dft_flush_launch<2>(ff, ts_ptr, upto, st)
+         : nf == 4 ? dft_flush_launch<4>(ff, ts_ptr, upto, st)
+                   : dft_flush_launch<8>(ff, ts_ptr, upto, st);
 }
 
 }  // namespace fdtd

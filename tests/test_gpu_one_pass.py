@@ -150,3 +150,22 @@ def test_batch_chains_match_members_alone(blocks, group, per_launch):
     finally:
         for e in engs:
             e.close()
+
+
+@pytest.mark.parametrize("freqs,block,runs", [(1, 2, (5, 18)), (3, 6, (8, 15)), (7, 4, (4, 19)), (8, 33, (23,)), (9, 5, (1, 1, 21)), (17, 7, (9, 14))])
+def test_blocked_dft_sums_in_step_order(freqs, block, runs):
+    """Compensated FP32 sums are the same bits whether a step's samples are
+    added at once or with their block: frequency groups of 8 full and ragged,
+    point groups of 32 ragged, blocks closed by a run's end, longer than a run
+    and longer than the phasors staged at a time."""
+    scn, _ = _problem(SHAPES[1])
+    scn["farfield"]["frequencies"] = [1e9 * (2 + q) for q in range(freqs)]
+    p = build_problem_from_scenario(scn, STEPS)
+    out = []
+    for b in (0, block):
+        with Engine(p, "f32-table", dft_accumulator="kahan-f32", dft_block=b) as eng:
+            for n in runs:
+                eng.run(n)
+            out.append(eng.farfield())
+    for a in FF_NAMES:
+        assert np.array_equal(out[0][a][0], out[1][a][0]) and np.array_equal(out[0][a][1], out[1][a][1]), a
