@@ -57,7 +57,9 @@ def algorithmic_bytes(p, precision: str) -> dict:
     """Compulsory DRAM bytes of one H and one E launch: each own-field value read
     and written once, each other-field value read once, the per-cell coefficient
     data read once (3 one-byte ids, or 3 FP64 arrays), each Psi element read and
-    written once (plus its CPsi for the per-cell layout)."""
+    written once (plus its CPsi for the per-cell layout).  "step": of the
+    one-pass step's launch: each field and Psi value read and written once, and
+    a two-byte class per cell."""
     sh = p.grid.shapes
     nH = sum(int(np.prod(sh[c])) for c in ("Hx", "Hy", "Hz"))
     nE = sum(int(np.prod(sh[c])) for c in ("Ex", "Ey", "Ez"))
@@ -71,7 +73,21 @@ def algorithmic_bytes(p, precision: str) -> dict:
     # bytes per component value: field word, coefficient data, Psi traffic per Psi element
     w, coef, psi_w = {"f32-table": (4, 1, 8), "f32": (4, 12, 12), "f64": (8, 24, 24)}[precision]
     return {"h": nH * (2 * w + coef) + nE * w + psi_m * psi_w,
-            "e": nE * (2 * w + coef) + nH * w + psi_e * psi_w}
+            "e": nE * (2 * w + coef) + nH * w + psi_e * psi_w,
+            "step": 2 * w * (nH + nE + psi_m + psi_e) + 2 * (p.grid.nx + 1) * (p.grid.ny + 1) * (p.grid.nz + 1)}
+
+
+def one_pass(kern: dict) -> bool:
+    """Whether a profile is of the one-pass step, which has no E launch."""
+    return kern["e"] == 0.0
+
+
+def dominant(kern: dict, byts: dict) -> tuple:
+    """(name, algorithmic bytes, ms) of the step's longest launch."""
+    if one_pass(kern):
+        return "k_fused", byts["step"], kern["h"]
+    dom = "e" if kern["e"] >= kern["h"] else "h"
+    return f"k_step_{dom}", byts[dom], kern[dom]
 
 
 def _psi_sizes(p, f):
@@ -366,9 +382,9 @@ def main():
     eng.close()
     value = world * cells * K / (ms / 1e3) / 1e9
     byts = algorithmic_bytes(prob, args.precision)
-    dom = "e" if kern["e"] >= kern["h"] else "h"
+    dom, dom_bytes, dom_ms = dominant(kern, byts)
     peak, peak_kind = hbm_peak()
-    achieved = byts[dom] / (kern[dom] / 1e3) / 1e9
+    achieved = dom_bytes / (dom_ms / 1e3) / 1e9
     traffic = ncu_traffic(workload)
     line = {
         "metric": METRIC, "value": value, "unit": "Gcell-updates/s", "n_gpus": world, "steps": K, "warmup": W,
@@ -380,16 +396,19 @@ def main():
                   "far_field_dft": f"time-blocked, {dft_block} steps per block" if dft_block else "every step",
                   "x_wall": "Ey, Ez at i = nx held at zero (FP32 default)" if args.precision != "f64"
                             else "the reference's reads at i = nx"},
-        "roofline": {"bound": "hbm", "kernel": f"k_step_{dom}", "achieved": achieved, "peak": peak,
+        "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
                      "frac_of_nominal_8TBs": achieved / NOMINAL_HBM_GBS,
-                     "algorithmic_bytes_per_launch": byts[dom], "launch_ms": kern[dom],
+                     "algorithmic_bytes_per_launch": dom_bytes, "launch_ms": dom_ms,
                      "traffic": traffic},
         "kernel_ms": kern,
         "tiling": {k: tuning.get(k, 32 if k == "width" else None) for k in ("chunk", "rows", "prefetch", "width", "ms_per_step")}
                   if tuning else "default",
         "clocks": clk.summary(),
-        "gpu_launches": (5 if dft_block else 4) * K,   # H, mid, E, epilogue (+ the DFT flush)
+        # H, mid, E, epilogue (+ the DFT flush); one-pass: the step, its epilogue, the wall where the reference's
+        # reads are kept, and a flush per block
+        "gpu_launches": ((3 if args.precision == "f64" else 2) * K + (K // dft_block if dft_block else 0)
+                         if one_pass(kern) else (5 if dft_block else 4) * K),
         "e2e": e2e,
         "setup_s": setup_s,
     }
@@ -502,8 +521,8 @@ def _best_by_mode(table: list) -> dict:
 def batched_side(problems, K: int = 1000, W: int = 8, tune_steps: int = 16, device: int = 0,
                  barrier=lambda: None, fixed: str | None = None, dft_block: int = 0) -> dict:
     """The batched sweep (FP32 fields, material tables): every member advanced
-    either by one set of four launches per step for the whole batch (tile-list
-    mode) or by its own four kernels per step on worker streams inside one
+    by its own one-pass steps as a chain, by one set of four launches per step for
+    the whole batch (tile-list mode) or by its own four kernels per step on worker streams inside one
     graph (member-kernel mode); mode and launch shape from the batch
     autotuner."""
     from special_topics_b200 import autotune
@@ -531,14 +550,16 @@ def batched_side(problems, K: int = 1000, W: int = 8, tune_steps: int = 16, devi
     finally:
         for e in engs:
             e.close()
-    byts = {"h": 0, "e": 0}
+    byts = {"h": 0, "e": 0, "step": 0}
     for p in problems:
-        a = algorithmic_bytes(p, "f32-table")
-        byts["h"] += a["h"]
-        byts["e"] += a["e"]
+        for k, v in algorithmic_bytes(p, "f32-table").items():
+            byts[k] += v
     dom = "e" if kern["e"] >= kern["h"] else "h"
     peak, peak_kind = hbm_peak()
-    if tiling.get("streams", 0) > 0:
+    if one_pass(kern):
+        roof_kernel = "k_fused of every member, chains side by side (whole step)"
+        roof_bytes, roof_ms = byts["step"], ms / K
+    elif tiling.get("streams", 0) > 0:
         # member-kernel mode: the members' launches overlap on the worker
         # streams, so a launch timed alone says little; the roofline is the
         # whole step's H and E algorithmic bytes over the measured step time
@@ -680,12 +701,12 @@ def _leg(p, precision: str, K: int, W: int, tiling: dict | None, device: int = 0
         kern = eng.profile_kernels(8)
     byts = algorithmic_bytes(p, precision)
     peak, peak_kind = hbm_peak()
-    dom = "e" if kern["e"] >= kern["h"] else "h"
-    ach = byts[dom] / (kern[dom] / 1e3) / 1e9
+    dom, dom_bytes, dom_ms = dominant(kern, byts)
+    ach = dom_bytes / (dom_ms / 1e3) / 1e9
     return {"precision": precision, "value": p.grid.cells * K / (ms / 1e3) / 1e9, "unit": "Gcell-updates/s",
             "steps": K, "ms_per_step": ms / K, "kernel_ms": kern,
-            "roofline": {"kernel": f"k_step_{dom}", "achieved": ach, "peak": peak, "peak_kind": peak_kind,
-                         "frac": ach / peak, "algorithmic_bytes_per_launch": byts[dom]}}
+            "roofline": {"kernel": dom, "achieved": ach, "peak": peak, "peak_kind": peak_kind,
+                         "frac": ach / peak, "algorithmic_bytes_per_launch": dom_bytes}}
 
 
 def scaling_sweep_side(tiling32: dict | None, tiling64: dict | None, device: int = 0, dft_block: int = 0,
@@ -783,11 +804,11 @@ def fp64_side(pkg, n=(256, 256, 256), K: int = 300, W: int = 8) -> dict:
     eng.close()
     byts = algorithmic_bytes(p, "f64")
     peak, _ = hbm_peak()
-    dom = "e" if kern["e"] >= kern["h"] else "h"
-    ach = byts[dom] / (kern[dom] / 1e3) / 1e9
+    dom, dom_bytes, dom_ms = dominant(kern, byts)
+    ach = dom_bytes / (dom_ms / 1e3) / 1e9
     return {"workload": f"scaling-box-{n[0]}x{n[1]}x{n[2]}", "value": p.grid.cells * K / (ms / 1e3) / 1e9,
             "unit": "Gcell-updates/s", "ms_per_step": ms / K, "tiling": {k: tuning[k] for k in ("chunk", "rows", "prefetch")},
-            "roofline": {"kernel": f"k_step_{dom}", "achieved": ach, "peak": peak, "frac": ach / peak}}
+            "roofline": {"kernel": dom, "achieved": ach, "peak": peak, "frac": ach / peak}}
 
 
 if __name__ == "__main__":

@@ -189,9 +189,8 @@ int fdtd_ctx_run(fdtd_ctx* ctx, int count);
  * `block_rows` (1, 2, 4, 8 or 16) along j, in whole warps of at most 256
  * threads (checked at the next run).  Any shape gives the same results; the
  * autotuner (special-topics_b200/autotune.py) picks the fastest per grid.
- * A problem that runs the one-pass step (csrc/fdtd_fused.cuh) alone uses only
- * the x planes, as the length of a block's chunk; without a call it picks its
- * own.  The rest is the shape of the half-step kernels. */
+ * It is the shape of the half-step kernels: the one-pass step (csrc/
+ * fdtd_fused.cuh), which most problems run, picks its own. */
 int fdtd_ctx_set_tiling(fdtd_ctx* ctx, int x_planes_per_thread, int block_rows);
 int fdtd_ctx_get_tiling(const fdtd_ctx* ctx, int* x_planes_per_thread, int* block_rows);
 int fdtd_ctx_set_block_width(fdtd_ctx* ctx, int threads_along_k);
@@ -208,8 +207,8 @@ int fdtd_ctx_set_prefetch(fdtd_ctx* ctx, int planes);
 int fdtd_ctx_run_timed(fdtd_ctx* ctx, int count, float* ms);
 /* Runs `count` steps one at a time with CUDA events around every launch and
  * returns the mean duration (ms) of the H, mid-step, E and epilogue kernels;
- * of the whole step, the x = max wall, nothing and the epilogue where the
- * one-pass step runs. */
+ * of the whole step, the x = max wall (0 where it is held), 0 and the epilogue
+ * where the one-pass step runs. */
 int fdtd_ctx_profile_kernels(fdtd_ctx* ctx, int count, double* avg_ms);
 /* Current step index (number of completed steps). */
 int fdtd_ctx_step(const fdtd_ctx* ctx);

@@ -169,7 +169,6 @@ struct fdtd_ctx {
   // launch shape of the step kernels: x planes per thread, thread rows per block
   int ichunk = 1, block_rows = 8, prefetch = 1;
   int block_w = 32;   // threads of a block along k (32: a warp is one row; 16: a warp spans two rows)
-  bool chunk_set = false;   // x planes per thread chosen by the caller
   FusedState fs;
   bool dense_valid = true;  // `fields` and the faces' Psi hold the current state
   // graph cache
@@ -948,10 +947,6 @@ void fused_shape(const fdtd_ctx* c, FusedParams<T>& p, double share) {
   slow(p.axis[1], kTileRows - 1, p.tj, p.slow_j);
   slow(p.axis[2], (p.rk - p.halo_k) * V, p.tk, p.slow_k);
   const int nxp = c->nx + 1;
-  if (c->chunk_set && share == 1) {
-    p.tx = (nxp + c->ichunk - 1) / c->ichunk;
-    return;
-  }
   // Blocks of the three kinds that fused_place orders, per x chunk, and their
   // time per plane: the device takes them in that order, a free slot the next.
   const int nj = p.slow_j[0] + p.slow_j[1], nk = p.slow_k[0] + p.slow_k[1];
@@ -1080,6 +1075,7 @@ int fused_enqueue_steps(fdtd_ctx* c, int count, int flip, int ts, KernelTimer* t
       CK(cudaEventRecord(tm->ev[4], st));
       CK(cudaEventSynchronize(tm->ev[4]));
       for (int q = 0; q < 4; q++) {
+        if (q == 2 || (q == 1 && p.x_wall)) continue;  // no launch
         float ms = 0;
         CK(cudaEventElapsedTime(&ms, tm->ev[q], tm->ev[q + 1]));
         tm->ms[q] += ms;
@@ -1986,7 +1982,6 @@ int fdtd_ctx_set_tiling(fdtd_ctx* c, int x_planes_per_thread, int block_rows) {
     return fail(FDTD_ERR_BADARG, "block rows %d not in {1,2,4,8,16}", block_rows);
   c->ichunk = x_planes_per_thread;
   c->block_rows = block_rows;
-  c->chunk_set = true;
   invalidate(c);
   return FDTD_OK;
 }

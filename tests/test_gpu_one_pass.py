@@ -13,7 +13,6 @@ from conftest import load_package
 from scenarios_small import small_scenario
 
 pkg = load_package()
-from special_topics_b200 import _native as N  # noqa: E402
 from special_topics_b200.backend import Batch, Engine  # noqa: E402
 from special_topics_b200.scenario import FF_NAMES, build_problem_from_scenario  # noqa: E402
 
@@ -108,17 +107,23 @@ def test_fp32_one_pass_matches_half_steps(shape, precision):
             _assert_same(want, _state(eng))
 
 
-@pytest.mark.parametrize("planes", [1, 2, 3, 5, 8, 26])
-def test_chunks_of_any_length_match(planes):
-    _, p = _problem(SHAPES[4])
-    states = []
-    for n in (None, planes):
-        with Engine(p, "f32-table") as eng:
-            if n:
-                N.check(N.lib().fdtd_ctx_set_tiling(eng._h, n, 8))
-            eng.run(STEPS)
-            states.append(_state(eng))
-    _assert_same(*states)
+@pytest.mark.parametrize("members", [2, 5, 24])
+def test_chunks_of_any_length_match(members):
+    """A member's share of the device, and so the x planes of its blocks, depends
+    on how many there are."""
+    _, p = _problem(SHAPES[6])
+    with Engine(p, "f32-table") as eng:
+        eng.run(STEPS)
+        want = _state(eng)
+    engs = [Engine(p, "f32-table") for _ in range(members)]
+    try:
+        with Batch(engs) as b:
+            b.run(STEPS)
+        for e in (engs[0], engs[-1]):
+            _assert_same(want, _state(e))
+    finally:
+        for e in engs:
+            e.close()
 
 
 @pytest.mark.parametrize("blocks", [(0, 0, 0), (4, 4, 4), (0, 4, 3)], ids=str)
