@@ -2294,6 +2294,53 @@ int fdtd_dft(const double* x, int N, double dt, const double* freqs, int M, doub
   return rc;
 }
 
+// A run of directions [a0, a1) of a far-field call and the distinct values among
+// their thetas, [t0, t1) of the call's list.
+struct FFRun {
+  int a0, a1, t0, t1;
+};
+
+// Cuts the directions into runs of at most `most` distinct thetas; cth: their
+// cosines, ith: each direction's place among its run's.
+static std::vector<FFRun> ff_runs(const double* theta, int nang, int most, std::vector<double>* cth,
+                                  std::vector<int>* ith) {
+  size_t slots = 16;
+  while (slots < 2 * (size_t)std::min(most, nang)) slots *= 2;
+  std::vector<int> slot(slots, -1);
+  std::vector<double> val;  // of the current run
+  std::vector<FFRun> runs;
+  cth->clear();
+  ith->resize(nang);
+  auto cut = [&](int a1) {
+    const int a0 = runs.empty() ? 0 : runs.back().a1, t0 = (int)cth->size();
+    for (double t : val) cth->push_back(cos(t));
+    runs.push_back({a0, a1, t0, (int)cth->size()});
+    val.clear();
+    std::fill(slot.begin(), slot.end(), -1);
+  };
+  for (int q = 0; q < nang; q++) {
+    unsigned long long bits;
+    memcpy(&bits, theta + q, sizeof(bits));
+    size_t h = 0;
+    auto find = [&] {
+      h = (bits * 0x9E3779B97F4A7C15ull >> 32) & (slots - 1);
+      while (slot[h] >= 0 && memcmp(&val[slot[h]], &bits, sizeof(bits))) h = (h + 1) & (slots - 1);
+      return slot[h] >= 0;
+    };
+    if (!find()) {
+      if ((int)val.size() >= most) {
+        cut(q);
+        find();
+      }
+      slot[h] = (int)val.size();
+      val.push_back(theta[q]);
+    }
+    (*ith)[q] = slot[h];
+  }
+  if (nang > 0) cut(nang);
+  return runs;
+}
+
 int fdtd_ctx_farfield_post(fdtd_ctx* c, const double* theta, const double* phi, int nang, double* radp,
                            double* d_theta, double* d_phi) {
   if (!c || !radp || (nang > 0 && (!theta || !phi || !d_theta || !d_phi)) || nang < 0)
@@ -2325,45 +2372,79 @@ int fdtd_ctx_farfield_post(fdtd_ctx* c, const double* theta, const double* phi, 
     P.face[a][1] = (lo[a] - centre) * d[a];
   }
   const int F = c->nFreq;
-  double *dfreq = nullptr, *dradp = nullptr, *dang = nullptr, *dout = nullptr;
+  const size_t na = (size_t)nang;
+  const size_t R = 2 * (size_t)(P.ni + P.nj);
+  std::vector<double> cth;
+  std::vector<int> ith;
+  std::vector<FFRun> runs;
+  // one buffer: frequencies, radiated power, angles, results, then the row sums
+  // of one run of directions, for as many frequencies as fit `room` values; with
+  // less memory left, shorter runs and fewer frequencies at a time
+  const size_t n_out = 8 * (size_t)F + 2 * na + 2 * F * na;
+  size_t n_rows = 0, n_z = 0;
+  int parts = 1, fb = 1;
+  double* buf = nullptr;
   int rc = FDTD_OK;
-  const size_t na = (size_t)std::max(nang, 1);
-  if (cudaMalloc(&dfreq, F * sizeof(double)) != cudaSuccess || cudaMalloc(&dradp, F * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&dang, 2 * na * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&dout, 2 * F * na * sizeof(double)) != cudaSuccess) {
-    rc = fail(FDTD_ERR_OOM, "far-field post buffers");
-  }
-  cudaError_t e = cudaSuccess;
-  if (!rc) {
-    e = cudaMemcpyAsync(dfreq, c->ffreq.data(), F * sizeof(double), cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess && nang > 0)
-      e = cudaMemcpyAsync(dang, theta, nang * sizeof(double), cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess && nang > 0)
-      e = cudaMemcpyAsync(dang + na, phi, nang * sizeof(double), cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) {
-      k_ff_power<<<F, 256, 0, c->stream>>>(P, dradp);
-      if (nang > 0) {
-        const dim3 grd((nang + 256 * kFFAng - 1) / (256 * kFFAng), F);
-        k_ff_pattern<<<grd, 256, 0, c->stream>>>(P, dfreq, dang, dang + na, nang, dradp, dout, dout + F * na);
+  for (size_t room = (size_t)128 << 20; !buf; room /= 8) {
+    const int most = (int)std::max<size_t>(64, std::min<size_t>(1 << 20, room / 2 / (8 * R)));
+    runs = ff_runs(theta, nang, most, &cth, &ith);
+    int ang = 0, th = 0;
+    for (const FFRun& u : runs) {
+      ang = std::max(ang, u.a1 - u.a0);
+      th = std::max(th, u.t1 - u.t0);
+    }
+    // z-face rows in parts, for some eight blocks of k_ff_zrows a multiprocessor
+    const int ztiles = ang / (kFFZThreads * kFFZAng) + 1;
+    parts = std::max(1, std::min(P.ni, 8 * 148 / (ztiles * F)));
+    n_rows = R * 8 * th;
+    n_z = (size_t)parts * 8 * ang;
+    fb = (int)std::min<size_t>(F, std::max<size_t>(1, room / std::max<size_t>(1, n_rows + n_z)));
+    if (cudaMalloc(&buf, (n_out + fb * (n_rows + n_z) + cth.size() + na) * sizeof(double)) != cudaSuccess) {
+      cudaGetLastError();
+      buf = nullptr;
+      if (room < 65536) {
+        rc = fail(FDTD_ERR_OOM, "far-field post buffers");
+        break;
       }
+    }
+  }
+  if (!rc) {
+    double *dfreq = buf, *dradp = dfreq + F, *dpow = dradp + F, *dang = dpow + 6 * F, *dout = dang + 2 * na;
+    double *dth = dout + 2 * F * na, *drows = dth + cth.size(), *dz = drows + fb * n_rows;
+    int* dith = (int*)(dz + fb * n_z);
+    auto up = [&](void* d, const void* h, size_t bytes) {
+      return bytes ? cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, c->stream) : cudaSuccess;
+    };
+    cudaError_t e = up(dfreq, c->ffreq.data(), F * sizeof(double));
+    if (e == cudaSuccess) e = up(dang, theta, na * sizeof(double));
+    if (e == cudaSuccess) e = up(dang + na, phi, na * sizeof(double));
+    if (e == cudaSuccess) e = up(dth, cth.data(), cth.size() * sizeof(double));
+    if (e == cudaSuccess) e = up(dith, ith.data(), na * sizeof(int));
+    if (e == cudaSuccess) {
+      k_ff_power<<<dim3(F, 6), 256, 0, c->stream>>>(P, dpow);
+      k_ff_power_sum<<<(F + 127) / 128, 128, 0, c->stream>>>(dpow, F, dradp);
+      for (const FFRun& u : runs)
+        for (int f0 = 0; f0 < F; f0 += fb) {
+          const int per = kFFRowThreads * kFFRowAng, zper = kFFZThreads * kFFZAng, nth = u.t1 - u.t0, ang = u.a1 - u.a0;
+          const unsigned nf = (unsigned)std::min(fb, F - f0);
+          const FFSums W{f0,  nth,   dth + u.t0, dith + u.a0, dang + u.a0, dang + na + u.a0,
+                         ang, drows, dz,         parts};
+          k_ff_rows<<<dim3((nth + per - 1) / per, (unsigned)R, nf), kFFRowThreads, 0, c->stream>>>(P, W, dfreq);
+          k_ff_zrows<<<dim3((ang + zper - 1) / zper, parts, nf), kFFZThreads, 0, c->stream>>>(P, W, dfreq);
+          k_ff_pattern<<<dim3((ang + 127) / 128, nf), 128, 0, c->stream>>>(P, W, dfreq, dradp, (long long)na, dout + u.a0,
+                                                                          dout + F * na + u.a0);
+        }
       e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(radp, dradp, F * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess && nang > 0)
-      for (int f = 0; f < F && e == cudaSuccess; f++) {
-        e = cudaMemcpyAsync(d_theta + (size_t)f * nang, dout + f * na, nang * sizeof(double), cudaMemcpyDeviceToHost,
-                            c->stream);
-        if (e == cudaSuccess)
-          e = cudaMemcpyAsync(d_phi + (size_t)f * nang, dout + F * na + f * na, nang * sizeof(double),
-                              cudaMemcpyDeviceToHost, c->stream);
-      }
+      e = cudaMemcpyAsync(d_theta, dout, F * na * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess && nang > 0)
+      e = cudaMemcpyAsync(d_phi, dout + F * na, F * na * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) rc = fail(FDTD_ERR_CUDA, "far-field post: %s", cudaGetErrorString(e));
   }
-  cudaFree(dfreq);
-  cudaFree(dradp);
-  cudaFree(dang);
-  cudaFree(dout);
+  cudaFree(buf);
   cudaFree(conv);
   return rc;
 }

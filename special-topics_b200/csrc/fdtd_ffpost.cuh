@@ -10,11 +10,23 @@
 // vectors N = sum J exp(jk r'.r) dA and L = sum M exp(jk r'.r) dA over the six
 // faces, projected on theta/phi (farfield.js:328-607), then
 // D_theta = k^2 |L_phi + eta N_theta|^2 / (8 pi eta P_rad), and D_phi alike
-// with |L_theta - eta N_phi|^2.  Face points lie on a regular grid, so along
-// the fastest-varying point index the phase factor advances by one complex
-// multiply per point; one sincos starts each run of points.  Each block takes
-// one frequency and 512 directions (two per thread), staging the face points'
-// currents through shared memory so that every point is read once per block.
+// with |L_theta - eta N_phi|^2.
+//
+// Face points lie on a regular grid, so along a row of points the phase factor
+// advances by one complex multiply per point; one sincos starts each run.  The
+// points of a row are taken in pairs about its middle: with u and v the sum and
+// the difference of a pair's currents, the pair adds cos(x) u + j sin(x) v, half
+// the multiplications of two single points.  All of it is FP64 arithmetic on the
+// CUDA cores, and that bounds it, so the rows are summed where they need be:
+//   * along z the phase depends on theta alone.  The rows of the x and y faces
+//     run along z, so k_ff_rows sums each of them once per distinct theta, and
+//     a direction (k_ff_pattern) sums the row sums;
+//   * the rows of the z faces run along y, and k_ff_zrows sums them for every
+//     direction, both faces together as they share the phase in the plane.
+// Summing every point for every direction (4.4 ms for up to 2,000 directions,
+// 13.8 ms for 16,380, on a 13 x 110 x 110 box at 12 frequencies) was slower for
+// one direction (0.26 ms), for a 2-degree grid (2.4 ms, of which the kernels 1.3)
+// and for 16,000 directions without a theta in common (9.6 ms).
 #pragma once
 #include "fdtd_common.cuh"
 
@@ -54,37 +66,41 @@ __global__ void k_kahan_to_f64(const double* __restrict__ acc, double* __restric
   out[q] = (double)v.x - (double)v.y;
 }
 
-// Radiated power of every frequency: block f, fixed-order reduction.
-__global__ void __launch_bounds__(256) k_ff_power(FFPost P, double* __restrict__ radp) {
+// Radiated power: the sum of each face pair's points, a block per (frequency,
+// term), fixed-order reduction; k_ff_power_sum adds a frequency's terms.
+__global__ void __launch_bounds__(256) k_ff_power(FFPost P, double* __restrict__ part) {
   __shared__ double red[256];
-  const int f = blockIdx.x;
-  double s = 0.0;
+  const int f = blockIdx.x, t = blockIdx.y;
   // (face, area, M1, J1, M2, J2, sign) as farfield.js:257-325 pairs them
   const int terms[6][5] = {{CMYZP, CJXZP, CMXZP, CJYZP, 1},  {CMYZN, CJXZN, CMXZN, CJYZN, -1},
                            {CMXYP, CJZYP, CMZYP, CJXYP, 1},  {CMXYN, CJZYN, CMZYN, CJXYN, -1},
                            {CMZXP, CJYXP, CMYXP, CJZXP, 1},  {CMZXN, CJYXN, CMYXN, CJZXN, -1}};
-  const int ax[6] = {2, 2, 1, 1, 0, 0};
-  for (int t = 0; t < 6; t++) {
-    const int a = ax[t];
-    const long long n = P.sz[a];
-    const double area = a == 0 ? P.d[1] * P.d[2] : a == 1 ? P.d[0] * P.d[2] : P.d[0] * P.d[1];
-    const double* m1 = P.acc + P.off[terms[t][0]] + (long long)f * n;
-    const double* j1 = P.acc + P.off[terms[t][1]] + (long long)f * n;
-    const double* m2 = P.acc + P.off[terms[t][2]] + (long long)f * n;
-    const double* j2 = P.acc + P.off[terms[t][3]] + (long long)f * n;
-    const long long im = (long long)P.nFreq * n;  // imaginary parts follow the real ones
-    double fs = 0.0;
-    for (long long p = threadIdx.x; p < n; p += 256)
-      fs += m1[p] * j1[p] + m1[p + im] * j1[p + im] - m2[p] * j2[p] - m2[p + im] * j2[p + im];
-    s += terms[t][4] * area * fs;
-  }
-  red[threadIdx.x] = s;
+  const int a = 2 - t / 2;
+  const long long n = P.sz[a];
+  const double area = a == 0 ? P.d[1] * P.d[2] : a == 1 ? P.d[0] * P.d[2] : P.d[0] * P.d[1];
+  const double* m1 = P.acc + P.off[terms[t][0]] + (long long)f * n;
+  const double* j1 = P.acc + P.off[terms[t][1]] + (long long)f * n;
+  const double* m2 = P.acc + P.off[terms[t][2]] + (long long)f * n;
+  const double* j2 = P.acc + P.off[terms[t][3]] + (long long)f * n;
+  const long long im = (long long)P.nFreq * n;  // imaginary parts follow the real ones
+  double fs = 0.0;
+#pragma unroll 4
+  for (long long p = threadIdx.x; p < n; p += 256)
+    fs += m1[p] * j1[p] + m1[p + im] * j1[p + im] - m2[p] * j2[p] - m2[p + im] * j2[p + im];
+  red[threadIdx.x] = terms[t][4] * area * fs;
   __syncthreads();
   for (int w = 128; w > 0; w >>= 1) {
     if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
     __syncthreads();
   }
-  if (threadIdx.x == 0) radp[f] = 0.5 * red[0];
+  if (threadIdx.x == 0) part[f * 6 + t] = red[0];
+}
+__global__ void k_ff_power_sum(const double* __restrict__ part, int F, double* __restrict__ radp) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= F) return;
+  double s = 0.0;
+  for (int t = 0; t < 6; t++) s += part[f * 6 + t];
+  radp[f] = 0.5 * s;
 }
 
 struct Cplx {
@@ -101,100 +117,228 @@ __device__ __forceinline__ Cplx cexpj(double phase) {
   return {c, s};
 }
 
-constexpr int kFFAng = 2;  // directions per thread
-
-__global__ void __launch_bounds__(256) k_ff_pattern(FFPost P, const double* __restrict__ freqs,
-                                                    const double* __restrict__ theta, const double* __restrict__ phi,
-                                                    int nang, const double* __restrict__ radp, double* __restrict__ dth,
-                                                    double* __restrict__ dph) {
-  __shared__ double sd[8][256];  // J1 J2 M1 M2 (re, im) of up to 256 points
-  const int f = blockIdx.y;
-  const double k = 2.0 * kPi * freqs[f] / kC0;
-  double dir[kFFAng][3], st[kFFAng], ct[kFFAng], sp[kFFAng], cp[kFFAng];
-  Cplx Nt[kFFAng], Np[kFFAng], Lt[kFFAng], Lp[kFFAng];
-  for (int q = 0; q < kFFAng; q++) {
-    const int a = (blockIdx.x * kFFAng + q) * 256 + threadIdx.x;
-    const double th = a < nang ? theta[a] : 0.0, ph = a < nang ? phi[a] : 0.0;
-    sincos(th, &st[q], &ct[q]);
-    sincos(ph, &sp[q], &cp[q]);
-    dir[q][0] = st[q] * cp[q];
-    dir[q][1] = st[q] * sp[q];
-    dir[q][2] = ct[q];
-    Nt[q] = Np[q] = Lt[q] = Lp[q] = Cplx{0.0, 0.0};
-  }
-  const long long im_stride[3] = {(long long)P.nFreq * P.sz[0], (long long)P.nFreq * P.sz[1],
-                                   (long long)P.nFreq * P.sz[2]};
-  const int ext[3] = {P.ni, P.nj, P.nk};
-  for (int fc = 0; fc < 6; fc++) {
-    const int a = fc / 2, side = fc % 2;
-    // point grid of the face: outer axis o, inner (fastest) axis n
-    const int o = a == 0 ? 1 : 0, n = a == 2 ? 1 : 2;
-    const int no = ext[o], nn = ext[n];
-    int j1, j2, m1, m2;
-    face_arrays(fc, j1, j2, m1, m2);
-    const long long base = (long long)f * P.sz[a];
-    Cplx S[kFFAng][4];
-    Cplx step[kFFAng];
-    for (int q = 0; q < kFFAng; q++) {
-      for (int w = 0; w < 4; w++) S[q][w] = Cplx{0.0, 0.0};
-      step[q] = cexpj(k * P.d[n] * dir[q][n]);
-    }
-    for (int r = 0; r < no; r++) {
-      for (int c0 = 0; c0 < nn; c0 += 256) {
-        const int cnt = min(256, nn - c0);
-        __syncthreads();
-        if (threadIdx.x < cnt) {
-          const long long p = base + (long long)r * nn + c0 + threadIdx.x;
-          const int arr[4] = {j1, j2, m1, m2};
+// Rows of points along axis `n` of a face, summed for one thread's directions.
+// Stages the pairs of `rows` rows (the same row of that many faces) in shared
+// memory and adds their sums, phases relative to the rows' middles.
+constexpr int kFFPairs = 64;  // pairs staged at a time
+template <int ANG, int ROWS>
+struct FFRows {
+  double (*sm)[kFFPairs][16];  // [ROWS]: u then v of J1 J2 M1 M2 (re, im)
+  // arr[row][w]: current w of the row's first point; its imaginary part `im` on
+  __device__ __forceinline__ void sum(const double* const (*arr)[4], long long im, int nn, const double* kx, double d,
+                                      Cplx (*S)[ROWS][4]) const {
+    const int half = nn / 2, odd = nn & 1, np = half + odd;
+    for (int t0 = 0; t0 < np; t0 += kFFPairs) {
+      const int cnt = min(kFFPairs, np - t0);
+      __syncthreads();
+      for (int x = threadIdx.x; x < ROWS * 8 * cnt; x += blockDim.x) {
+        const int t = x % cnt, w = x / cnt % 8, row = x / cnt / 8;
+        const double* A = arr[row][w / 2] + (w & 1 ? im : 0);
+        const int hi = half + t0 + t;          // the pair's upper point; of an odd row the middle comes first
+        const int lo = nn - 1 - hi;
+        const double p = A[hi], m = lo == hi ? 0.0 : A[lo];
+        sm[row][t][w] = p + m;
+        sm[row][t][8 + w] = lo == hi ? 0.0 : p - m;
+      }
+      __syncthreads();
+      Cplx e[ANG], step[ANG];
+#pragma unroll
+      for (int q = 0; q < ANG; q++) {
+        e[q] = cexpj(kx[q] * d * (t0 + (odd ? 0.0 : 0.5)));
+        step[q] = cexpj(kx[q] * d);
+      }
+      for (int t = 0; t < cnt; t++) {
+#pragma unroll
+        for (int row = 0; row < ROWS; row++)
+#pragma unroll
           for (int w = 0; w < 4; w++) {
-            const double* A = P.acc + P.off[arr[w]];
-            sd[2 * w][threadIdx.x] = A[p];
-            sd[2 * w + 1][threadIdx.x] = A[p + im_stride[a]];
+            const double2 u = *reinterpret_cast<const double2*>(&sm[row][t][2 * w]);
+            const double2 v = *reinterpret_cast<const double2*>(&sm[row][t][8 + 2 * w]);
+#pragma unroll
+            for (int q = 0; q < ANG; q++) {
+              Cplx& s = S[q][row][w];
+              s.re += e[q].re * u.x - e[q].im * v.y;
+              s.im += e[q].re * u.y + e[q].im * v.x;
+            }
           }
-        }
-        __syncthreads();
-        for (int q = 0; q < kFFAng; q++) {
-          const double ph0 = k * (P.face[a][side] * dir[q][a] + (P.pos0[o] + r * P.d[o]) * dir[q][o] +
-                                  (P.pos0[n] + c0 * P.d[n]) * dir[q][n]);
-          Cplx e = cexpj(ph0);
-          for (int t = 0; t < cnt; t++) {
-            for (int w = 0; w < 4; w++) cmac(S[q][w], e, sd[2 * w][t], sd[2 * w + 1][t]);
-            e = cmul(e, step[q]);
-          }
-        }
+#pragma unroll
+        for (int q = 0; q < ANG; q++) e[q] = cmul(e[q], step[q]);
       }
     }
-    // project the face sums (farfield.js:328-607)
-    const double A = a == 0 ? P.d[1] * P.d[2] : a == 1 ? P.d[0] * P.d[2] : P.d[0] * P.d[1];
-    for (int q = 0; q < kFFAng; q++) {
-      const Cplx J1 = S[q][0], J2 = S[q][1], M1 = S[q][2], M2 = S[q][3];
-      double t1, t2, p1, p2;  // N_theta = t1 J1 + t2 J2, N_phi = p1 J1 + p2 J2 (same for L with M)
-      if (a == 0) {           // J1 = Jy, J2 = Jz
-        t1 = A * ct[q] * sp[q]; t2 = -A * st[q]; p1 = A * cp[q]; p2 = 0.0;
-      } else if (a == 1) {    // J1 = Jx, J2 = Jz
-        t1 = A * ct[q] * cp[q]; t2 = -A * st[q]; p1 = -A * sp[q]; p2 = 0.0;
-      } else {                // J1 = Jx, J2 = Jy
-        t1 = A * ct[q] * cp[q]; t2 = A * ct[q] * sp[q]; p1 = -A * sp[q]; p2 = A * cp[q];
-      }
-      Nt[q].re += t1 * J1.re + t2 * J2.re;
-      Nt[q].im += t1 * J1.im + t2 * J2.im;
-      Np[q].re += p1 * J1.re + p2 * J2.re;
-      Np[q].im += p1 * J1.im + p2 * J2.im;
-      Lt[q].re += t1 * M1.re + t2 * M2.re;
-      Lt[q].im += t1 * M1.im + t2 * M2.im;
-      Lp[q].re += p1 * M1.re + p2 * M2.re;
-      Lp[q].im += p1 * M1.im + p2 * M2.im;
+  }
+};
+
+// Workspace of the row sums.
+struct FFSums {
+  int f0;             // first frequency
+  int nth;            // distinct thetas of the directions
+  const double* cth;  // their cosines
+  const int* ith;     // [directions] which of them
+  const double *theta, *phi;
+  int nang;           // directions
+  double* rows;       // [freq][row][8][theta]: rows of xp, xn (nj each), yp, yn (ni each)
+  double* z;          // [freq][part][8][direction]: the z faces' sums
+  int parts;          // each of a part of their rows
+};
+
+constexpr int kFFRowThreads = 64, kFFRowAng = 2;
+__global__ void __launch_bounds__(kFFRowThreads)
+    k_ff_rows(FFPost P, FFSums W, const double* __restrict__ freqs) {
+  __shared__ __align__(16) double sm[1][kFFPairs][16];
+  const int f = W.f0 + blockIdx.z;
+  int r = blockIdx.y, fc = 0;
+  for (; fc < 3 && r >= (fc < 2 ? P.nj : P.ni); fc++) r -= fc < 2 ? P.nj : P.ni;
+  const int a = fc / 2, nn = P.nk;
+  const double k = 2.0 * kPi * freqs[f] / kC0;
+  int c[4];
+  face_arrays(fc, c[0], c[1], c[2], c[3]);
+  const double* arr[1][4];
+  for (int w = 0; w < 4; w++) arr[0][w] = P.acc + P.off[c[w]] + (long long)f * P.sz[a] + (long long)r * nn;
+  double kx[kFFRowAng];
+  Cplx S[kFFRowAng][1][4] = {};
+  const int th0 = blockIdx.x * kFFRowThreads * kFFRowAng + threadIdx.x;
+  for (int q = 0; q < kFFRowAng; q++) {
+    const int th = th0 + q * kFFRowThreads;
+    kx[q] = th < W.nth ? k * W.cth[th] : 0.0;
+  }
+  FFRows<kFFRowAng, 1>{sm}.sum(arr, (long long)P.nFreq * P.sz[a], nn, kx, P.d[2], S);
+  const int R = 2 * (P.ni + P.nj);
+  for (int q = 0; q < kFFRowAng; q++) {
+    const int th = th0 + q * kFFRowThreads;
+    if (th >= W.nth) continue;
+    const Cplx mid = cexpj(kx[q] * (P.pos0[2] + 0.5 * (nn - 1) * P.d[2]));
+    double* out = W.rows + ((long long)blockIdx.z * R + blockIdx.y) * 8 * W.nth + th;
+    for (int w = 0; w < 4; w++) {
+      const Cplx v = cmul(mid, S[q][0][w]);
+      out[2 * w * (long long)W.nth] = v.re;
+      out[(2 * w + 1) * (long long)W.nth] = v.im;
     }
   }
-  const double scale = k * k / (8.0 * kPi * kEta0 * radp[f]);
-  for (int q = 0; q < kFFAng; q++) {
-    const int a = (blockIdx.x * kFFAng + q) * 256 + threadIdx.x;
-    if (a >= nang) continue;
-    const double ar = Lp[q].re + kEta0 * Nt[q].re, ai = Lp[q].im + kEta0 * Nt[q].im;
-    const double br = Lt[q].re - kEta0 * Np[q].re, bi = Lt[q].im - kEta0 * Np[q].im;
-    dth[(long long)f * nang + a] = scale * (ar * ar + ai * ai);
-    dph[(long long)f * nang + a] = scale * (br * br + bi * bi);
+}
+
+// Directions: (sin theta cos phi, sin theta sin phi, cos theta).
+constexpr int kFFZThreads = 64, kFFZAng = 2;
+__global__ void __launch_bounds__(kFFZThreads) k_ff_zrows(FFPost P, FFSums W, const double* __restrict__ freqs) {
+  __shared__ __align__(16) double sm[2][kFFPairs][16];
+  const int f = W.f0 + blockIdx.z, part = blockIdx.y, nn = P.nj;
+  const double k = 2.0 * kPi * freqs[f] / kC0;
+  double dx[kFFZAng], kx[kFFZAng];
+  Cplx side[kFFZAng][2];
+  int c[2][4];
+  for (int s = 0; s < 2; s++) face_arrays(4 + s, c[s][0], c[s][1], c[s][2], c[s][3]);
+  const int ang0 = blockIdx.x * kFFZThreads * kFFZAng + threadIdx.x;
+  for (int q = 0; q < kFFZAng; q++) {
+    const int ang = ang0 + q * kFFZThreads;
+    const double th = ang < W.nang ? W.theta[ang] : 0.0, ph = ang < W.nang ? W.phi[ang] : 0.0;
+    double st, ct, sp, cp;
+    sincos(th, &st, &ct);
+    sincos(ph, &sp, &cp);
+    const double dy = st * sp;
+    dx[q] = st * cp;
+    kx[q] = k * dy;
+    for (int s = 0; s < 2; s++) side[q][s] = cexpj(k * (P.face[2][s] * ct + (P.pos0[1] + 0.5 * (nn - 1) * P.d[1]) * dy));
   }
+  Cplx T[kFFZAng][4] = {};
+  const int r0 = (int)((long long)part * P.ni / W.parts), r1 = (int)((long long)(part + 1) * P.ni / W.parts);
+  for (int r = r0; r < r1; r++) {
+    const double* arr[2][4];
+    for (int s = 0; s < 2; s++)
+      for (int w = 0; w < 4; w++) arr[s][w] = P.acc + P.off[c[s][w]] + (long long)f * P.sz[2] + (long long)r * nn;
+    Cplx S[kFFZAng][2][4] = {};
+    FFRows<kFFZAng, 2>{sm}.sum(arr, (long long)P.nFreq * P.sz[2], nn, kx, P.d[1], S);
+    for (int q = 0; q < kFFZAng; q++) {
+      const Cplx e = cexpj(k * (P.pos0[0] + r * P.d[0]) * dx[q]);
+      for (int s = 0; s < 2; s++) {
+        const Cplx es = cmul(e, side[q][s]);
+        for (int w = 0; w < 4; w++) cmac(T[q][w], es, S[q][s][w].re, S[q][s][w].im);
+      }
+    }
+  }
+  for (int q = 0; q < kFFZAng; q++) {
+    const int ang = ang0 + q * kFFZThreads;
+    if (ang >= W.nang) continue;
+    double* out = W.z + ((long long)blockIdx.z * W.parts + part) * 8 * W.nang + ang;
+    for (int w = 0; w < 4; w++) {
+      out[2 * w * (long long)W.nang] = T[q][w].re;
+      out[(2 * w + 1) * (long long)W.nang] = T[q][w].im;
+    }
+  }
+}
+
+// A direction's radiation vectors.
+struct FFVectors {
+  double st, ct, sp, cp;
+  Cplx Nt{0.0, 0.0}, Np{0.0, 0.0}, Lt{0.0, 0.0}, Lp{0.0, 0.0};
+  // adds a face's sums, or several of one axis's (farfield.js:328-607)
+  __device__ __forceinline__ void add(int a, double A, const Cplx* S) {
+    const Cplx J1 = S[0], J2 = S[1], M1 = S[2], M2 = S[3];
+    double t1, t2, p1, p2;  // N_theta = t1 J1 + t2 J2, N_phi = p1 J1 + p2 J2 (same for L with M)
+    if (a == 0) {           // J1 = Jy, J2 = Jz
+      t1 = A * ct * sp; t2 = -A * st; p1 = A * cp; p2 = 0.0;
+    } else if (a == 1) {    // J1 = Jx, J2 = Jz
+      t1 = A * ct * cp; t2 = -A * st; p1 = -A * sp; p2 = 0.0;
+    } else {                // J1 = Jx, J2 = Jy
+      t1 = A * ct * cp; t2 = A * ct * sp; p1 = -A * sp; p2 = A * cp;
+    }
+    Nt.re += t1 * J1.re + t2 * J2.re;
+    Nt.im += t1 * J1.im + t2 * J2.im;
+    Np.re += p1 * J1.re + p2 * J2.re;
+    Np.im += p1 * J1.im + p2 * J2.im;
+    Lt.re += t1 * M1.re + t2 * M2.re;
+    Lt.im += t1 * M1.im + t2 * M2.im;
+    Lp.re += p1 * M1.re + p2 * M2.re;
+    Lp.im += p1 * M1.im + p2 * M2.im;
+  }
+  __device__ __forceinline__ void out(double k, double radp, double& dth, double& dph) const {
+    const double scale = k * k / (8.0 * kPi * kEta0 * radp);
+    const double ar = Lp.re + kEta0 * Nt.re, ai = Lp.im + kEta0 * Nt.im;
+    const double br = Lt.re - kEta0 * Np.re, bi = Lt.im - kEta0 * Np.im;
+    dth = scale * (ar * ar + ai * ai);
+    dph = scale * (br * br + bi * bi);
+  }
+};
+
+// Directions from the row sums: one thread per (direction, frequency).  dth and
+// dph: [freq][stride], from the first direction.
+__global__ void __launch_bounds__(128)
+    k_ff_pattern(FFPost P, FFSums W, const double* __restrict__ freqs, const double* __restrict__ radp, long long stride,
+                 double* __restrict__ dth, double* __restrict__ dph) {
+  const int f = W.f0 + blockIdx.y, ang = blockIdx.x * 128 + threadIdx.x, nang = W.nang;
+  if (ang >= nang) return;
+  const double k = 2.0 * kPi * freqs[f] / kC0;
+  FFVectors V;
+  sincos(W.theta[ang], &V.st, &V.ct);
+  sincos(W.phi[ang], &V.sp, &V.cp);
+  const double dir[2] = {V.st * V.cp, V.st * V.sp};
+  const double* g = W.rows + (long long)blockIdx.y * 2 * (P.ni + P.nj) * 8 * W.nth + W.ith[ang];
+  for (int fc = 0; fc < 4; fc++) {
+    const int a = fc / 2, o = 1 - a, no = a == 0 ? P.nj : P.ni;
+    Cplx S[4] = {};
+    const Cplx step = cexpj(k * P.d[o] * dir[o]);
+    for (int r0 = 0; r0 < no; r0 += 64) {
+      Cplx e = cexpj(k * (P.face[a][fc % 2] * dir[a] + (P.pos0[o] + r0 * P.d[o]) * dir[o]));
+      const int r1 = min(r0 + 64, no);
+#pragma unroll 1  // the loads of more rows cost registers, and so warps: 430 us for 341 when unrolled by two
+      for (int r = r0; r < r1; r++) {
+#pragma unroll
+        for (int w = 0; w < 4; w++)
+          cmac(S[w], e, __ldg(g + 2 * w * (long long)W.nth), __ldg(g + (2 * w + 1) * (long long)W.nth));
+        e = cmul(e, step);
+        g += 8 * (long long)W.nth;
+      }
+    }
+    V.add(a, a == 0 ? P.d[1] * P.d[2] : P.d[0] * P.d[2], S);
+  }
+  Cplx S[4] = {};
+  for (int part = 0; part < W.parts; part++) {
+    const double* z = W.z + ((long long)blockIdx.y * W.parts + part) * 8 * nang + ang;
+    for (int w = 0; w < 4; w++) {
+      S[w].re += z[2 * w * (long long)nang];
+      S[w].im += z[(2 * w + 1) * (long long)nang];
+    }
+  }
+  V.add(2, P.d[0] * P.d[1], S);
+  V.out(k, radp[f], dth[f * stride + ang], dph[f * stride + ang]);
 }
 
 }  // namespace fdtd
