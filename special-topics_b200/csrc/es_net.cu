@@ -3,11 +3,13 @@
 // inference kernels.  Weights live as FP32 master values plus BF16 copies; the
 // forward and backward passes read the BF16 copies and accumulate in FP32.
 //
-// Every layer is one GEMM: a convolution is an im2col gather followed by
-// out[(b,t)][co] = sum_{k,ci} cols[(b,t)][k*cin+ci] * W[co][k][ci], a dense
+// Every layer is one GEMM: a convolution is
+// out[(b,t)][co] = sum_{k,ci} in[b][t*stride+k-pad][ci] * W[co][k][ci], a dense
 // layer is out[b][o] = sum_i in[b][i] * W[o][i].  Activations are stored time
 // major with the channel fastest, so a convolution's GEMM output is directly
-// the next layer's input.  All reductions run in a fixed order (split sums are
+// the next layer's input, and the inputs of one output (its row of the GEMM) are
+// one run of ksz*cin values, cut off at the ends of the sample: the GEMM reads
+// them in place.  All reductions run in a fixed order (split sums are
 // combined by a second pass, never by atomics), so training is reproducible.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -45,144 +47,213 @@ int es_fail(int code, const char* fmt, ...) {
 __device__ __forceinline__ float ld(const float* p) { return *p; }
 __device__ __forceinline__ float ld(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 
-constexpr int kTM = 64, kTN = 64, kTK = 16;
+// The rows of inputs that a layer's outputs read: row r = (b, t) is `kdim`
+// values from in[b * width + off], off = (t * step - pad), zero where off + k
+// leaves [0, width).  Dense: lout = 1, pad = 0, width = kdim.
+struct Rows {
+  const float* in;
+  int lout, step, pad, width;
+  __device__ __forceinline__ void at(int r, const float*& p, int& off) const {
+    const int b = r / lout;
+    off = (r - b * lout) * step - pad;
+    p = in + (long long)b * width + off;
+  }
+};
 
-// C = op(A) op(B) (+ bias, ReLU).  op(A)[m][k] = TA ? A[k*lda+m] : A[m*lda+k];
-// op(B)[k][n] = TB ? B[n*ldb+k] : B[k*ldb+n].  blockIdx.z selects a slice of
-// the k range (kchunk wide) whose partial result goes to C + z*c_split; bias
-// and ReLU are applied only when there is a single slice.
-template <bool TA, bool TB, typename TAe, typename TBe>
-__global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const TAe* __restrict__ A, int lda,
-                                              const TBe* __restrict__ B, int ldb, float* __restrict__ Cm, int ldc,
-                                              long long c_split, int kchunk, const float* __restrict__ bias,
-                                              int relu) {
-  __shared__ float As[kTK][kTM + 4];
-  __shared__ float Bs[kTK][kTN + 4];
-  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+// Three products, FP32 accumulation in order of k within a slice of the k range
+// (kchunk wide, blockIdx.z):
+//   kForward:  C[m][n] = sum_k rows(m, k) W[n][k]     (rows of inputs, BF16 weights)
+//   kInput:    C[m][n] = sum_k Y[m][k] W[k][n]        (gradient with respect to the inputs)
+//   kWeights:  C[n][m] = sum_k rows(k, m) Y[k][n], and bsum[n] = sum_k Y[k][n]
+// With one slice (kForward, kInput) bias and ReLU, or the derivative of the ReLU
+// whose output `post` is, are applied here, otherwise the slices' partial results
+// go to C + z c_split for k_sum_slices.
+//
+// A tile is 128 x 64 x 16 with 8 x 4 results a thread, 3 shared-memory loads of
+// 16 bytes per 32 multiply-adds, and the next tile's values are in flight while
+// this one's are used.  The 64 x 64 tile with 4 x 4 results, scalar loads and no
+// prefetch, over an im2col matrix in memory, took 1.7 ms of a 256-sample
+// gradient's 2.1; these take 0.5 ms of 0.6.  (FP32 activations times BF16 weights on
+// the tensor cores would need three products each, and round their sums
+// otherwise.)
+enum GemmForm { kForward, kInput, kWeights };
+constexpr int kTM = 128, kTN = 64, kTK = 16;
+
+template <GemmForm F>
+__global__ void __launch_bounds__(256)
+    k_gemm(int M, int N, int K, Rows rows, const float* __restrict__ Y, const __nv_bfloat16* __restrict__ W, int ldw,
+           float* __restrict__ Cm, int ldc, long long c_split, int kchunk, const float* __restrict__ bias, int relu,
+           const float* __restrict__ post, float* __restrict__ bsum) {
+  __shared__ __align__(16) float As[2][kTK][kTM + 4];
+  __shared__ __align__(16) float Bs[2][kTK][kTN + 4];
+  const int tid = threadIdx.x;
   const int m0 = blockIdx.y * kTM, n0 = blockIdx.x * kTN;
   const int kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
-  float acc[4][4];
-  for (int a = 0; a < 4; a++)
+  // a thread's places in the tiles: kWeights walks m along a row, the others k
+  const int ak = F == kWeights ? tid / kTM : tid % kTK, am = F == kWeights ? tid % kTM : tid / kTK;
+  const int bk = F == kForward ? tid % kTK : tid / kTN, bn = F == kForward ? tid / kTK : tid % kTN;
+  const float* ap[8];
+  int aoff[8];
+  if (F == kForward) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const int m = m0 + am + 16 * q;
+      ap[q] = nullptr;
+      aoff[q] = 0;
+      if (m < M) rows.at(m, ap[q], aoff[q]);
+    }
+  }
+  float ra[8], rb[4];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      ra[q] = 0.f;
+      if (F == kForward) {
+        const int k = k0 + ak;
+        if (ap[q] && k < kend && (unsigned)(aoff[q] + k) < (unsigned)rows.width) ra[q] = ap[q][k];
+      } else if (F == kInput) {
+        const int k = k0 + ak, m = m0 + am + 16 * q;
+        if (m < M && k < kend) ra[q] = Y[(long long)m * K + k];
+      } else {
+        const int k = k0 + ak + 2 * q, m = m0 + am;
+        if (m < M && k < kend) {
+          const float* p;
+          int off;
+          rows.at(k, p, off);
+          if ((unsigned)(off + m) < (unsigned)rows.width) ra[q] = p[m];
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      rb[q] = 0.f;
+      if (F == kForward) {
+        const int k = k0 + bk, n = n0 + bn + 16 * q;
+        if (n < N && k < kend) rb[q] = __bfloat162float(W[(long long)n * ldw + k]);
+      } else {
+        const int k = k0 + bk + 4 * q, n = n0 + bn;
+        if (n < N && k < kend)
+          rb[q] = F == kInput ? __bfloat162float(W[(long long)k * ldw + n]) : Y[(long long)k * N + n];
+      }
+    }
+  };
+  auto store = [&](int buf) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) As[buf][F == kWeights ? ak + 2 * q : ak][F == kWeights ? am : am + 16 * q] = ra[q];
+#pragma unroll
+    for (int q = 0; q < 4; q++) Bs[buf][F == kForward ? bk : bk + 4 * q][F == kForward ? bn + 16 * q : bn] = rb[q];
+  };
+  const int tx = tid % 16, ty = tid / 16;
+  float acc[8][4];
+#pragma unroll
+  for (int a = 0; a < 8; a++)
+#pragma unroll
     for (int b = 0; b < 4; b++) acc[a][b] = 0.f;
-  for (int k0 = kbeg; k0 < kend; k0 += kTK) {
-    for (int e = tid; e < kTM * kTK; e += 256) {
-      int mm, kk;
-      if (TA) { mm = e % kTM; kk = e / kTM; } else { kk = e % kTK; mm = e / kTK; }
-      const int gm = m0 + mm, gk = k0 + kk;
-      float v = 0.f;
-      if (gm < M && gk < kend) v = TA ? ld(A + (long long)gk * lda + gm) : ld(A + (long long)gm * lda + gk);
-      As[kk][mm] = v;
-    }
-    for (int e = tid; e < kTN * kTK; e += 256) {
-      int nn, kk;
-      if (TB) { kk = e % kTK; nn = e / kTK; } else { nn = e % kTN; kk = e / kTN; }
-      const int gn = n0 + nn, gk = k0 + kk;
-      float v = 0.f;
-      if (gn < N && gk < kend) v = TB ? ld(B + (long long)gn * ldb + gk) : ld(B + (long long)gk * ldb + gn);
-      Bs[kk][nn] = v;
-    }
-    __syncthreads();
+  float bs = 0.f;
+  const bool sums = F == kWeights && blockIdx.y == 0 && tid < kTN;
+  load(kbeg);
+  store(0);
+  __syncthreads();
+  for (int k0 = kbeg, buf = 0; k0 < kend; k0 += kTK, buf ^= 1) {
+    const bool more = k0 + kTK < kend;
+    if (more) load(k0 + kTK);
 #pragma unroll
     for (int kk = 0; kk < kTK; kk++) {
-      float a[4], b[4];
+      float a[8], b[4];
+      *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&As[buf][kk][4 * ty]);
+      *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&As[buf][kk][64 + 4 * ty]);
+      *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(&Bs[buf][kk][4 * tx]);
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        a[q] = As[kk][ty + 16 * q];
-        b[q] = Bs[kk][tx + 16 * q];
-      }
-#pragma unroll
-      for (int p = 0; p < 4; p++)
+      for (int p = 0; p < 8; p++)
 #pragma unroll
         for (int q = 0; q < 4; q++) acc[p][q] = fmaf(a[p], b[q], acc[p][q]);
     }
+    if (sums) {
+      float t = 0.f;
+#pragma unroll
+      for (int kk = 0; kk < kTK; kk++) t += Bs[buf][kk][tid];
+      bs += t;
+    }
+    if (more) store(buf ^ 1);
     __syncthreads();
   }
   float* C = Cm + (long long)blockIdx.z * c_split;
   const bool single = gridDim.z == 1;
 #pragma unroll
-  for (int p = 0; p < 4; p++) {
-    const int m = m0 + ty + 16 * p;
+  for (int p = 0; p < 8; p++) {
+    const int m = m0 + (p < 4 ? 0 : 60) + 4 * ty + p;
     if (m >= M) continue;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-      const int n = n0 + tx + 16 * q;
+      const int n = n0 + 4 * tx + q;
       if (n >= N) continue;
       float v = acc[p][q];
+      if (F == kWeights) {
+        C[(long long)n * ldc + m] = v;
+        continue;
+      }
       if (single) {
         if (bias) v += bias[n];
         if (relu) v = fmaxf(v, 0.f);
+        if (post && !(post[(long long)m * ldc + n] > 0.f)) v = 0.f;
       }
       C[(long long)m * ldc + n] = v;
     }
   }
+  if (sums && n0 + tid < N) bsum[(long long)blockIdx.z * c_split + n0 + tid] = bs;
 }
 
-// out[i] = sum over s of part[s*n + i], s in order.
-__global__ void k_sum_slices(const float* __restrict__ part, int slices, long long n, float* __restrict__ out) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// out[i] = sum over s of part[s*n + i] (+ bias of column i % cols, ReLU, or the
+// derivative of the ReLU whose output `post` is).  A block has 256 / Y values and
+// Y threads each: thread y sums slices y, y + Y, ... in order, then the Y sums are
+// added in order.  Y = 8 where there are many slices of few values: 296 slices of
+// 704 values took 25 us with one thread each.
+template <int Y>
+__global__ void __launch_bounds__(256)
+    k_sum_slices(const float* __restrict__ part, int slices, long long n, const float* __restrict__ bias, int cols,
+                 int relu, const float* __restrict__ post, float* __restrict__ out) {
+  constexpr int X = 256 / Y;
+  __shared__ float red[Y][X];
+  const int x = threadIdx.x % X, y = threadIdx.x / X;
+  const long long i = (long long)blockIdx.x * X + x;
   float s = 0.f;
-  for (int q = 0; q < slices; q++) s += part[(long long)q * n + i];
+  if (i < n) {
+#pragma unroll 8
+    for (int q = y; q < slices; q += Y) s += part[(long long)q * n + i];
+  }
+  if constexpr (Y > 1) {
+    red[y][x] = s;
+    __syncthreads();
+    if (y > 0) return;
+    for (int q = 1; q < Y; q++) s += red[q][x];
+  }
+  if (i >= n) return;
+  if (bias) s += bias[i % cols];
+  if (relu) s = fmaxf(s, 0.f);
+  if (post && !(post[i] > 0.f)) s = 0.f;
   out[i] = s;
 }
 
-// Column sums of a rows x cols matrix: one block per column, fixed-order tree.
-__global__ void __launch_bounds__(256) k_col_sums(const float* __restrict__ x, int rows, int cols,
-                                                  float* __restrict__ out) {
-  __shared__ float red[256];
-  const int c = blockIdx.x;
-  float s = 0.f;
-  for (int r = threadIdx.x; r < rows; r += 256) s += x[(long long)r * cols + c];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[c] = red[0];
-}
-
-// cols[(b*lout + t)][k*cin + c] = in[b][t*stride + k - pad][c] (0 outside).
-__global__ void k_im2col(const float* __restrict__ in, int B, int lin, int cin, int lout, int ksz, int stride,
-                         int pad, float* __restrict__ cols) {
-  const long long w = (long long)ksz * cin;
-  const long long n = (long long)B * lout * w;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n;
-       e += (long long)gridDim.x * blockDim.x) {
-    const long long row = e / w;
-    const int kc = (int)(e % w), k = kc / cin, c = kc % cin;
-    const int b = (int)(row / lout), t = (int)(row % lout);
-    const int s = t * stride + k - pad;
-    cols[e] = (s >= 0 && s < lin) ? in[((long long)b * lin + s) * cin + c] : 0.f;
-  }
-}
-
-// Adjoint of k_im2col: din[b][s][c] = sum_k dcols[(b*lout + t)][k*cin + c],
-// t = (s + pad - k) / stride where that is a whole number in [0, lout).
+// Adjoint of the rows' reads: din[b][s][c] = sum_k dcols[(b*lout + t)][k*cin + c],
+// t = (s + pad - k) / stride where that is a whole number in [0, lout); times the
+// derivative of the ReLU whose output `post` is.
 __global__ void k_col2im(const float* __restrict__ dcols, int B, int lin, int cin, int lout, int ksz, int stride,
-                         int pad, float* __restrict__ din) {
-  const long long n = (long long)B * lin * cin;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(e % cin);
-    const long long bs = e / cin;
-    const int s = (int)(bs % lin), b = (int)(bs / lin);
+                         int pad, const float* __restrict__ post, float* __restrict__ din) {
+  const int width = lin * cin;  // a sample's values; one per thread along x, samples along y
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= width) return;
+  const int s = e / cin, c = e - s * cin;
+  for (int b = blockIdx.y; b < B; b += gridDim.y) {
+    const long long at = (long long)b * width + e;
     float acc = 0.f;
-    for (int k = 0; k < ksz; k++) {
-      const int num = s + pad - k;
-      if (num < 0 || num % stride) continue;
-      const int t = num / stride;
+    for (int k = (s + pad) % stride; k < ksz; k += stride) {
+      const int t = (s + pad - k) / stride;
+      if (s + pad < k) break;
       if (t >= lout) continue;
-      acc += dcols[((long long)b * lout + t) * ((long long)ksz * cin) + (long long)k * cin + c];
+      acc += dcols[((long long)b * lout + t) * (ksz * cin) + k * cin + c];
     }
-    din[e] = acc;
+    din[at] = post && !(post[at] > 0.f) ? 0.f : acc;
   }
-}
-
-// dpre = dpost * (post > 0), in place.
-__global__ void k_relu_back(float* __restrict__ d, const float* __restrict__ post, long long n) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && !(post[i] > 0.f)) d[i] = 0.f;
 }
 
 // Per-sample weighted squared error and dL/dy = 2 w (y - t) / B.
@@ -313,7 +384,7 @@ struct fdtd_es_net {
   __nv_bfloat16* p16 = nullptr;
   float *grad = nullptr, *m = nullptr, *v = nullptr;
   std::vector<float*> act;  // act[0] input, act[l+1] output of layer l (max_batch samples)
-  float *cols = nullptr, *dcols = nullptr, *da = nullptr, *db = nullptr, *ws = nullptr;
+  float *dcols = nullptr, *da = nullptr, *db = nullptr, *ws = nullptr;
   float *target = nullptr, *wout = nullptr, *dy = nullptr, *per = nullptr, *loss = nullptr;
   float *dset_x = nullptr, *dset_y = nullptr;
   int* d_perm = nullptr;  // shuffled sample order of the current epoch
@@ -346,54 +417,75 @@ void es_release(fdtd_es_net* n, void* p) {
   n->owned.erase(std::remove(n->owned.begin(), n->owned.end(), p), n->owned.end());
 }
 
-template <bool TA, bool TB, typename TAe, typename TBe>
-void gemm(fdtd_es_net* n, int M, int N, int K, const TAe* A, int lda, const TBe* B, int ldb, float* C, int ldc,
-          const float* bias, bool relu, int slices = 1, long long c_split = 0) {
+Rows layer_rows(const Layer& L, const float* in) {
+  return Rows{in, L.lout, L.stride * L.cin, L.conv ? L.pad * L.cin : 0, (int)L.in_width()};
+}
+
+// One product of the given form in `slices` slices of the k range.
+template <GemmForm F>
+void gemm(fdtd_es_net* n, int M, int N, int K, const Rows& rows, const float* Y, const __nv_bfloat16* W, int ldw,
+          float* C, int ldc, const float* bias, bool relu, const float* post, int slices, long long c_split, float* bsum) {
   const int kchunk = ((K + slices - 1) / slices + kTK - 1) / kTK * kTK;
   const dim3 grd((N + kTN - 1) / kTN, (M + kTM - 1) / kTM, slices);
-  k_gemm<TA, TB, TAe, TBe><<<grd, 256, 0, n->stream>>>(M, N, K, A, lda, B, ldb, C, ldc, c_split, kchunk, bias,
-                                                       relu ? 1 : 0);
+  k_gemm<F><<<grd, 256, 0, n->stream>>>(M, N, K, rows, Y, W, ldw, C, ldc, c_split, kchunk, bias, relu ? 1 : 0, post,
+                                         bsum);
+}
+
+// Slices of a dense layer's k range: its few rows fill few tiles.  Never a
+// function of the batch, so a sample's outputs do not depend on the others.
+int dense_slices(long long k) { return (int)std::max<long long>(1, std::min<long long>(16, k / 128)); }
+
+void sum_slices(fdtd_es_net* n, int slices, long long e, const float* bias, int cols, bool relu, const float* post,
+                float* out) {
+  if (slices >= 32)
+    k_sum_slices<8><<<(unsigned)((e + 31) / 32), 256, 0, n->stream>>>(n->ws, slices, e, bias, cols, relu, post, out);
+  else
+    k_sum_slices<1><<<(unsigned)((e + 255) / 256), 256, 0, n->stream>>>(n->ws, slices, e, bias, cols, relu, post, out);
+}
+
+// rows x width results of kForward or kInput, through the slices' sums if need be.
+template <GemmForm F>
+void product(fdtd_es_net* n, const Layer& L, int M, int N, int K, const Rows& rows, const float* Y, float* C,
+             const float* bias, bool relu, const float* post) {
+  const int slices = L.conv ? 1 : dense_slices(K), ldw = (int)L.kdim();
+  const __nv_bfloat16* W = n->p16 + L.w_off;
+  if (slices == 1) {
+    gemm<F>(n, M, N, K, rows, Y, W, ldw, C, N, bias, relu, post, 1, 0, nullptr);
+  } else {
+    const long long e = (long long)M * N;
+    gemm<F>(n, M, N, K, rows, Y, W, ldw, n->ws, N, nullptr, false, nullptr, slices, e, nullptr);
+    sum_slices(n, slices, e, bias, N, relu, post, C);
+  }
 }
 
 // Forward pass of B samples already in act[0].
 void forward(fdtd_es_net* n, int B) {
   for (size_t l = 0; l < n->layers.size(); l++) {
     const Layer& L = n->layers[l];
-    const __nv_bfloat16* W = n->p16 + L.w_off;
-    const float* bias = n->p32 + L.b_off;  // biases stay FP32
-    if (L.conv) {
-      const long long e = (long long)B * L.lout * L.kdim();
-      k_im2col<<<blocks_for(e), 256, 0, n->stream>>>(n->act[l], B, L.lin, L.cin, L.lout, L.ksz, L.stride, L.pad,
-                                                      n->cols);
-      gemm<false, true>(n, B * L.lout, L.cout, (int)L.kdim(), (const float*)n->cols, (int)L.kdim(), W,
-                        (int)L.kdim(), n->act[l + 1], L.cout, bias, L.relu);
-    } else {
-      gemm<false, true>(n, B, L.cout, L.cin, (const float*)n->act[l], L.cin, W, L.cin, n->act[l + 1], L.cout, bias,
-                        L.relu);
-    }
+    product<kForward>(n, L, L.conv ? B * L.lout : B, L.cout, (int)L.kdim(), layer_rows(L, n->act[l]), nullptr,
+                      n->act[l + 1], n->p32 + L.b_off, L.relu, nullptr);  // biases stay FP32
   }
 }
 
-// Number of row slices the weight-gradient reduction over `rows` is split into.
-long long grad_slices(long long rows) { return std::max<long long>(1, std::min<long long>(64, rows / 512)); }
+// Slices of the weight-gradient reduction over `rows`: two blocks a
+// multiprocessor, none below 64 rows.
+int grad_slices(const Layer& L, long long rows) {
+  const long long tiles = (L.kdim() + kTM - 1) / kTM * ((L.cout + kTN - 1) / kTN);
+  return (int)std::max<long long>(1, std::min<long long>(296 / tiles, (rows + 63) / 64));
+}
 
-// dW (and db) of one layer from dpre (rows x cout) and its input matrix X (rows x kdim).
-void weight_grads(fdtd_es_net* n, const Layer& L, const float* dpre, const float* X, int rows) {
-  const int N = L.cout, K = (int)L.kdim();
-  const int slices = (int)grad_slices(rows);
-  float* gW = n->grad + L.w_off;
-  if (slices == 1) {
-    gemm<true, false>(n, N, K, rows, dpre, N, X, K, gW, K, nullptr, false);
-  } else {
-    // slice s sums its own range of rows; the slices are then added in order
-    gemm<true, false>(n, N, K, rows, dpre, N, X, K, n->ws, K, nullptr, false, slices, (long long)N * K);
-    k_sum_slices<<<blocks_for((long long)N * K), 256, 0, n->stream>>>(n->ws, slices, (long long)N * K, gW);
-  }
-  k_col_sums<<<N, 256, 0, n->stream>>>(dpre, rows, N, n->grad + L.b_off);
+// dW and db of one layer from dpre (rows x cout) and its input: slice s sums its
+// own range of rows; the slices are then added in order.
+void weight_grads(fdtd_es_net* n, const Layer& L, const float* dpre, const float* in, int rows) {
+  const int N = L.cout, K = (int)L.kdim(), slices = grad_slices(L, rows);
+  const long long e = (long long)N * K + N;  // a slice: dW, then db, as in the gradient
+  gemm<kWeights>(n, K, N, rows, layer_rows(L, in), dpre, nullptr, 0, n->ws, K, nullptr, false, nullptr, slices,
+                 e, n->ws + (long long)N * K);
+  sum_slices(n, slices, e, nullptr, 1, false, nullptr, n->grad + L.w_off);
 }
 
 // Backward pass: dy (B x out_dim) -> n->grad.  Activations of the forward pass
-// are still in act[]; the im2col matrix of each convolution is rebuilt.
+// are still in act[].
 void backward(fdtd_es_net* n, int B) {
   float* dcur = n->dy;  // gradient with respect to the current layer's output
   float* bufs[2] = {n->da, n->db};
@@ -401,26 +493,15 @@ void backward(fdtd_es_net* n, int B) {
   for (int l = (int)n->layers.size() - 1; l >= 0; l--) {
     const Layer& L = n->layers[l];
     const int rows = L.conv ? B * L.lout : B;
-    if (L.relu)
-      k_relu_back<<<blocks_for((long long)rows * L.cout), 256, 0, n->stream>>>(dcur, n->act[l + 1],
-                                                                               (long long)rows * L.cout);
-    const __nv_bfloat16* W = n->p16 + L.w_off;
     float* dnext = bufs[flip];
-    if (L.conv) {
-      const long long e = (long long)rows * L.kdim();
-      k_im2col<<<blocks_for(e), 256, 0, n->stream>>>(n->act[l], B, L.lin, L.cin, L.lout, L.ksz, L.stride, L.pad,
-                                                      n->cols);
-      weight_grads(n, L, dcur, n->cols, rows);
-      if (l > 0) {
-        gemm<false, false>(n, rows, (int)L.kdim(), L.cout, (const float*)dcur, L.cout, W, (int)L.kdim(), n->dcols,
-                           (int)L.kdim(), nullptr, false);
-        k_col2im<<<blocks_for((long long)B * L.lin * L.cin), 256, 0, n->stream>>>(n->dcols, B, L.lin, L.cin, L.lout,
-                                                                                   L.ksz, L.stride, L.pad, dnext);
-      }
-    } else {
-      weight_grads(n, L, dcur, n->act[l], rows);
-      if (l > 0)
-        gemm<false, false>(n, B, L.cin, L.cout, (const float*)dcur, L.cout, W, L.cin, dnext, L.cin, nullptr, false);
+    weight_grads(n, L, dcur, n->act[l], rows);
+    if (l > 0) {
+      const float* post = n->layers[l - 1].relu ? n->act[l] : nullptr;  // the gradient passes its ReLU too
+      product<kInput>(n, L, rows, (int)L.kdim(), L.cout, Rows{}, dcur, L.conv ? n->dcols : dnext, nullptr, false,
+                      L.conv ? nullptr : post);
+      if (L.conv)
+        k_col2im<<<dim3((L.lin * L.cin + 255) / 256, std::min(B, 1024)), 256, 0, n->stream>>>(
+            n->dcols, B, L.lin, L.cin, L.lout, L.ksz, L.stride, L.pad, post, dnext);
     }
     dcur = dnext;
     flip ^= 1;
@@ -576,8 +657,8 @@ int fdtd_es_create(const FdtdEsConfig* cfg, fdtd_es_net** out) {
     max_act = std::max(max_act, std::max(L.in_width(), L.out_width()));
     const long long rows = L.conv ? B * L.lout : B;
     if (L.conv) max_cols = std::max(max_cols, rows * L.kdim());
-    const long long slices = grad_slices(rows);
-    if (slices > 1) max_ws = std::max(max_ws, slices * L.cout * L.kdim());
+    max_ws = std::max(max_ws, grad_slices(L, rows) * (L.cout * L.kdim() + L.cout));
+    if (!L.conv) max_ws = std::max(max_ws, rows * std::max(dense_slices(L.cin) * L.cout, dense_slices(L.cout) * L.cin));
   }
   int rc = es_alloc(n, (void**)&n->p32, n->nparam * sizeof(float));
   if (!rc) rc = es_alloc(n, (void**)&n->p16, n->nparam * sizeof(__nv_bfloat16));
@@ -588,7 +669,6 @@ int fdtd_es_create(const FdtdEsConfig* cfg, fdtd_es_net** out) {
     const long long w = l == 0 ? in_width(n) : n->layers[l - 1].out_width();
     rc = es_alloc(n, (void**)&n->act[l], B * w * sizeof(float));
   }
-  if (!rc) rc = es_alloc(n, (void**)&n->cols, max_cols * sizeof(float));
   if (!rc) rc = es_alloc(n, (void**)&n->dcols, max_cols * sizeof(float));
   if (!rc) rc = es_alloc(n, (void**)&n->da, B * max_act * sizeof(float));
   if (!rc) rc = es_alloc(n, (void**)&n->db, B * max_act * sizeof(float));
