@@ -11,6 +11,7 @@
 #include <cstdio>
 #include <cstring>
 #include <initializer_list>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -25,7 +26,6 @@
 #include "fdtd_internal.h"
 
 #include <map>
-#include <mutex>
 #include <utility>
 
 using namespace fdtd;
@@ -179,13 +179,48 @@ struct fdtd_ctx {
   // dt, step count, precision and the arguments of every upload call in call
   // order.  A saved state carries it and loads only where it matches.
   unsigned long long setup_digest = 0x6a09e667f3bcc908ULL;
+  std::recursive_mutex mu;  // held by a call while it uses `fs`, see reclaim_padded
 };
 
 namespace {
 
+int to_dense(fdtd_ctx* c);
+int fused_drop(fdtd_ctx* c);
+using Using = std::lock_guard<std::recursive_mutex>;
+
+// The handles of the process, so that one short of memory can take back what
+// others hold for speed alone.
+struct Handles {
+  std::mutex mu;
+  std::vector<fdtd_ctx*> all;
+};
+Handles& handles() {
+  static Handles* h = new Handles;
+  return *h;
+}
+
+// Another handle on c's device gives up its padded state (its next run builds it
+// again, or takes the half-step path): without it, a problem that fits beside the
+// dense arrays of the others would not.  A handle that is in a call keeps its own.
+// False: none had any.
+bool reclaim_padded(const fdtd_ctx* c) {
+  std::lock_guard<std::mutex> g(handles().mu);
+  for (fdtd_ctx* o : handles().all) {
+    if (o == c || o->device != c->device) continue;
+    std::unique_lock<std::recursive_mutex> use(o->mu, std::try_to_lock);
+    if (use.owns_lock() && !o->fs.owned.empty() && to_dense(o) == FDTD_OK && fused_drop(o) == FDTD_OK) return true;
+  }
+  return false;
+}
+
 int dalloc(fdtd_ctx* c, void** p, size_t bytes) {
   if (bytes == 0) bytes = 16;
   cudaError_t e = cudaMalloc(p, bytes);
+  while (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    if (!reclaim_padded(c)) break;
+    e = cudaMalloc(p, bytes);
+  }
   if (e != cudaSuccess) {
     *p = nullptr;
     return fail(FDTD_ERR_OOM, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
@@ -681,6 +716,7 @@ void fused_free(fdtd_ctx* c) {
 
 // Frees the padded state (after saving what it holds): the set-up changes.
 int fused_drop(fdtd_ctx* c) {
+  Using use(c->mu);
   int rc = to_dense(c);
   c->graphs.clear();
   if (c->stream) cudaStreamSynchronize(c->stream);
@@ -1174,6 +1210,7 @@ constexpr int kMaxBatchStreams = 32;
 
 int run_steps(fdtd_ctx* c, int count, float* elapsed_ms = nullptr, KernelTimer* tm = nullptr) {
   if (count < 0) return fail(FDTD_ERR_BADARG, "negative step count %d", count);
+  Using use(c->mu);
   if (c->ts + count > c->nsteps)
     return fail(FDTD_ERR_BADARG, "running %d steps from step %d exceeds numberOfTimeSteps=%d", count, c->ts,
                 c->nsteps);
@@ -1396,12 +1433,21 @@ int fdtd_create(const FdtdConfig* cfg, fdtd_ctx** out) {
     fdtd_free(c);
     return fail(rc, "%s", msg.c_str());
   }
+  {
+    std::lock_guard<std::mutex> g(handles().mu);
+    handles().all.push_back(c);
+  }
   *out = c;
   return FDTD_OK;
 }
 
 void fdtd_free(fdtd_ctx* c) {
   if (!c) return;
+  {
+    std::lock_guard<std::mutex> g(handles().mu);
+    auto& all = handles().all;
+    all.erase(std::remove(all.begin(), all.end(), c), all.end());
+  }
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   c->graphs.clear();
@@ -2053,6 +2099,7 @@ int fdtd_ctx_read_field(fdtd_ctx* c, int which, double* host, long n) {
   if (which < 0 || which > 5) return fail(FDTD_ERR_BADARG, "field id %d not in 0..5", which);
   if (n != c->ncomp[which]) return fail(FDTD_ERR_BADARG, "field %d: buffer of %ld, need %lld", which, n, c->ncomp[which]);
   CK(cudaSetDevice(c->device));
+  Using use(c->mu);
   if (int rc = to_dense(c)) return rc;
   return read_real(c, field_ptr(c, which), host, n);
 }
@@ -2062,6 +2109,7 @@ int fdtd_ctx_read_psi(fdtd_ctx* c, int f, int slot, double* host, long n) {
   if (f < 0 || f > 5 || slot < 0 || slot > 3 || !c->face[f].present) return fail(FDTD_ERR_BADARG, "no Psi slot %d on face %d", slot, f);
   if (n != c->face[f].n[slot]) return fail(FDTD_ERR_BADARG, "Psi buffer of %ld, need %lld", n, c->face[f].n[slot]);
   CK(cudaSetDevice(c->device));
+  Using use(c->mu);
   if (int rc = to_dense(c)) return rc;
   return read_real(c, c->face[f].psi[slot], host, n);
 }
@@ -2152,6 +2200,7 @@ int fdtd_ctx_save_state(fdtd_ctx* c, void* buf, long long bytes) {
   if (rc) return rc;
   const StateHeader h = state_header(c);
   if (bytes != h.bytes) return fail(FDTD_ERR_BADARG, "state buffer of %lld bytes, need %lld", bytes, h.bytes);
+  Using use(c->mu);
   rc = to_dense(c);
   if (rc) return rc;
   char* p = (char*)buf;
@@ -2182,6 +2231,7 @@ int fdtd_ctx_load_state(fdtd_ctx* c, const void* buf, long long bytes) {
     return fail(FDTD_ERR_BADARG, "state was saved from a problem of another shape, precision or probe set");
   if (theirs.ts < 0 || theirs.ts > c->nsteps) return fail(FDTD_ERR_BADARG, "state step %d out of range", theirs.ts);
   const char* p = (const char*)buf + sizeof(StateHeader);
+  Using use(c->mu);
   c->dense_valid = true;   // every value of the state is replaced
   c->fs.valid = false;
   for (auto& q : state_ranges(c)) {
@@ -2387,7 +2437,12 @@ int fdtd_ctx_farfield_post(fdtd_ctx* c, const double* theta, const double* phi, 
   int rc = FDTD_OK;
   for (size_t room = (size_t)128 << 20; !buf; room /= 8) {
     const int most = (int)std::max<size_t>(64, std::min<size_t>(1 << 20, room / 2 / (8 * R)));
-    runs = ff_runs(theta, nang, most, &cth, &ith);
+    try {
+      runs = ff_runs(theta, nang, most, &cth, &ith);
+    } catch (const std::bad_alloc&) {
+      rc = fail(FDTD_ERR_OOM, "far-field post: host memory for %d directions", nang);
+      break;
+    }
     int ang = 0, th = 0;
     for (const FFRun& u : runs) {
       ang = std::max(ang, u.a1 - u.a0);
@@ -2979,6 +3034,8 @@ int batch_run_members(fdtd_batch* b, int count, bool chain, float* elapsed_ms, K
 
 int batch_run(fdtd_batch* b, int count, float* elapsed_ms = nullptr, KernelTimer* tm = nullptr) {
   if (count < 0) return fail(FDTD_ERR_BADARG, "negative step count %d", count);
+  std::vector<std::unique_lock<std::recursive_mutex>> use;
+  for (fdtd_ctx* c : b->m) use.emplace_back(c->mu);
   const int ts = b->m[0]->ts;
   for (size_t q = 0; q < b->m.size(); q++) {
     fdtd_ctx* c = b->m[q];

@@ -174,3 +174,32 @@ def test_blocked_dft_sums_in_step_order(freqs, block, runs):
             out.append(eng.farfield())
     for a in FF_NAMES:
         assert np.array_equal(out[0][a][0], out[1][a][0]) and np.array_equal(out[0][a][1], out[1][a][1]), a
+
+
+def test_memory_held_for_speed_is_given_back():
+    """A problem that fits beside another's fields, but not beside the padded
+    copies that the other keeps, is accepted, and both go on with the same
+    results.  (The rest of the device's memory is taken, so that neither fits
+    twice: 128^3 keeps some 110 MB of padded copies, 144^3 needs some 95 MB.)"""
+    import torch
+    from special_topics_b200.workloads import scaling_box
+    probs = [build_problem_from_scenario(scaling_box((n, n, n), seed=3, steps=STEPS), STEPS, per_cell=False)
+             for n in (128, 144)]
+    want = []
+    for p in probs:
+        with Engine(p, "f32-table") as eng:
+            eng.run(STEPS)
+            want.append(_state(eng))
+    with Engine(probs[0], "f32-table") as a:
+        a.run(9)
+        free, _ = torch.cuda.mem_get_info()
+        rest = torch.empty(free - (80 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            with Engine(probs[1], "f32-table") as b:
+                b.run(STEPS)
+                _assert_same(want[1], _state(b))
+            a.run(STEPS - 9)
+            _assert_same(want[0], _state(a))
+        finally:
+            del rest
+            torch.cuda.empty_cache()
