@@ -2600,16 +2600,34 @@ struct fdtd_batch {
   std::vector<unsigned char> groups;  // host copies of the BatchGroup parameter structs
   int ngroups = 0;
   size_t group_size = 0;
-  // one-pass mode (streams == 0, every member can run the one-pass step): what
-  // the cached graphs were captured from, two numbers a member
-  std::vector<long long> chain_key;
+  // what the cached graphs were captured from, see batch_take_path
+  std::vector<long long> graph_key;
 };
 
 namespace {
 
-void batch_drop_graph(fdtd_batch* b) {
-  b->graphs.clear();
-  b->chain_key.clear();
+void batch_drop_graph(fdtd_batch* b) { b->graphs.clear(); }
+
+// How a run of a batch advances its members.
+enum BatchPath { kTileList, kMemberKernels, kChains };
+
+// Graphs of one path are cached by step count and place in a DFT block, which
+// say nothing about the path, nor about what the launches of member kernels and
+// chains carry of the members themselves: their set-up, and the copies of the
+// state that chains start from, relative to the first member's.  Graphs captured
+// from anything else are dropped.  (The tile list reads the members' parameters
+// from device memory; batch_prepare drops its graphs where the lists, or the
+// grouped launches' parameters, change.)
+void batch_take_path(fdtd_batch* b, BatchPath path) {
+  std::vector<long long> key{path};
+  for (const fdtd_ctx* c : b->m) {
+    if (path == kTileList) break;
+    key.push_back(c->graphs.rev);
+    key.push_back(path == kChains ? c->fs.cur ^ b->m[0]->fs.cur : 0);
+  }
+  if (key == b->graph_key) return;
+  batch_drop_graph(b);
+  b->graph_key.swap(key);
 }
 
 template <class V>
@@ -2964,19 +2982,7 @@ int batch_run_members(fdtd_batch* b, int count, bool chain, float* elapsed_ms, K
   const int ts = b->m[0]->ts;
   int rc = batch_worker_streams(b, chain ? batch_chain_streams(b) : b->streams);
   if (rc) return rc;
-  if (chain) {
-    std::vector<long long> key;
-    for (fdtd_ctx* c : b->m) {
-      key.push_back(c->graphs.rev);
-      key.push_back(c->fs.cur ^ b->m[0]->fs.cur);
-    }
-    if (key != b->chain_key) {
-      batch_drop_graph(b);
-      b->chain_key = key;
-    }
-  } else if (!b->chain_key.empty()) {
-    batch_drop_graph(b);
-  }
+  batch_take_path(b, chain ? kChains : kMemberKernels);
   // the whole run as cached graphs, captured before the first launch
   std::vector<cudaGraphExec_t> plan;
   if (!tm) {
@@ -3065,6 +3071,7 @@ int batch_run(fdtd_batch* b, int count, float* elapsed_ms = nullptr, KernelTimer
       return fail(rc, "batch member %zu: %s", q, msg.c_str());
     }
   if (b->streams > 0) return batch_run_members(b, count, false, elapsed_ms, tm);
+  batch_take_path(b, kTileList);
   rc = batch_prepare_any(b);
   if (rc) return rc;
   const int ctl_ts = ts - 1;
