@@ -1214,6 +1214,17 @@ int run_plan(RunGraphs& rg, cudaStream_t st, int count, int launches_per_step, E
 
 constexpr int kMaxBatchStreams = 32;
 
+// What the handle's two status words say about the run that just ended, read on
+// stream `st`; `who` names the handle in the message ("" or "batch member 3: ").
+int check_status(const fdtd_ctx* c, cudaStream_t st, const std::string& who = "") {
+  int w[2];
+  CK(cudaMemcpyAsync(w, c->d_status, sizeof(w), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  if (w[0] == FDTD_ERR_CUDA) return fail(FDTD_ERR_CUDA, "%sa bounded device wait of the step ran out", who.c_str());
+  if (w[0] != 0) return fail(FDTD_ERR_NONFINITE, "%snon-finite port sample at step %d", who.c_str(), w[1]);
+  return FDTD_OK;
+}
+
 int run_steps(fdtd_ctx* c, int count, float* elapsed_ms = nullptr, KernelTimer* tm = nullptr) {
   if (count < 0) return fail(FDTD_ERR_BADARG, "negative step count %d", count);
   Using use(c->mu);
@@ -1289,11 +1300,7 @@ int run_steps(fdtd_ctx* c, int count, float* elapsed_ms = nullptr, KernelTimer* 
   }
   CK(cudaStreamSynchronize(c->stream));
   c->ts += count;
-  int st[2];
-  CK(xfer(c, st, c->d_status, sizeof(st), cudaMemcpyDeviceToHost));
-  if (st[0] == FDTD_ERR_CUDA) return fail(FDTD_ERR_CUDA, "a bounded device wait of the staged step ran out");
-  if (st[0] != 0) return fail(FDTD_ERR_NONFINITE, "non-finite port sample at step %d", st[1]);
-  return FDTD_OK;
+  return check_status(c, c->stream);
 }
 
 unsigned long long mix64(unsigned long long h, unsigned long long w) {
@@ -2976,6 +2983,13 @@ int batch_chain_ready(fdtd_batch* b, bool* use) {
   return FDTD_OK;
 }
 
+// The first member that a run left with a status.
+int batch_status(const fdtd_batch* b) {
+  for (size_t q = 0; q < b->m.size(); q++)
+    if (int rc = check_status(b->m[q], b->stream, "batch member " + std::to_string(q) + ": ")) return rc;
+  return FDTD_OK;
+}
+
 // Runs the members: by their own step kernels on worker streams, or (chain) as
 // one-pass chains.
 int batch_run_members(fdtd_batch* b, int count, bool chain, float* elapsed_ms, KernelTimer* tm) {
@@ -3032,13 +3046,7 @@ int batch_run_members(fdtd_batch* b, int count, bool chain, float* elapsed_ms, K
   }
   CK(cudaStreamSynchronize(b->stream));
   for (fdtd_ctx* c : b->m) c->ts += count;
-  for (size_t q = 0; q < b->m.size(); q++) {
-    int st[2];
-    CK(cudaMemcpyAsync(st, b->m[q]->d_status, sizeof(st), cudaMemcpyDeviceToHost, b->stream));
-    CK(cudaStreamSynchronize(b->stream));
-    if (st[0] != 0) return fail(FDTD_ERR_NONFINITE, "batch member %zu: non-finite port sample at step %d", q, st[1]);
-  }
-  return FDTD_OK;
+  return batch_status(b);
 }
 
 int batch_run(fdtd_batch* b, int count, float* elapsed_ms = nullptr, KernelTimer* tm = nullptr) {
@@ -3110,13 +3118,7 @@ int batch_run(fdtd_batch* b, int count, float* elapsed_ms = nullptr, KernelTimer
   for (fdtd_ctx* c : b->m) CK(cudaMemcpyAsync(c->d_ts, &b->d_ctl->ts, sizeof(int), cudaMemcpyDeviceToDevice, b->stream));
   CK(cudaStreamSynchronize(b->stream));
   for (fdtd_ctx* c : b->m) c->ts += count;
-  for (size_t q = 0; q < b->m.size(); q++) {
-    int st[2];
-    CK(cudaMemcpyAsync(st, b->m[q]->d_status, sizeof(st), cudaMemcpyDeviceToHost, b->stream));
-    CK(cudaStreamSynchronize(b->stream));
-    if (st[0] != 0) return fail(FDTD_ERR_NONFINITE, "batch member %zu: non-finite port sample at step %d", q, st[1]);
-  }
-  return FDTD_OK;
+  return batch_status(b);
 }
 
 }  // namespace

@@ -139,7 +139,7 @@ __device__ void voltage_probe(const Fields<T>& f, const Probes& pr, int q, int t
   const double v = mul(pr.v_csvf[q], sum);
   pr.V[(long long)q * pr.nsteps + ts] = v;
   if (!isfinite(v)) {
-    atomicExch(&pr.status[0], 5);
+    atomicCAS(&pr.status[0], 0, 5);  // a wait that ran out stays the cause
     atomicMin(&pr.status[1], ts);
   }
 }
@@ -165,7 +165,7 @@ __device__ void probe_warp(const Fields<T>& f, const Probes& pr, int q, int ts, 
     const double v = mul(pr.v_csvf[u], sum);
     pr.V[(long long)u * pr.nsteps + ts] = v;
     if (!isfinite(v)) {
-      atomicExch(&pr.status[0], 5);
+      atomicCAS(&pr.status[0], 0, 5);  // a wait that ran out stays the cause
       atomicMin(&pr.status[1], ts);
     }
   } else {
