@@ -10,6 +10,7 @@
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <initializer_list>
 #include <mutex>
 #include <string>
@@ -180,7 +181,7 @@ struct fdtd_ctx {
   // dt, step count, precision and the arguments of every upload call in call
   // order.  A saved state carries it and loads only where it matches.
   unsigned long long setup_digest = 0x6a09e667f3bcc908ULL;
-  std::recursive_mutex mu;  // held by a call while it uses `fs`, see reclaim_padded
+  std::recursive_mutex mu;  // held by every call that touches the set-up, the graphs or `fs`, see reclaim_padded
 };
 
 namespace {
@@ -724,10 +725,11 @@ void fused_free(fdtd_ctx* c) {
 int fused_drop(fdtd_ctx* c) {
   Using use(c->mu);
   int rc = to_dense(c);
+  if (rc) return rc;
   c->graphs.clear();
   if (c->stream) cudaStreamSynchronize(c->stream);
   fused_free(c);
-  return rc;
+  return FDTD_OK;
 }
 
 // Layout of a class row for the problem's bands, and the z bands widened to
@@ -1457,6 +1459,7 @@ int fdtd_create(const FdtdConfig* cfg, fdtd_ctx** out) {
 void fdtd_free(fdtd_ctx* c) {
   if (!c) return;
   {
+    // after this no other thread's reclaim_padded finds the handle
     std::lock_guard<std::mutex> g(handles().mu);
     auto& all = handles().all;
     all.erase(std::remove(all.begin(), all.end(), c), all.end());
@@ -1472,6 +1475,7 @@ void fdtd_free(fdtd_ctx* c) {
 
 int fdtd_ctx_upload_coeff(fdtd_ctx* c, int which, const double* host, long n) {
   if (!c || !host) return fail(FDTD_ERR_BADARG, "NULL argument");
+  Using use(c->mu);
   if (c->prec == FDTD_PREC_F32_TABLE) return fail(FDTD_ERR_STATE, "material-table problem takes fdtd_ctx_upload_material");
   if (which < 0 || which >= 18) return fail(FDTD_ERR_BADARG, "coefficient id %d out of range 0..17", which);
   if (n != coef_count(c, which)) return fail(FDTD_ERR_BADARG, "coefficient %d: got %ld values, expected %lld", which, n, coef_count(c, which));
@@ -1526,6 +1530,7 @@ int fdtd_ctx_upload_cpml(fdtd_ctx* c, int f, int nc, const double* b_e, const do
                          long n0, const double* CPsi1, long n1, const double* CPsi2, long n2, const double* CPsi3,
                          long n3, int m_start, int e_start) {
   if (!c) return fail(FDTD_ERR_BADARG, "NULL handle");
+  Using use(c->mu);
   if (f < 0 || f >= 6) return fail(FDTD_ERR_BADARG, "face id %d out of range 0..5", f);
   if (nc < 0) return fail(FDTD_ERR_BADARG, "negative cell count");
   const int axis_n = f / 2 == 0 ? c->nx : (f / 2 == 1 ? c->ny : c->nz);
@@ -1601,6 +1606,7 @@ int fdtd_ctx_upload_cpml(fdtd_ctx* c, int f, int nc, const double* b_e, const do
 int fdtd_ctx_add_vsource(fdtd_ctx* c, int dir, const int* idx, const double* coef, int count, const double* wave,
                          int nSteps) {
   if (!c || !idx || !coef || !wave) return fail(FDTD_ERR_BADARG, "NULL argument");
+  Using use(c->mu);
   if (dir < 0 || dir > 2) return fail(FDTD_ERR_BADARG, "source direction %d not in 0..2", dir);
   if (count <= 0) return fail(FDTD_ERR_BADARG, "source has no cells");
   if (nSteps < c->nsteps) return fail(FDTD_ERR_BADARG, "waveform has %d values, need %d", nSteps, c->nsteps);
@@ -1647,6 +1653,7 @@ int fdtd_ctx_add_vsource(fdtd_ctx* c, int dir, const int* idx, const double* coe
 
 int fdtd_ctx_add_svoltage(fdtd_ctx* c, int dir, const int* idx, int count, double Csvf) {
   if (!c || !idx) return fail(FDTD_ERR_BADARG, "NULL argument");
+  Using use(c->mu);
   if (dir < 0 || dir > 2) return fail(FDTD_ERR_BADARG, "probe direction %d not in 0..2", dir);
   if (count <= 0) return fail(FDTD_ERR_BADARG, "probe has no cells");
   if ((int)c->vprobe.size() >= kMaxProbes) return fail(FDTD_ERR_BADARG, "at most %d voltage probes", kMaxProbes);
@@ -1668,6 +1675,7 @@ int fdtd_ctx_add_svoltage(fdtd_ctx* c, int dir, const int* idx, int count, doubl
 
 int fdtd_ctx_add_scurrent(fdtd_ctx* c, const int* comp, const int* idx, const double* w, int count) {
   if (!c || !comp || !idx || !w) return fail(FDTD_ERR_BADARG, "NULL argument");
+  Using use(c->mu);
   if (count <= 0) return fail(FDTD_ERR_BADARG, "probe has no samples");
   if ((int)c->iprobe.size() >= kMaxProbes) return fail(FDTD_ERR_BADARG, "at most %d current probes", kMaxProbes);
   for (int q = 0; q < count; q++) {
@@ -1697,6 +1705,7 @@ int fdtd_ctx_add_scurrent(fdtd_ctx* c, const int* comp, const int* idx, const do
 int fdtd_ctx_setup_farfield(fdtd_ctx* c, int nFreq, const double* freqs, int li, int lj, int lk, int ui, int uj,
                             int uk) {
   if (!c) return fail(FDTD_ERR_BADARG, "NULL handle");
+  Using use(c->mu);
   if (nFreq < 0 || (nFreq > 0 && !freqs)) return fail(FDTD_ERR_BADARG, "bad frequency list");
   if (c->nFreq > 0) return fail(FDTD_ERR_STATE, "far field already set up");
   if (nFreq == 0) return FDTD_OK;
@@ -1742,6 +1751,7 @@ int fdtd_ctx_setup_farfield(fdtd_ctx* c, int nFreq, const double* freqs, int li,
 
 int fdtd_ctx_upload_material(fdtd_ctx* c, int comp, const unsigned char* ids, long n, const double* table, int rows) {
   if (!c || !ids || !table) return fail(FDTD_ERR_BADARG, "NULL argument");
+  Using use(c->mu);
   if (c->prec != FDTD_PREC_F32_TABLE) return fail(FDTD_ERR_STATE, "not a material-table problem");
   if (comp < 0 || comp > 5) return fail(FDTD_ERR_BADARG, "component %d not in 0..5", comp);
   const long long want = c->ncomp[(comp + 3) % 6];
@@ -1794,6 +1804,7 @@ static int set_rows(fdtd_ctx* c, int comp, const std::vector<double>& rows) {
 int fdtd_ctx_build_material(fdtd_ctx* c, const unsigned char* mat, long ncells, int ntypes, const double* props,
                             int nplates, const int* plates, const double* plate_sigma) {
   if (!c || !mat || !props || (nplates > 0 && (!plates || !plate_sigma))) return fail(FDTD_ERR_BADARG, "NULL argument");
+  Using use(c->mu);
   if (c->prec == FDTD_PREC_F32)
     return fail(FDTD_ERR_STATE, "per-cell FP32 problems take fdtd_ctx_upload_coeff (FP64 and material-table problems build here)");
   const bool f64 = c->prec == FDTD_PREC_F64;
@@ -1974,6 +1985,7 @@ static int override_coef64(fdtd_ctx* c, int comp, const int* idx, const double* 
 
 int fdtd_ctx_override_material(fdtd_ctx* c, int comp, const int* idx, const double* triples, int count) {
   if (!c || !idx || !triples) return fail(FDTD_ERR_BADARG, "NULL argument");
+  Using use(c->mu);
   if (count > 0) {
     digest_vals(c, 10, {(double)comp, (double)count});
     digest(c, 10, idx, (size_t)count * sizeof(int));
@@ -2022,6 +2034,7 @@ int fdtd_ctx_run(fdtd_ctx* c, int count) {
 
 int fdtd_ctx_set_prefetch(fdtd_ctx* c, int planes) {
   if (!c) return fail(FDTD_ERR_BADARG, "NULL handle");
+  Using use(c->mu);
   if (planes < 1 || planes > 5) return fail(FDTD_ERR_BADARG, "prefetch depth %d not in 1..5", planes);
   if (planes > 2 && c->prec != FDTD_PREC_F32_TABLE)
     return fail(FDTD_ERR_BADARG, "prefetch modes 3..5 (shared-memory stages) need a material-table problem");
@@ -2032,6 +2045,7 @@ int fdtd_ctx_set_prefetch(fdtd_ctx* c, int planes) {
 
 int fdtd_ctx_set_tiling(fdtd_ctx* c, int x_planes_per_thread, int block_rows) {
   if (!c) return fail(FDTD_ERR_BADARG, "NULL handle");
+  Using use(c->mu);
   if (x_planes_per_thread < 1 || x_planes_per_thread > c->nx + 1)
     return fail(FDTD_ERR_BADARG, "x planes per thread %d not in 1..%d", x_planes_per_thread, c->nx + 1);
   if (block_rows != 1 && block_rows != 2 && block_rows != 4 && block_rows != 8 && block_rows != 16)
@@ -2044,6 +2058,7 @@ int fdtd_ctx_set_tiling(fdtd_ctx* c, int x_planes_per_thread, int block_rows) {
 
 int fdtd_ctx_set_block_width(fdtd_ctx* c, int threads_along_k) {
   if (!c) return fail(FDTD_ERR_BADARG, "NULL handle");
+  Using use(c->mu);
   if (threads_along_k != 16 && threads_along_k != 32)
     return fail(FDTD_ERR_BADARG, "block width %d not 16 or 32", threads_along_k);
   c->block_w = threads_along_k;
@@ -2197,6 +2212,7 @@ StateHeader state_header(fdtd_ctx* c) {
 
 int fdtd_ctx_state_size(fdtd_ctx* c, long long* bytes) {
   if (!c || !bytes) return fail(FDTD_ERR_BADARG, "NULL argument");
+  Using use(c->mu);
   int rc = ensure_traces(c);
   if (rc) return rc;
   *bytes = state_header(c).bytes;
@@ -2205,12 +2221,12 @@ int fdtd_ctx_state_size(fdtd_ctx* c, long long* bytes) {
 
 int fdtd_ctx_save_state(fdtd_ctx* c, void* buf, long long bytes) {
   if (!c || !buf) return fail(FDTD_ERR_BADARG, "NULL argument");
+  Using use(c->mu);
   CK(cudaSetDevice(c->device));
   int rc = ensure_traces(c);
   if (rc) return rc;
   const StateHeader h = state_header(c);
   if (bytes != h.bytes) return fail(FDTD_ERR_BADARG, "state buffer of %lld bytes, need %lld", bytes, h.bytes);
-  Using use(c->mu);
   rc = to_dense(c);
   if (rc) return rc;
   char* p = (char*)buf;
@@ -2226,6 +2242,7 @@ int fdtd_ctx_save_state(fdtd_ctx* c, void* buf, long long bytes) {
 
 int fdtd_ctx_load_state(fdtd_ctx* c, const void* buf, long long bytes) {
   if (!c || !buf) return fail(FDTD_ERR_BADARG, "NULL argument");
+  Using use(c->mu);
   CK(cudaSetDevice(c->device));
   int rc = ensure_traces(c);
   if (rc) return rc;
@@ -2241,7 +2258,6 @@ int fdtd_ctx_load_state(fdtd_ctx* c, const void* buf, long long bytes) {
     return fail(FDTD_ERR_BADARG, "state was saved from a problem of another shape, precision or probe set");
   if (theirs.ts < 0 || theirs.ts > c->nsteps) return fail(FDTD_ERR_BADARG, "state step %d out of range", theirs.ts);
   const char* p = (const char*)buf + sizeof(StateHeader);
-  Using use(c->mu);
   c->dense_valid = true;   // every value of the state is replaced
   c->fs.valid = false;
   for (auto& q : state_ranges(c)) {
@@ -2259,6 +2275,7 @@ int fdtd_ctx_load_state(fdtd_ctx* c, const void* buf, long long bytes) {
 
 int fdtd_ctx_set_dft_block(fdtd_ctx* c, int steps) {
   if (!c) return fail(FDTD_ERR_BADARG, "NULL handle");
+  Using use(c->mu);
   if (steps < 0 || steps == 1 || steps > 1024) return fail(FDTD_ERR_BADARG, "DFT block of %d steps not in {0, 2..1024}", steps);
   if (steps && c->prec == FDTD_PREC_F64) return fail(FDTD_ERR_BADARG, "FP64 problems keep the per-step DFT");
   if (steps && c->nFreq == 0) return fail(FDTD_ERR_STATE, "no far field set up");
@@ -2280,6 +2297,7 @@ int fdtd_ctx_set_dft_block(fdtd_ctx* c, int steps) {
 
 int fdtd_ctx_set_dft_accumulator(fdtd_ctx* c, int kahan_fp32) {
   if (!c) return fail(FDTD_ERR_BADARG, "NULL handle");
+  Using use(c->mu);
   if (kahan_fp32 != 0 && kahan_fp32 != 1) return fail(FDTD_ERR_BADARG, "accumulator mode %d not in {0,1}", kahan_fp32);
   if (kahan_fp32 && c->prec == FDTD_PREC_F64) return fail(FDTD_ERR_BADARG, "FP64 problems keep FP64 accumulators");
   if (c->ts != 0) return fail(FDTD_ERR_STATE, "the accumulator mode is set before the first step");
@@ -2290,6 +2308,7 @@ int fdtd_ctx_set_dft_accumulator(fdtd_ctx* c, int kahan_fp32) {
 
 int fdtd_ctx_set_x_wall(fdtd_ctx* c, int wall) {
   if (!c) return fail(FDTD_ERR_BADARG, "NULL handle");
+  Using use(c->mu);
   if (wall != 0 && wall != 1) return fail(FDTD_ERR_BADARG, "x wall mode %d not in {0,1}", wall);
   c->x_wall = wall;
   invalidate(c);
@@ -3051,8 +3070,11 @@ int batch_run_members(fdtd_batch* b, int count, bool chain, float* elapsed_ms, K
 
 int batch_run(fdtd_batch* b, int count, float* elapsed_ms = nullptr, KernelTimer* tm = nullptr) {
   if (count < 0) return fail(FDTD_ERR_BADARG, "negative step count %d", count);
+  // in one order for all batches, as two with members in common may run at once
+  std::vector<fdtd_ctx*> order = b->m;
+  std::sort(order.begin(), order.end(), std::less<fdtd_ctx*>());
   std::vector<std::unique_lock<std::recursive_mutex>> use;
-  for (fdtd_ctx* c : b->m) use.emplace_back(c->mu);
+  for (fdtd_ctx* c : order) use.emplace_back(c->mu);
   const int ts = b->m[0]->ts;
   for (size_t q = 0; q < b->m.size(); q++) {
     fdtd_ctx* c = b->m[q];
