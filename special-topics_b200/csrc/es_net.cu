@@ -399,11 +399,8 @@ namespace {
 
 int es_alloc(fdtd_es_net* n, void** p, size_t bytes) {
   if (bytes == 0) bytes = 16;
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e != cudaSuccess) {
-    *p = nullptr;
-    return es_fail(FDTD_ERR_OOM, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
-  }
+  cudaError_t e = fdtd_internal_malloc(n->cfg.device, p, bytes);
+  if (e != cudaSuccess) return es_fail(FDTD_ERR_OOM, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
   n->owned.push_back(*p);
   e = cudaMemsetAsync(*p, 0, bytes, n->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(n->stream);

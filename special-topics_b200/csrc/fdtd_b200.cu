@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstdarg>
 #include <cstddef>
@@ -14,6 +16,7 @@
 #include <initializer_list>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/fdtd_b200.h"
@@ -40,6 +43,12 @@ static int fail(int code, const char* fmt, ...) {
   va_end(ap);
   return code;
 }
+
+namespace {
+cudaError_t dev_malloc(int device, void** p, size_t bytes);
+}
+
+cudaError_t fdtd_internal_malloc(int device, void** p, size_t bytes) { return dev_malloc(device, p, bytes); }
 
 int fdtd_internal_fail(int code, const char* msg) { return fail(code, "%s", msg); }
 
@@ -182,6 +191,8 @@ struct fdtd_ctx {
   // order.  A saved state carries it and loads only where it matches.
   unsigned long long setup_digest = 0x6a09e667f3bcc908ULL;
   std::recursive_mutex mu;  // held by every call that touches the set-up, the graphs or `fs`, see reclaim_padded
+  std::atomic<bool> padded{false};  // `fs` holds memory
+  std::atomic<bool> wanted{false};  // another thread waits for that memory
 };
 
 namespace {
@@ -201,32 +212,54 @@ Handles& handles() {
   return *h;
 }
 
-// Another handle on c's device gives up its padded state (its next run builds it
-// again, or takes the half-step path): without it, a problem that fits beside the
-// dense arrays of the others would not.  A handle that is in a call keeps its own.
-// False: none had any.
-bool reclaim_padded(const fdtd_ctx* c) {
-  std::lock_guard<std::mutex> g(handles().mu);
-  for (fdtd_ctx* o : handles().all) {
-    if (o == c || o->device != c->device) continue;
-    std::unique_lock<std::recursive_mutex> use(o->mu, std::try_to_lock);
-    if (use.owns_lock() && !o->fs.owned.empty() && to_dense(o) == FDTD_OK && fused_drop(o) == FDTD_OK) return true;
+// A handle on the device gives up its padded state (a later run builds it again,
+// or takes the half-step path): without it, what fits beside the dense arrays of
+// the handles would not.  A handle in another thread's call is asked to, and
+// waited for: it does at its next run, or is idle by then.  A handle in a call of
+// this thread gives up its own; no call allocates through here between making its
+// padded state current and launching on it.  False: none had any.
+bool reclaim_padded(int device) {
+  constexpr int kWaitMs = 60000;
+  for (int waited = 0;; waited++) {
+    bool busy = false;
+    {
+      std::lock_guard<std::mutex> g(handles().mu);
+      for (fdtd_ctx* o : handles().all) {
+        if (o->device != device || !o->padded) continue;
+        std::unique_lock<std::recursive_mutex> use(o->mu, std::try_to_lock);
+        if (!use.owns_lock())
+          o->wanted = busy = true;
+        else if (fused_drop(o) == FDTD_OK)
+          return true;
+      }
+    }
+    if (!busy) return waited > 0;  // given up meanwhile
+    if (waited >= kWaitMs) return false;
+    std::this_thread::sleep_for(std::chrono::milliseconds(1));
   }
-  return false;
+}
+
+// cudaMalloc on the current device, `device`, that takes back padded states while
+// memory is short.  Every allocation of the library but the padded states' own.
+cudaError_t dev_malloc(int device, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  for (int tries = 0; e == cudaErrorMemoryAllocation && tries < 1000; tries++) {
+    cudaGetLastError();
+    if (!reclaim_padded(device)) break;
+    e = cudaMalloc(p, bytes);
+  }
+  if (e != cudaSuccess) *p = nullptr;
+  return e;
+}
+template <typename V>
+cudaError_t dev_malloc(const fdtd_ctx* c, V** p, size_t bytes) {
+  return dev_malloc(c->device, (void**)p, bytes);
 }
 
 int dalloc(fdtd_ctx* c, void** p, size_t bytes) {
   if (bytes == 0) bytes = 16;
-  cudaError_t e = cudaMalloc(p, bytes);
-  while (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    if (!reclaim_padded(c)) break;
-    e = cudaMalloc(p, bytes);
-  }
-  if (e != cudaSuccess) {
-    *p = nullptr;
-    return fail(FDTD_ERR_OOM, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
-  }
+  cudaError_t e = dev_malloc(c, p, bytes);
+  if (e != cudaSuccess) return fail(FDTD_ERR_OOM, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
   c->owned.push_back(*p);
   // Zero on the handle's stream and wait: later uploads may use either stream,
   // and the zeroing must not land after them.
@@ -643,6 +676,7 @@ int fused_alloc(fdtd_ctx* c, void** p, size_t bytes) {
     return FDTD_ERR_OOM;
   }
   c->fs.owned.push_back(*p);
+  c->padded = true;
   CK(cudaMemsetAsync(*p, 0, bytes, c->stream));
   return FDTD_OK;
 }
@@ -719,6 +753,7 @@ int claim_dense(fdtd_ctx* c) {
 void fused_free(fdtd_ctx* c) {
   for (void* p : c->fs.owned) cudaFree(p);
   c->fs = FusedState();
+  c->padded = c->wanted = false;
 }
 
 // Frees the padded state (after saving what it holds): the set-up changes.
@@ -896,10 +931,11 @@ int fused_build(fdtd_ctx* c) {
   return rc;
 }
 
-// Makes the padded state hold the current step; *use = false: half-step path.
+// Builds the padded state where there is none; *use = false: half-step path.
 int fused_usable(fdtd_ctx* c, bool* use) {
   FusedState& fs = c->fs;
   *use = false;
+  if (c->wanted) return fused_drop(c);  // this run takes the half-step path, a later one builds again
   if (!fs.tried) {
     int rc = fused_build(c);
     if (rc || !fs.ok) {
@@ -914,7 +950,7 @@ int fused_usable(fdtd_ctx* c, bool* use) {
   return FDTD_OK;
 }
 
-// And makes it hold the current fields and step.
+// And makes it hold the current fields and step, where the one-pass step is used.
 int fused_ready(fdtd_ctx* c, bool* use) {
   FusedState& fs = c->fs;
   int rc = fused_usable(c, use);
@@ -1259,10 +1295,11 @@ int run_steps(fdtd_ctx* c, int count, float* elapsed_ms = nullptr, KernelTimer* 
   }
   std::vector<cudaGraphExec_t> plan;
   if (!tm && fused) {
-    // a graph depends on the copy it starts from and on where DFT blocks close
+    // a graph depends on the copy it starts from and on where DFT blocks close;
+    // tag 0 is the half-step path
     const int per = c->dft_block > 0 ? c->dft_block : 1;
     rc = run_plan(c->graphs, c->stream, count, 3, [c](int n) { return fused_enqueue(c, n); }, &plan, 2 * per,
-                  2 * (c->ts % per) + c->fs.cur);
+                  2 * (c->ts % per) + c->fs.cur + 1);
     if (rc) return rc;
   } else if (!tm) {
     rc = run_plan(c->graphs, c->stream, count, c->dft_block > 0 ? 5 : 4,
@@ -1502,7 +1539,7 @@ static int cpml_band_on_device(fdtd_ctx* c, int f, const double* kappa_e, const 
   HostFace& h = c->face[f];
   const double cell = axis == 0 ? c->dx : (axis == 1 ? c->dy : c->dz);
   double* d_kap = nullptr;
-  if (cudaMalloc((void**)&d_kap, 2 * h.nc * sizeof(double)) != cudaSuccess) return fail(FDTD_ERR_OOM, "kappa profiles");
+  if (dev_malloc(c, &d_kap, 2 * h.nc * sizeof(double)) != cudaSuccess) return fail(FDTD_ERR_OOM, "kappa profiles");
   int rc = FDTD_OK;
   if (xfer(c, d_kap, kappa_e, h.nc * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
       xfer(c, d_kap + h.nc, kappa_m, h.nc * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
@@ -1847,9 +1884,10 @@ int fdtd_ctx_build_material(fdtd_ctx* c, const unsigned char* mat, long ncells, 
   const long long ncode_e = (M * M * M * M + 1) * (long long)(psig.size() + 1);
   const long long ncode_h = M * M + 1;
   int rc = FDTD_OK;
-  if (cudaMalloc(&d_mat, ncells) != cudaSuccess || cudaMalloc(&d_present, std::max(ncode_e, ncode_h)) != cudaSuccess ||
-      cudaMalloc(&d_map, std::max(ncode_e, ncode_h)) != cudaSuccess ||
-      (f64 && cudaMalloc((void**)&d_map64, std::max(ncode_e, ncode_h) * sizeof(int)) != cudaSuccess)) {
+  if (dev_malloc(c, &d_mat, ncells) != cudaSuccess ||
+      dev_malloc(c, &d_present, std::max(ncode_e, ncode_h)) != cudaSuccess ||
+      dev_malloc(c, &d_map, std::max(ncode_e, ncode_h)) != cudaSuccess ||
+      (f64 && dev_malloc(c, &d_map64, std::max(ncode_e, ncode_h) * sizeof(int)) != cudaSuccess)) {
     rc = fail(FDTD_ERR_OOM, "material build buffers");
   }
   if (!rc && xfer(c, d_mat, mat, ncells, cudaMemcpyHostToDevice) != cudaSuccess) rc = fail(FDTD_ERR_CUDA, "material grid upload");
@@ -1913,7 +1951,7 @@ int fdtd_ctx_build_material(fdtd_ctx* c, const unsigned char* mat, long ncells, 
       const std::vector<int>& map64 = row_of_code;
       cudaFree(d_rows);
       d_rows = nullptr;
-      if (cudaMalloc((void**)&d_rows, std::max<size_t>(rows.size(), 1) * sizeof(double)) != cudaSuccess) {
+      if (dev_malloc(c, &d_rows, std::max<size_t>(rows.size(), 1) * sizeof(double)) != cudaSuccess) {
         rc = fail(FDTD_ERR_OOM, "coefficient rows");
         break;
       }
@@ -1965,8 +2003,8 @@ static int override_coef64(fdtd_ctx* c, int comp, const int* idx, const double* 
   int* d_idx = nullptr;
   double* d_trip = nullptr;
   int rc = FDTD_OK;
-  if (cudaMalloc((void**)&d_idx, count * sizeof(int)) != cudaSuccess ||
-      cudaMalloc((void**)&d_trip, 3 * count * sizeof(double)) != cudaSuccess)
+  if (dev_malloc(c, &d_idx, count * sizeof(int)) != cudaSuccess ||
+      dev_malloc(c, &d_trip, 3 * count * sizeof(double)) != cudaSuccess)
     rc = fail(FDTD_ERR_OOM, "override buffers");
   if (!rc && (xfer(c, d_idx, idx, count * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
               xfer(c, d_trip, triples, 3 * count * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess))
@@ -2354,9 +2392,11 @@ __global__ void __launch_bounds__(256) k_dft(const double* x, int N, double dt, 
 int fdtd_dft(const double* x, int N, double dt, const double* freqs, int M, double shift, double* re, double* im) {
   if (!x || !freqs || !re || !im || N <= 0 || M <= 0) return fail(FDTD_ERR_BADARG, "bad DFT arguments");
   double *dx_ = nullptr, *df = nullptr, *dr = nullptr;
-  int rc = FDTD_OK;
-  if (cudaMalloc(&dx_, N * sizeof(double)) != cudaSuccess || cudaMalloc(&df, M * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&dr, 2 * M * sizeof(double)) != cudaSuccess) {
+  int rc = FDTD_OK, dev = 0;
+  CK(cudaGetDevice(&dev));
+  if (dev_malloc(dev, (void**)&dx_, N * sizeof(double)) != cudaSuccess ||
+      dev_malloc(dev, (void**)&df, M * sizeof(double)) != cudaSuccess ||
+      dev_malloc(dev, (void**)&dr, 2 * M * sizeof(double)) != cudaSuccess) {
     rc = fail(FDTD_ERR_OOM, "DFT buffers");
   } else if (cudaMemcpy(dx_, x, N * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
              cudaMemcpy(df, freqs, M * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
@@ -2431,7 +2471,7 @@ int fdtd_ctx_farfield_post(fdtd_ctx* c, const double* theta, const double* phi, 
   double* conv = nullptr;
   if (c->acc_kahan) {
     const long long n = c->ffoff[23] + 2LL * c->nFreq * c->ffsz[2];
-    if (cudaMalloc(&conv, n * sizeof(double)) != cudaSuccess) return fail(FDTD_ERR_OOM, "far-field post buffer");
+    if (dev_malloc(c, &conv, n * sizeof(double)) != cudaSuccess) return fail(FDTD_ERR_OOM, "far-field post buffer");
     k_kahan_to_f64<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->acc, conv, n);
     P.acc = conv;
   }
@@ -2483,10 +2523,13 @@ int fdtd_ctx_farfield_post(fdtd_ctx* c, const double* theta, const double* phi, 
     n_rows = R * 8 * th;
     n_z = (size_t)parts * 8 * ang;
     fb = (int)std::min<size_t>(F, std::max<size_t>(1, room / std::max<size_t>(1, n_rows + n_z)));
-    if (cudaMalloc(&buf, (n_out + fb * (n_rows + n_z) + cth.size() + na) * sizeof(double)) != cudaSuccess) {
+    // the smallest form is worth other handles' padded state, the larger ones are not
+    const size_t bytes = (n_out + fb * (n_rows + n_z) + cth.size() + na) * sizeof(double);
+    const bool least = room < 65536;
+    if ((least ? dev_malloc(c, &buf, bytes) : cudaMalloc(&buf, bytes)) != cudaSuccess) {
       cudaGetLastError();
       buf = nullptr;
-      if (room < 65536) {
+      if (least) {
         rc = fail(FDTD_ERR_OOM, "far-field post buffers");
         break;
       }
@@ -2661,7 +2704,7 @@ int upload_vec(fdtd_batch* b, V** dst, const std::vector<V>& v) {
   if (*dst) cudaFree(*dst);
   *dst = nullptr;
   const size_t bytes = std::max<size_t>(v.size(), 1) * sizeof(V);
-  CK(cudaMalloc((void**)dst, bytes));
+  CK(dev_malloc(b->device, (void**)dst, bytes));
   if (!v.empty()) CK(cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice, b->stream));
   CK(cudaStreamSynchronize(b->stream));
   return FDTD_OK;
@@ -2764,7 +2807,7 @@ int batch_prepare(fdtd_batch* b, C (*coef_of)(fdtd_ctx*)) {
   if (!b->d_inst || b->inst_size != sizeof(In)) {
     if (b->d_inst) cudaFree(b->d_inst);
     b->d_inst = nullptr;
-    CK(cudaMalloc(&b->d_inst, host.size()));
+    CK(dev_malloc(b->device, &b->d_inst, host.size()));
     b->inst_size = sizeof(In);
   }
   CK(cudaMemcpyAsync(b->d_inst, host.data(), host.size(), cudaMemcpyHostToDevice, b->stream));
@@ -2983,12 +3026,17 @@ int batch_chain_enqueue(fdtd_batch* b, int count) {
 // together); then makes them hold the current state in that form.
 int batch_chain_ready(fdtd_batch* b, bool* use) {
   *use = b->streams == 0;
+  for (const fdtd_ctx* c : b->m) *use = *use && c->dft_block == b->m[0]->dft_block && (c->fs.ok || !c->fs.tried);
+  std::vector<fdtd_ctx*> built;
   for (size_t q = 0; q < b->m.size() && *use; q++) {
-    *use = b->m[q]->dft_block == b->m[0]->dft_block;
-    if (!*use) break;
+    const bool had = b->m[q]->fs.ok;
     int rc = fused_usable(b->m[q], use);
     if (rc) return rc;
+    if (!had && *use) built.push_back(b->m[q]);
   }
+  if (!*use)  // built in vain
+    for (fdtd_ctx* c : built)
+      if (int rc = fused_drop(c)) return rc;
   for (size_t q = 0; q < b->m.size() && *use; q++) {
     fdtd_ctx* c = b->m[q];
     int rc = fused_ready(c, use);
@@ -3168,7 +3216,7 @@ int fdtd_batch_create(fdtd_ctx* const* members, int count, fdtd_batch** out) {
     return fail(FDTD_ERR_CUDA, "cannot create a stream on device %d", members[0]->device);
   }
   BatchCtl zero{};
-  if (cudaMalloc((void**)&b->d_ctl, sizeof(BatchCtl)) != cudaSuccess ||
+  if (dev_malloc(b->device, (void**)&b->d_ctl, sizeof(BatchCtl)) != cudaSuccess ||
       cudaMemcpyAsync(b->d_ctl, &zero, sizeof(BatchCtl), cudaMemcpyHostToDevice, b->stream) != cudaSuccess ||
       cudaStreamSynchronize(b->stream) != cudaSuccess) {
     fdtd_batch_free(b);

@@ -1,7 +1,10 @@
 // fdtd_internal.h -- what the library's translation units share and do not
-// export: the thread-local error message behind fdtd_last_error() and the
-// device port traces of a handle.
+// export: the thread-local error message behind fdtd_last_error(), device
+// memory and the device port traces of a handle.
 #pragma once
+#include <cstddef>
+
+#include <cuda_runtime.h>
 
 struct fdtd_ctx;
 
@@ -14,3 +17,7 @@ __attribute__((visibility("hidden"))) int fdtd_internal_fail(int code, const cha
 __attribute__((visibility("hidden"))) int fdtd_internal_traces(const fdtd_ctx* c, const double** V,
                                                                const double** I, int* nsteps, int* steps,
                                                                int* device);
+
+// cudaMalloc on the current device, `device`; while memory is short, handles there
+// give back what they hold for speed alone.  *p = NULL on failure.
+__attribute__((visibility("hidden"))) cudaError_t fdtd_internal_malloc(int device, void** p, size_t bytes);

@@ -17,7 +17,8 @@ from test_gpu_one_pass import _assert_same, _state
 pkg = load_package()
 from special_topics_b200 import _native as N  # noqa: E402
 from special_topics_b200 import autotune  # noqa: E402
-from special_topics_b200.backend import Engine  # noqa: E402
+from special_topics_b200 import earlystop as ES  # noqa: E402
+from special_topics_b200.backend import Batch, Engine  # noqa: E402
 from special_topics_b200.scenario import build_problem_from_scenario  # noqa: E402
 from special_topics_b200.workloads import scaling_box  # noqa: E402
 
@@ -111,3 +112,85 @@ def test_settings_beside_another_threads_reclaim():
     with Engine(p, "f32-table") as a:
         a.run(ran)
         _assert_same(_state(a), got)
+
+
+def test_a_handle_fits_beside_one_that_is_running():
+    """The first handle is in one run after another in another thread."""
+    steps = 20000
+    p, q, keeps, need = _sizes(steps)
+    left = keeps + 8 * MB
+    assert left < need < left + keeps
+    done, ran, errors = threading.Event(), [64], []
+
+    def other(a):
+        try:
+            while not done.is_set() and ran[0] + 500 <= steps:
+                a.run(500)
+                ran[0] += 500
+        except Exception as e:      # noqa: BLE001
+            errors.append(e)
+
+    with Engine(p, "f32-table") as a:
+        a.run(64)
+        with _only(left):
+            t = threading.Thread(target=other, args=(a,))
+            t.start()
+            try:
+                for _ in range(3):
+                    with Engine(q, "f32-table") as b:
+                        b.run(3)
+            finally:
+                done.set()
+                t.join()
+        got = _state(a)
+    assert not errors
+    with Engine(p, "f32-table") as a:
+        a.run(ran[0])
+        _assert_same(_state(a), got)
+
+
+def _dft_block(eng):
+    N.check(N.lib().fdtd_ctx_set_dft_block(eng._h, 64))          # 64 steps' samples: some 80 MB
+
+
+def _network(eng):
+    ES.EsNet(out_dim=4, max_batch=256).close()
+
+
+def _material(eng):
+    eng._build_tables_on_device()                                # one byte per cell
+
+
+@pytest.mark.parametrize("act,left", [(_dft_block, 24 * MB), (_network, 24 * MB), (_material, 2 * MB)],
+                         ids=["samples", "network", "material"])
+def test_calls_that_need_memory_after_a_run(act, left):
+    """What the handle itself keeps is given up too."""
+    p = _box(152, 200)
+    out = []
+    for short in (False, True):
+        with Engine(p, "f32-table") as a:
+            a.run(64)
+            if short:
+                with _only(left):
+                    act(a)
+            else:
+                need, _ = _cost(lambda: act(a))
+                assert act is not _dft_block or need > left
+            a.run(64)
+            out.append(_state(a))
+    _assert_same(*out)
+
+
+def test_copies_built_for_a_batch_that_cannot_use_them_are_freed():
+    """The second member's copies do not fit, so the batch takes the tile list
+    and the first member keeps none."""
+    p, q = _box(64, 200), _box(128, 200)
+    with Engine(q, "f32-table") as b:
+        keeps, _ = _cost(lambda: b.run(64))
+    with Engine(p, "f32-table") as a, Engine(q, "f32-table") as b, Batch([a, b]) as batch:
+        with _only(keeps):
+            held, _ = _cost(lambda: batch.run(128))
+            assert batch.profile_kernels(1)["e"] > 0
+    with Engine(p, "f32-table") as a:
+        kept, _ = _cost(lambda: a.run(128))
+    assert held < kept
