@@ -2318,6 +2318,9 @@ int fdtd_ctx_set_dft_block(fdtd_ctx* c, int steps) {
   if (steps && c->prec == FDTD_PREC_F64) return fail(FDTD_ERR_BADARG, "FP64 problems keep the per-step DFT");
   if (steps && c->nFreq == 0) return fail(FDTD_ERR_STATE, "no far field set up");
   CK(cudaSetDevice(c->device));
+  // without a block until the buffer is there: no graph keeps the old one's address
+  c->dft_block = 0;
+  invalidate(c);
   if (steps) {
     dfree(c, c->dft_samples);
     c->dft_samples = nullptr;
@@ -2329,7 +2332,6 @@ int fdtd_ctx_set_dft_block(fdtd_ctx* c, int steps) {
     CK(xfer(c, c->d_dft_done, &c->ts, sizeof(int), cudaMemcpyHostToDevice));
   }
   c->dft_block = steps;
-  invalidate(c);
   return FDTD_OK;
 }
 

@@ -194,3 +194,19 @@ def test_copies_built_for_a_batch_that_cannot_use_them_are_freed():
     with Engine(p, "f32-table") as a:
         kept, _ = _cost(lambda: a.run(128))
     assert held < kept
+
+
+def test_a_dft_block_that_does_not_fit_leaves_per_step_sums():
+    """The old block's buffer is gone by then, so the sums are per step from there."""
+    p = _box(128, 200)
+    with Engine(p, "f32-table", dft_accumulator="kahan-f32", dft_block=16) as a:
+        a.run(64)
+        with _only(64 * MB):
+            with pytest.raises(N.FdtdError) as ei:
+                N.check(N.lib().fdtd_ctx_set_dft_block(a._h, 1024))
+            assert ei.value.code == N.FDTD_ERR_OOM
+        a.run(64)
+        got = _state(a)
+    with Engine(p, "f32-table", dft_accumulator="kahan-f32") as a:
+        a.run(128)
+        _assert_same(_state(a), got)
