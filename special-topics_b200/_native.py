@@ -15,7 +15,8 @@ LIB_PATH = os.path.join(BUILD_DIR, "libfdtd_b200.so")
 SOURCES = [os.path.join(PKG_DIR, "csrc", f) for f in
            ("fdtd_b200.cu", "fdtd_fused.cu", "fdtd_half_f64.cu", "fdtd_half_f32.cu",
             "fdtd_half_table.cu", "es_net.cu", "fdtd_common.cuh", "fdtd_step.cuh", "fdtd_material.cuh",
-            "fdtd_batch.cuh", "fdtd_internal.h", "fdtd_ffpost.cuh", "fdtd_fused.cuh", "fdtd_half.cuh")]
+            "fdtd_batch.cuh", "fdtd_internal.h", "fdtd_ffpost.cuh", "fdtd_fused.cuh", "fdtd_half.cuh",
+            "run_plan.h")]
 CU_SOURCES = [p for p in SOURCES if p.endswith(".cu")]
 HEADER = os.path.join(ROOT, "include", "fdtd_b200.h")
 

@@ -28,6 +28,7 @@
 #include "fdtd_fused.cuh"
 #include "fdtd_half.cuh"
 #include "fdtd_internal.h"
+#include "run_plan.h"
 
 #include <map>
 #include <utility>
@@ -102,10 +103,10 @@ struct HostIProbe {
 // timed region.  A handful of counts is kept (early-stop runs advance in
 // checkpoints of a few different lengths).
 struct RunGraphs {
-  std::vector<std::pair<long long, cudaGraphExec_t>> g;  // key: steps, and a tag of the state it starts from
+  GraphCache<cudaGraphExec_t> cache;  // key: steps, and a tag of the state it starts from
   void clear() {
-    for (auto& e : g) cudaGraphExecDestroy(e.second);
-    g.clear();
+    for (auto& e : cache.g) cudaGraphExecDestroy(e.exec);
+    cache.g.clear();
     rev++;
   }
   long long rev = 0;  // times cleared: what else captured the same set-up is stale then
@@ -1194,21 +1195,15 @@ int close_dft_block(fdtd_ctx* c, int upto, cudaStream_t st) {
 
 constexpr int kGraphSteps = 64;       // shortest graph (and the cap's floor)
 constexpr int kMaxGraphNodes = 40000;  // kernel launches held by one graph at most
-constexpr size_t kMaxCachedGraphs = 6;
 
 // The graph of `steps` steps from the cache, captured on `st` through `enq`
 // (which enqueues that many steps) when missing.
 template <class Enq>
 int graph_for(RunGraphs& rg, cudaStream_t st, int steps, int tag, Enq enq, cudaGraphExec_t* out) {
   const long long key = (long long)steps << 16 | tag;
-  for (auto& e : rg.g)
-    if (e.first == key) {
-      *out = e.second;
-      return FDTD_OK;
-    }
-  if (rg.g.size() >= kMaxCachedGraphs) {
-    cudaGraphExecDestroy(rg.g.front().second);
-    rg.g.erase(rg.g.begin());
+  if (cudaGraphExec_t* have = rg.cache.find(key)) {
+    *out = *have;
+    return FDTD_OK;
   }
   cudaGraph_t g;
   CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -1220,7 +1215,7 @@ int graph_for(RunGraphs& rg, cudaStream_t st, int steps, int tag, Enq enq, cudaG
   ce = cudaGraphInstantiate(&ge, g, 0);
   cudaGraphDestroy(g);
   if (ce != cudaSuccess) return fail(FDTD_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(ce));
-  rg.g.push_back({key, ge});
+  rg.cache.add(key, ge, [](cudaGraphExec_t old) { cudaGraphExecDestroy(old); });
   *out = ge;
   return FDTD_OK;
 }
