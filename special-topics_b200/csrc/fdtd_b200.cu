@@ -96,14 +96,10 @@ struct HostIProbe {
 
 }  // namespace
 
-// CUDA graphs of whole runs, keyed by their step count.  A run of `count`
-// steps replays graphs of at most the handle's cap (kMaxGraphNodes over the
-// launches one step takes) and one of the remainder; every graph a run needs
-// is captured before the run's first launch, so no capture falls inside a
-// timed region.  A handful of counts is kept (early-stop runs advance in
-// checkpoints of a few different lengths).
+// CUDA graphs of whole runs (run_plan.h).  Every graph a run needs is captured
+// before the run's first launch, so no capture falls inside a timed region.
 struct RunGraphs {
-  GraphCache<cudaGraphExec_t> cache;  // key: steps, and a tag of the state it starts from
+  GraphCache<cudaGraphExec_t> cache;
   void clear() {
     for (auto& e : cache.g) cudaGraphExecDestroy(e.exec);
     cache.g.clear();
@@ -1167,9 +1163,11 @@ int fused_enqueue_steps(fdtd_ctx* c, int count, int flip, int ts, KernelTimer* t
   return FDTD_OK;
 }
 
-int fused_enqueue(fdtd_ctx* c, int count, KernelTimer* tm = nullptr, cudaStream_t st = nullptr, double share = 1) {
+// `count` steps, `at` steps on from the handle's present state.
+int fused_enqueue(fdtd_ctx* c, int at, int count, KernelTimer* tm = nullptr, cudaStream_t st = nullptr,
+                  double share = 1) {
   if (!st) st = c->stream;
-  const int flip = c->fs.cur, ts = c->ts;
+  const int flip = c->fs.cur ^ (at & 1), ts = c->ts + at;
   if (c->prec == FDTD_PREC_F64) return fused_enqueue_steps<double, true>(c, count, flip, ts, tm, st, share);
   if (c->prec == FDTD_PREC_F32) return fused_enqueue_steps<float, true>(c, count, flip, ts, tm, st, share);
   return fused_enqueue_steps<float, false>(c, count, flip, ts, tm, st, share);
@@ -1193,21 +1191,19 @@ int close_dft_block(fdtd_ctx* c, int upto, cudaStream_t st) {
   return FDTD_OK;
 }
 
-constexpr int kGraphSteps = 64;       // shortest graph (and the cap's floor)
-constexpr int kMaxGraphNodes = 40000;  // kernel launches held by one graph at most
-
-// The graph of `steps` steps from the cache, captured on `st` through `enq`
-// (which enqueues that many steps) when missing.
+// The graph of a piece of a run that starts as `s` says, from the cache, captured
+// on `st` through `enq` (which enqueues those steps) when missing.
 template <class Enq>
-int graph_for(RunGraphs& rg, cudaStream_t st, int steps, int tag, Enq enq, cudaGraphExec_t* out) {
-  const long long key = (long long)steps << 16 | tag;
+int graph_for(RunGraphs& rg, cudaStream_t st, const RunPiece& piece, const RunStart& s, int launches_per_step, Enq enq,
+              cudaGraphExec_t* out) {
+  const long long key = s.after(piece.at).key(piece.steps);
   if (cudaGraphExec_t* have = rg.cache.find(key)) {
     *out = *have;
     return FDTD_OK;
   }
   cudaGraph_t g;
   CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-  int erc = enq(steps);
+  int erc = enq(piece.at, piece.steps);
   cudaError_t ce = cudaStreamEndCapture(st, &g);
   if (erc) return erc;
   if (ce != cudaSuccess) return fail(FDTD_ERR_CUDA, "graph capture: %s", cudaGetErrorString(ce));
@@ -1215,34 +1211,34 @@ int graph_for(RunGraphs& rg, cudaStream_t st, int steps, int tag, Enq enq, cudaG
   ce = cudaGraphInstantiate(&ge, g, 0);
   cudaGraphDestroy(g);
   if (ce != cudaSuccess) return fail(FDTD_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(ce));
-  rg.cache.add(key, ge, [](cudaGraphExec_t old) { cudaGraphExecDestroy(old); });
+  rg.cache.add(key, (long long)piece.steps * launches_per_step, ge, [](cudaGraphExec_t old) { cudaGraphExecDestroy(old); });
   *out = ge;
   return FDTD_OK;
 }
 
-// The graph launches of a run of `count` steps: full graphs of `cap` steps
-// and one of the remainder, each captured (if missing) now.  `period` and
-// `tag`: what a graph's steps depend on beyond their number repeats every
-// `period` steps, and `tag` is where in it the run starts.
+// The graph launches of a run of `count` steps that starts as `s` says, in pieces
+// of at most `cap` steps (0: as many as a graph may hold), each captured (if
+// missing) now: enq(at, steps) enqueues `steps` steps, `at` steps into the run.
 template <class Enq>
-int run_plan(RunGraphs& rg, cudaStream_t st, int count, int launches_per_step, Enq enq,
-             std::vector<cudaGraphExec_t>* plan, int period = 1, int tag = 0, int cap = 0) {
-  if (!cap) cap = std::max(kGraphSteps, kMaxGraphNodes / std::max(1, launches_per_step));
-  cap = std::max(cap / period, 1) * period;
+int run_plan(RunGraphs& rg, cudaStream_t st, int count, int launches_per_step, const RunStart& s, Enq enq,
+             std::vector<cudaGraphExec_t>* plan, int cap = 0) {
   plan->clear();
-  if (count <= 0) return FDTD_OK;
-  cudaGraphExec_t full = nullptr, rest = nullptr;
-  if (count >= cap) {
-    int rc = graph_for(rg, st, cap, tag, enq, &full);
-    if (rc) return rc;
+  for (const RunPiece& piece : run_pieces(count, s, launches_per_step, cap)) {
+    cudaGraphExec_t ge = nullptr;
+    if (int rc = graph_for(rg, st, piece, s, launches_per_step, enq, &ge)) return rc;
+    plan->push_back(ge);
   }
-  if (count % cap) {
-    int rc = graph_for(rg, st, count % cap, tag, enq, &rest);
-    if (rc) return rc;
-  }
-  for (int q = 0; q < count / cap; q++) plan->push_back(full);
-  if (rest) plan->push_back(rest);
   return FDTD_OK;
+}
+
+// Where the one-pass step's next run starts.
+RunStart fused_start(const fdtd_ctx* c) {
+  RunStart s;
+  s.one_pass = true;
+  s.copy = c->fs.cur;
+  s.block = c->dft_block;
+  s.phase = s.block > 0 ? c->ts % s.block : 0;
+  return s;
 }
 
 constexpr int kMaxBatchStreams = 32;
@@ -1290,15 +1286,12 @@ int run_steps(fdtd_ctx* c, int count, float* elapsed_ms = nullptr, KernelTimer* 
   }
   std::vector<cudaGraphExec_t> plan;
   if (!tm && fused) {
-    // a graph depends on the copy it starts from and on where DFT blocks close;
-    // tag 0 is the half-step path
-    const int per = c->dft_block > 0 ? c->dft_block : 1;
-    rc = run_plan(c->graphs, c->stream, count, 3, [c](int n) { return fused_enqueue(c, n); }, &plan, 2 * per,
-                  2 * (c->ts % per) + c->fs.cur + 1);
+    rc = run_plan(c->graphs, c->stream, count, 3, fused_start(c), [c](int at, int n) { return fused_enqueue(c, at, n); },
+                  &plan);
     if (rc) return rc;
   } else if (!tm) {
-    rc = run_plan(c->graphs, c->stream, count, c->dft_block > 0 ? 5 : 4,
-                  [c](int n) { return enqueue(c, n); }, &plan);
+    rc = run_plan(c->graphs, c->stream, count, c->dft_block > 0 ? 5 : 4, RunStart(),
+                  [c](int, int n) { return enqueue(c, n); }, &plan);
     if (rc) return rc;
   }
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -1313,7 +1306,7 @@ int run_steps(fdtd_ctx* c, int count, float* elapsed_ms = nullptr, KernelTimer* 
     c->fs.valid = true;
   }
   if (tm) {
-    rc = fused ? fused_enqueue(c, count, tm) : enqueue(c, count, tm);
+    rc = fused ? fused_enqueue(c, 0, count, tm) : enqueue(c, count, tm);
     if (rc) return rc;
   }
   for (cudaGraphExec_t ge : plan) CK(cudaGraphLaunch(ge, c->stream));
@@ -3005,13 +2998,13 @@ int batch_member_enqueue(fdtd_batch* b, int count) {
 constexpr int kChainNodes = 4096;
 int batch_chain_streams(const fdtd_batch* b) { return std::min((int)b->m.size(), kMaxBatchStreams); }
 
-int batch_chain_enqueue(fdtd_batch* b, int count) {
+int batch_chain_enqueue(fdtd_batch* b, int at, int count) {
   const int S = batch_chain_streams(b);
   CK(cudaEventRecord(b->fork_ev, b->stream));
   for (int q = 0; q < S; q++) CK(cudaStreamWaitEvent(b->ws[q], b->fork_ev, 0));
   int rc = FDTD_OK;
   for (size_t q = 0; q < b->m.size() && !rc; q++)
-    rc = fused_enqueue(b->m[q], count, nullptr, b->ws[q % S], S > 1 ? 1.0 / S : 1);
+    rc = fused_enqueue(b->m[q], at, count, nullptr, b->ws[q % S], S > 1 ? 1.0 / S : 1);
   for (int q = 0; q < S; q++) {
     CK(cudaEventRecord(b->wev[q], b->ws[q]));
     CK(cudaStreamWaitEvent(b->stream, b->wev[q], 0));
@@ -3066,13 +3059,13 @@ int batch_run_members(fdtd_batch* b, int count, bool chain, float* elapsed_ms, K
   if (!tm) {
     int per_step = 0;
     for (fdtd_ctx* c : b->m) per_step += c->dft_block > 0 ? 5 : 4;
-    if (chain) {
-      const int per = b->m[0]->dft_block > 0 ? b->m[0]->dft_block : 1;
-      rc = run_plan(b->graphs, b->stream, count, per_step, [b](int n) { return batch_chain_enqueue(b, n); }, &plan,
-                    2 * per, 2 * (ts % per) + b->m[0]->fs.cur, std::max(1, kChainNodes / per_step));
-    } else {
-      rc = run_plan(b->graphs, b->stream, count, per_step, [b](int n) { return batch_member_enqueue(b, n); }, &plan);
-    }
+    if (chain)
+      rc = run_plan(b->graphs, b->stream, count, per_step, fused_start(b->m[0]),
+                    [b](int at, int n) { return batch_chain_enqueue(b, at, n); }, &plan,
+                    std::max(1, kChainNodes / per_step));
+    else
+      rc = run_plan(b->graphs, b->stream, count, per_step, RunStart(),
+                    [b](int, int n) { return batch_member_enqueue(b, n); }, &plan);
     if (rc) return rc;
   }
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -3085,7 +3078,7 @@ int batch_run_members(fdtd_batch* b, int count, bool chain, float* elapsed_ms, K
     // one member at a time on the batch's stream: per-kernel times summed over members
     for (size_t q = 0; q < b->m.size() && !rc; q++) {
       MemberShape shape(b->m[q], b);
-      rc = chain ? fused_enqueue(b->m[q], count, tm, b->stream) : enqueue(b->m[q], count, tm, b->stream);
+      rc = chain ? fused_enqueue(b->m[q], 0, count, tm, b->stream) : enqueue(b->m[q], count, tm, b->stream);
     }
     if (rc) return rc;
   }
@@ -3156,7 +3149,8 @@ int batch_run(fdtd_batch* b, int count, float* elapsed_ms = nullptr, KernelTimer
   std::vector<cudaGraphExec_t> plan;
   if (!tm) {
     const int per_step = (b->flush.empty() ? 2 : 3) + (b->ngroups > 0 ? 2 * b->ngroups : 2);
-    rc = run_plan(b->graphs, b->stream, count, per_step, [b](int n) { return batch_enqueue_any(b, n); }, &plan);
+    rc = run_plan(b->graphs, b->stream, count, per_step, RunStart(),
+                  [b](int, int n) { return batch_enqueue_any(b, n); }, &plan);
     if (rc) return rc;
   }
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
