@@ -830,17 +830,21 @@ int fused_classes(fdtd_ctx* c, const C& coef, bool* ok) {
   return rc == FDTD_ERR_OOM ? FDTD_OK : rc;
 }
 
-// Profiles b, a over a whole axis, zero outside the bands.
+// Profiles b, a over a whole axis, zero outside the bands; along z in FP32, where
+// a slab holds other columns too, b is -0 there (in_band).
 int fused_axis_values(const fdtd_ctx* c, int a) { return (a == 0 ? c->nx + 1 : a == 1 ? c->ny + 1 : fused_pitch(c)) + 8; }
 
 int fused_profiles(fdtd_ctx* c) {
-  for (int el = 0; el < 2; el++)
+  for (int el = 0; el < 2; el++) {
+    if (c->esz == 4)  // the sign bytes
+      CK(cudaMemset2DAsync((char*)c->fs.prof[el][2][0] + 3, 4, 0x80, 1, fused_axis_values(c, 2), c->stream));
     for (int f = 0; f < 6; f++) {
       const HostFace& h = c->face[f];
       for (int w = 0; w < 2 && h.present; w++)
         CK(cudaMemcpyAsync((char*)c->fs.prof[el][f / 2][w] + (el ? h.e_start : h.m_start) * c->esz,
                            h.prof[(el ? 0 : 2) + w], h.nc * c->esz, cudaMemcpyDeviceToDevice, c->stream));
     }
+  }
   return FDTD_OK;
 }
 

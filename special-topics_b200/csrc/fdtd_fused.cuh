@@ -19,10 +19,11 @@
 //     coefficients, its values along the band positions of its axis.  Classes
 //     and table are filled on the device from the problem's own coefficients
 //     and every cell is compared with its lookup bit for bit, so the table form
-//     loses nothing; values a step leaves alone, or that do not exist at a
-//     cell, are classes too (coefficients 1,0,0 and 0,0,0), so the update has
-//     no tests for walls and edges.  A thread keeps its coefficients in
-//     registers along x and reads the table only where the class changes.
+//     loses nothing.  Values a step leaves alone, or that do not exist at a
+//     cell, are classes too (coefficients 1,0,0 and 0,0,0); held values are kept
+//     by a select besides, as 0 times an infinity is not 0.  A thread keeps its
+//     coefficients in registers along x and reads the table only where the class
+//     changes.
 // The arithmetic of a value is that of fdtd_step.cuh, in the same order.
 //
 // A block owns six rows of up to 72 columns (with a halo row and, where a row
@@ -162,7 +163,7 @@ struct FusedAxis {
   const T* phi[2];         // H Psi (slots 0, 1 of the faces) of the copy read
   T* pho[2];               // and of the copy written
   T* pe[2];                // E Psi (slots 2, 3)
-  const T* prof[2][2];     // [H, E][b, a] over the whole axis
+  const T* prof[2][2];     // [H, E][b, a] over the whole axis; outside the bands a is 0 and b -0
 };
 
 // Layout of a class's table row, in values: the six components' (c0, c1, c2, -)
@@ -208,6 +209,12 @@ __device__ __forceinline__ int band_cell(const FusedAxis<T>& x, int pos) {
                                                       : -1;
 }
 
+// Whether a column of a z slab lies in the band.  Outside the bands b is -0 (no
+// band's b = exp(-x) is): such a column keeps a zero Psi and takes none of it, as
+// 0 times an infinite drive is not 0.  The slabs of one-column groups are the bands.
+__device__ __forceinline__ bool in_band(float b) { return __float_as_uint(b) != 0x80000000u; }
+__device__ __forceinline__ constexpr bool in_band(double) { return true; }
+
 // Programmatic launches: waits for the launch before this one (at once where
 // this is an ordinary launch), and lets the one after it start its blocks.
 __device__ __forceinline__ void launch_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -224,10 +231,11 @@ __device__ __forceinline__ void tma_tile(void* dst, const CUtensorMap* map, int 
       : "memory");
 }
 
-// One axis's CPML on a value: Psi = b Psi + a drive, v += CPsi Psi.
+// One axis's CPML on a value: Psi = b Psi + a drive, v += CPsi Psi; `in`: see in_band.
 template <bool EXACT, typename T>
-__device__ __forceinline__ void fused_cpml(T& psi, T b, T a, T cp, T d, T& v) {
-  psi = Ar<T, EXACT>::lin2(b, psi, a, d);
+__device__ __forceinline__ void fused_cpml(T& psi, T b, T a, T cp, T d, T& v, bool in = true) {
+  const T n = Ar<T, EXACT>::lin2(b, psi, a, d);
+  psi = in ? n : T(0);
   v = Ar<T, EXACT>::axpy(v, cp, psi);
 }
 
@@ -282,12 +290,13 @@ __device__ __forceinline__ void fused_coef(const ClassRow& L, const T* row, int 
 
 // Values the update leaves alone along z: Hx and Hy do not exist at k = nz, Ex
 // and Ey are held at k = 0 and k = nz.  They keep their old value here, so that
-// the groups at the walls need no class of their own.
+// the groups at the walls need no class of their own.  `all`: the whole group is
+// held by another wall.
 template <bool ELECTRIC, typename T>
-__device__ __forceinline__ void fused_hold(int k, int nz, const Vec<T>& old, Vec<T>& v) {
+__device__ __forceinline__ void fused_hold(int k, int nz, bool all, const Vec<T>& old, Vec<T>& v) {
 #pragma unroll
   for (int q = 0; q < FusedShape<T>::V; q++)
-    if (k + q == nz || (ELECTRIC && q == 0 && k == 0)) v.v[q] = old.v[q];
+    if (all || k + q == nz || (ELECTRIC && q == 0 && k == 0)) v.v[q] = old.v[q];
 }
 
 // The coefficients of the cells of a group for one half-step.  Cells that share
@@ -380,8 +389,8 @@ __device__ __forceinline__ void fused_h(const FusedParams<T>& p, const FusedCell
     hy.v[q] = A::lin3(y.c0, oy.v[q], t.xc >= 0 ? cx0 : y.c1, dez_x.v[q], c.z1(q), dex_z.v[q]);
     hz.v[q] = A::lin3(z.c0, oz.v[q], z.c1, dex_y.v[q], t.xc >= 0 ? cx1 : z.c2, dey_x.v[q]);
   }
-  fused_hold<false>(t.k, p.nz, ox, hx);
-  fused_hold<false>(t.k, p.nz, oy, hy);
+  fused_hold<false>(t.k, p.nz, false, ox, hx);
+  fused_hold<false>(t.k, p.nz, false, oy, hy);
   if (t.xc >= 0) {
     const FusedAxis<T>& X = p.axis[0];
     const T b = __ldg(X.prof[0][0] + t.i), a = __ldg(X.prof[0][1] + t.i);
@@ -413,8 +422,8 @@ __device__ __forceinline__ void fused_h(const FusedParams<T>& p, const FusedCell
     const Vec<T> b = ldw<T>(t.pcol), a = ldw<T>(t.pcol + W);
 #pragma unroll
     for (int q = 0; q < V; q++) {
-      fused_cpml<EXACT>(f.z0.v[q], b.v[q], a.v[q], c.cpsi(q, 0), dey_z.v[q], hx.v[q]);
-      fused_cpml<EXACT>(f.z1.v[q], b.v[q], a.v[q], c.cpsi(q, 3), dex_z.v[q], hy.v[q]);
+      fused_cpml<EXACT>(f.z0.v[q], b.v[q], a.v[q], c.cpsi(q, 0), dey_z.v[q], hx.v[q], in_band(b.v[q]));
+      fused_cpml<EXACT>(f.z1.v[q], b.v[q], a.v[q], c.cpsi(q, 3), dex_z.v[q], hy.v[q], in_band(b.v[q]));
     }
     if (t.store) {
       stv(Z.pho[0] + t.oz, f.z0);
@@ -436,13 +445,14 @@ __device__ __forceinline__ void fused_e(const FusedParams<T>& p, const FusedCell
   const Vec<T> dhz_y = vsub(hz, ldw<T>(N + 2 * HS - W)), dhy_z = vdiff_dn(hy, N[HS - 1]);
   const Vec<T> dhx_z = vdiff_dn(hx, N[-1]), dhx_y = vsub(hx, ldw<T>(N - W));
   const Vec<T> dhz_x = vsub(hz, hzp), dhy_x = vsub(hy, hyp);
-  const Vec<T> oex = ex, oey = ey;
+  const Vec<T> oex = ex, oey = ey, oez = ez;
 #pragma unroll
   for (int q = 0; q < V; q++) {
     const Row<T> x = c.x(q);
     ex.v[q] = A::lin3(x.c0, ex.v[q], x.c1, dhz_y.v[q], c.z0(q), dhy_z.v[q]);
   }
-  fused_hold<true>(t.k, p.nz, oex, ex);
+  const bool wall_j = t.j == 0 || t.j == p.ny;
+  fused_hold<true>(t.k, p.nz, wall_j, oex, ex);
   if (yz) {
     T cx0 = T(0), cx1 = T(0);
 #pragma unroll
@@ -455,7 +465,8 @@ __device__ __forceinline__ void fused_e(const FusedParams<T>& p, const FusedCell
       ey.v[q] = A::lin3(y.c0, ey.v[q], c.z1(q), dhx_z.v[q], t.xc >= 0 ? cx0 : y.c2, dhz_x.v[q]);
       ez.v[q] = A::lin3(z.c0, ez.v[q], t.xc >= 0 ? cx1 : z.c1, dhy_x.v[q], z.c2, dhx_y.v[q]);
     }
-    fused_hold<true>(t.k, p.nz, oey, ey);
+    fused_hold<true>(t.k, p.nz, t.i == 0, oey, ey);
+    if (wall_j || t.i == 0) ez = oez;
     if (t.xc >= 0) {
       const FusedAxis<T>& X = p.axis[0];
       const T b = __ldg(X.prof[1][0] + t.i), a = __ldg(X.prof[1][1] + t.i);
@@ -484,11 +495,11 @@ __device__ __forceinline__ void fused_e(const FusedParams<T>& p, const FusedCell
     const FusedAxis<T>& Z = p.axis[2];
     const Vec<T> b = ldw<T>(t.pcol + 2 * W), a = ldw<T>(t.pcol + 3 * W);
 #pragma unroll
-    for (int q = 0; q < V; q++) fused_cpml<EXACT>(f.z0.v[q], b.v[q], a.v[q], c.cpsi(q, 7), dhy_z.v[q], ex.v[q]);
+    for (int q = 0; q < V; q++) fused_cpml<EXACT>(f.z0.v[q], b.v[q], a.v[q], c.cpsi(q, 7), dhy_z.v[q], ex.v[q], in_band(b.v[q]));
     stv(Z.pe[0] + t.oz, f.z0);
     if (yz) {
 #pragma unroll
-      for (int q = 0; q < V; q++) fused_cpml<EXACT>(f.z1.v[q], b.v[q], a.v[q], c.cpsi(q, 8), dhx_z.v[q], ey.v[q]);
+      for (int q = 0; q < V; q++) fused_cpml<EXACT>(f.z1.v[q], b.v[q], a.v[q], c.cpsi(q, 8), dhx_z.v[q], ey.v[q], in_band(b.v[q]));
       stv(Z.pe[1] + t.oz, f.z1);
     }
   }
@@ -554,8 +565,7 @@ __device__ __forceinline__ void fused_tile(const FusedParams<T>& p, int bx, int 
     fence_proxy_async();
     for (int m = 0; m <= min(NS - 1, last); m++) issue(m);
   }
-  // H where the grid has none is read into differences that nothing uses, but
-  // must be finite
+  // H where the grid has none is read into differences that nothing uses
   for (int w = tid; w < 2 * 3 * HS; w += NT) sx[w] = T(0);
 
   const unsigned plane = p.plane, jk = in ? (unsigned)(j * p.pitch + k) : 0u;
@@ -738,7 +748,7 @@ __device__ __forceinline__ void fused_wall_thread(const FusedParams<T>& p, int t
   constexpr int V = FusedShape<T>::V;
   const FusedAxis<T>&Y = p.axis[1], &Z = p.axis[2];
   const int kq = k % V;  // place in its group
-  const int yc = band_cell<true>(Y, j), zg = band_cell<true>(Z, k - kq), zc = zg >= 0 ? zg + kq : -1;
+  const int yc = band_cell<true>(Y, j), zg = band_cell<true>(Z, k - kq), zc = zg >= 0 && in_band(Z.prof[1][0][k]) ? zg + kq : -1;
   FusedCoef<T> n;
   fused_coef<true>(p.row, row, yc, zg, n);
   const T hx = (j < ny && k < nz) ? fo[0][off] : T(0);
