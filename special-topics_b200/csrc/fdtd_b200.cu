@@ -2550,7 +2550,7 @@ int fdtd_ctx_farfield_post(fdtd_ctx* c, const double* theta, const double* phi, 
           const unsigned nf = (unsigned)std::min(fb, F - f0);
           const FFSums W{f0,  nth,   dth + u.t0, dith + u.a0, dang + u.a0, dang + na + u.a0,
                          ang, drows, dz,         parts};
-          k_ff_rows<<<dim3((nth + per - 1) / per, (unsigned)R, nf), kFFRowThreads, 0, c->stream>>>(P, W, dfreq);
+          k_ff_rows<<<dim3((unsigned)R, (nth + per - 1) / per, nf), kFFRowThreads, 0, c->stream>>>(P, W, dfreq);
           k_ff_zrows<<<dim3((ang + zper - 1) / zper, parts, nf), kFFZThreads, 0, c->stream>>>(P, W, dfreq);
           k_ff_pattern<<<dim3((ang + 127) / 128, nf), 128, 0, c->stream>>>(P, W, dfreq, dradp, (long long)na, dout + u.a0,
                                                                           dout + F * na + u.a0);

@@ -181,12 +181,14 @@ struct FFSums {
   int parts;          // each of a part of their rows
 };
 
+// A block per (row, run of thetas, frequency); the rows along the grid's first axis,
+// as a long thin problem has more of them than the others hold (65,535).
 constexpr int kFFRowThreads = 64, kFFRowAng = 2;
 __global__ void __launch_bounds__(kFFRowThreads)
     k_ff_rows(FFPost P, FFSums W, const double* __restrict__ freqs) {
   __shared__ __align__(16) double sm[1][kFFPairs][16];
   const int f = W.f0 + blockIdx.z;
-  int r = blockIdx.y, fc = 0;
+  int r = blockIdx.x, fc = 0;
   for (; fc < 3 && r >= (fc < 2 ? P.nj : P.ni); fc++) r -= fc < 2 ? P.nj : P.ni;
   const int a = fc / 2, nn = P.nk;
   const double k = 2.0 * kPi * freqs[f] / kC0;
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(kFFRowThreads)
   for (int w = 0; w < 4; w++) arr[0][w] = P.acc + P.off[c[w]] + (long long)f * P.sz[a] + (long long)r * nn;
   double kx[kFFRowAng];
   Cplx S[kFFRowAng][1][4] = {};
-  const int th0 = blockIdx.x * kFFRowThreads * kFFRowAng + threadIdx.x;
+  const int th0 = blockIdx.y * kFFRowThreads * kFFRowAng + threadIdx.x;
   for (int q = 0; q < kFFRowAng; q++) {
     const int th = th0 + q * kFFRowThreads;
     kx[q] = th < W.nth ? k * W.cth[th] : 0.0;
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(kFFRowThreads)
     const int th = th0 + q * kFFRowThreads;
     if (th >= W.nth) continue;
     const Cplx mid = cexpj(kx[q] * (P.pos0[2] + 0.5 * (nn - 1) * P.d[2]));
-    double* out = W.rows + ((long long)blockIdx.z * R + blockIdx.y) * 8 * W.nth + th;
+    double* out = W.rows + ((long long)blockIdx.z * R + blockIdx.x) * 8 * W.nth + th;
     for (int w = 0; w < 4; w++) {
       const Cplx v = cmul(mid, S[q][0][w]);
       out[2 * w * (long long)W.nth] = v.re;
