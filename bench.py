@@ -402,7 +402,8 @@ def main():
                      "algorithmic_bytes_per_launch": dom_bytes, "launch_ms": dom_ms,
                      "traffic": traffic},
         "kernel_ms": kern,
-        "tiling": {k: tuning.get(k, 32 if k == "width" else None) for k in ("chunk", "rows", "prefetch", "width", "ms_per_step")}
+        "tiling": "the one-pass step's own" if one_pass(kern) else
+                  {k: tuning.get(k, 32 if k == "width" else None) for k in ("chunk", "rows", "prefetch", "width", "ms_per_step")}
                   if tuning else "default",
         "clocks": clk.summary(),
         # H, mid, E, epilogue (+ the DFT flush); one-pass: the step, its epilogue, the wall where the reference's
@@ -505,9 +506,11 @@ def _sum_over_ranks(x: float, dist, local: int) -> float:
 
 
 def _best_by_mode(table: list) -> dict:
-    """Fastest tuned step time (ms) of the tile-list and member-kernel modes."""
+    """Fastest tuned step time (ms) of each mode that was timed."""
     out = {}
-    for name, pick in (("tile_list", lambda r: r.get("streams", 0) == 0 and r.get("per_launch", 0) == 0),
+    for name, pick in (("chains", lambda r: r.get("chains", False)),
+                       ("tile_list", lambda r: not r.get("chains", False) and r.get("streams", 0) == 0 and
+                        r.get("per_launch", 0) == 0),
                        ("grouped", lambda r: r.get("streams", 0) == 0 and r.get("per_launch", 0) > 0),
                        ("member_kernels", lambda r: r.get("streams", 0) > 0)):
         rows = [r for r in table if pick(r)]
@@ -585,7 +588,9 @@ def batched_side(problems, K: int = 1000, W: int = 8, tune_steps: int = 16, devi
             "grid_max": list(max(dims, key=lambda d: d[0] * d[1] * d[2])),
             "value": cells * K / (ms / 1e3) / 1e9, "unit": "Gcell-updates/s", "steps": K, "warmup": W,
             "ms_per_step": ms / K,
-            "gpu_launches": K * ((5 if dft_block else 4) * len(problems) if tiling.get("streams", 0) else
+            # chains: each member's step and its epilogue, and a flush per block
+            "gpu_launches": (2 * K + (K // dft_block if dft_block else 0)) * len(problems) if one_pass(kern) else
+                            K * ((5 if dft_block else 4) * len(problems) if tiling.get("streams", 0) else
                                  (3 if dft_block else 2) + 2 * (-(-len(problems) // tiling["per_launch"])
                                                                 if tiling.get("per_launch", 0) else 1)),
             "kernel_ms": kern,
@@ -807,7 +812,8 @@ def fp64_side(pkg, n=(256, 256, 256), K: int = 300, W: int = 8) -> dict:
     dom, dom_bytes, dom_ms = dominant(kern, byts)
     ach = dom_bytes / (dom_ms / 1e3) / 1e9
     return {"workload": f"scaling-box-{n[0]}x{n[1]}x{n[2]}", "value": p.grid.cells * K / (ms / 1e3) / 1e9,
-            "unit": "Gcell-updates/s", "ms_per_step": ms / K, "tiling": {k: tuning[k] for k in ("chunk", "rows", "prefetch")},
+            "unit": "Gcell-updates/s", "ms_per_step": ms / K,
+            "tiling": "the one-pass step's own" if one_pass(kern) else {k: tuning[k] for k in ("chunk", "rows", "prefetch")},
             "roofline": {"kernel": dom, "achieved": ach, "peak": peak, "frac": ach / peak}}
 
 

@@ -223,9 +223,11 @@ typedef struct fdtd_batch fdtd_batch;
 /* Groups `count` handles of one device and one precision.  The batch owns no
  * member: members stay valid handles (readbacks, fdtd_status, their own runs)
  * and must outlive the batch.  By default, where every member can run the
- * one-pass step (csrc/fdtd_fused.cuh) and their DFT blocks are of one length,
- * each member's steps are a chain of its own, side by side on worker streams;
- * the launch shape then has no effect.  Otherwise each step of fdtd_batch_run is
+ * one-pass step (csrc/fdtd_fused.cuh; fdtd_ctx_set_step_path) and their DFT
+ * blocks are of one length, each member's steps are a chain of its own, side by
+ * side on worker streams; the x planes, block rows, width and prefetch depth then
+ * have no effect.  Otherwise, and where a tile group or members per launch are
+ * set, each step of fdtd_batch_run is
  * four launches for the whole batch: H over a tile list spanning every member,
  * the mid-step kernel, E over the tile list, and the far-field/port epilogue
  * (fdtd_batch_set_streams selects the member-kernel mode instead). */
@@ -328,6 +330,14 @@ int fdtd_ctx_set_dft_accumulator(fdtd_ctx* ctx, int kahan_fp32);
  * May be changed between runs. */
 int fdtd_ctx_set_x_wall(fdtd_ctx* ctx, int wall);
 int fdtd_ctx_get_x_wall(const fdtd_ctx* ctx, int* wall);
+
+/* Which kernels a handle's steps run: path = 0 (default), the one-pass step
+ * (csrc/fdtd_fused.cuh) where it serves the problem, else the half-step kernels;
+ * path = 1, the half-step kernels, whose launch shape the calls above set.
+ * Results are identical.  The one-pass step holds two more copies of the state,
+ * which path = 1 gives back.  May be changed between runs. */
+int fdtd_ctx_set_step_path(fdtd_ctx* ctx, int path);
+int fdtd_ctx_get_step_path(const fdtd_ctx* ctx, int* path);
 
 /* Far-field post-processing on the device from the handle's accumulators
  * (farfield.js:257-607): radp[f] = radiated power at frequency f, and the

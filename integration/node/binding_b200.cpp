@@ -30,6 +30,7 @@
 //   saveState(h) -> Buffer / loadState(h, Buffer)   fdtd_ctx_state_size / save_state / load_state
 //   setDftBlock(h, steps), setDftAccumulator(h, kahan)  fdtd_ctx_set_dft_block / set_dft_accumulator
 //   setXWall(h, wall)                               fdtd_ctx_set_x_wall (E at i = nx: 0 reference reads, 1 PEC wall)
+//   setStepPath(h, path)                            fdtd_ctx_set_step_path (0 one-pass step where it serves, 1 half-steps)
 //   batchCreate([h...]) -> b, batchRun(b, count), batchShape(b, chunk, rows, prefetch, group,
 //   streams, width[, perLaunch]), batchFree(b)      fdtd_batch_*
 //
@@ -258,6 +259,11 @@ Napi::Value SetXWall(const Napi::CallbackInfo& a) {
   return a.Env().Undefined();
 }
 
+Napi::Value SetStepPath(const Napi::CallbackInfo& a) {
+  Check(a.Env(), fdtd_ctx_set_step_path(Ctx(a[0]), Int(a[1])), "setStepPath");
+  return a.Env().Undefined();
+}
+
 Napi::Value BatchCreate(const Napi::CallbackInfo& a) {
   Napi::Array arr = a[0].As<Napi::Array>();
   std::vector<fdtd_ctx*> hs(arr.Length());
@@ -312,6 +318,7 @@ Napi::Object Init(Napi::Env env, Napi::Object e) {
   e.Set("setDftBlock", Napi::Function::New(env, SetDftBlock));
   e.Set("setDftAccumulator", Napi::Function::New(env, SetDftAccumulator));
   e.Set("setXWall", Napi::Function::New(env, SetXWall));
+  e.Set("setStepPath", Napi::Function::New(env, SetStepPath));
   e.Set("batchCreate", Napi::Function::New(env, BatchCreate));
   e.Set("batchRun", Napi::Function::New(env, BatchRun));
   e.Set("batchShape", Napi::Function::New(env, BatchShape));

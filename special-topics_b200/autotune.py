@@ -3,8 +3,9 @@
 Every launch shape computes the same values.  For a problem, the tuner times
 the candidate shapes (x planes per thread x thread rows per block) on a
 scratch copy of the problem, so the caller's engine state is untouched, and
-keeps the fastest.  Results are cached per (precision, nx, ny, nz) in a JSON
-file next to the built library.
+keeps the fastest.  The shapes are the half-step kernels': where the one-pass
+step serves the problem, which picks its own, none is tried.  Results are cached
+per (precision, nx, ny, nz) in a JSON file next to the built library.
 """
 from __future__ import annotations
 
@@ -15,6 +16,7 @@ import os
 from . import _native as N
 
 CACHE = os.path.join(N.BUILD_DIR, "tiling_cache.json")
+CACHE_VERSION = 2   # entries of version 1 were timed before the one-pass step
 CHUNKS = (1, 2, 4, 8, 16, 32, 64)
 ROWS = (2, 4, 8)
 PREFETCH = (1, 2)
@@ -33,9 +35,17 @@ def _key(problem, precision: str) -> str:
 def _load() -> dict:
     try:
         with open(CACHE) as f:
-            return json.load(f)
+            cache = json.load(f)
     except (OSError, ValueError):
         return {}
+    ours = isinstance(cache, dict) and cache.get("version") == CACHE_VERSION
+    return cache.get("entries", {}) if ours else {}
+
+
+def _store(cache: dict) -> None:
+    os.makedirs(os.path.dirname(CACHE), exist_ok=True)
+    with open(CACHE, "w") as f:
+        json.dump({"version": CACHE_VERSION, "entries": cache}, f, indent=1)
 
 
 def get_tiling(engine) -> tuple[int, int]:
@@ -56,7 +66,9 @@ NARROW_ROWS = (2, 4, 8, 16)
 
 
 def tune(problem, precision: str, device: int = 0, steps_per_candidate: int = 64, use_cache: bool = True) -> dict:
-    """Returns {"chunk", "rows", "ms_per_step", "table"} for the problem's grid."""
+    """Returns {"chunk", "rows", "ms_per_step", "table", "one_pass"} for the
+    problem's grid; where the one-pass step serves it, its time and the shape that
+    the half-steps would have."""
     from .backend import Engine
     key = _key(problem, precision)
     cache = _load()
@@ -70,8 +82,14 @@ def tune(problem, precision: str, device: int = 0, steps_per_candidate: int = 64
     table = []
     with Engine(problem, precision, device=device) as eng:
         eng.run(4)
+        one_pass = eng.profile_kernels(1)["e"] == 0
+        if one_pass:
+            eng.run_timed(steps_per_candidate)
+            ms = eng.run_timed(steps_per_candidate) / steps_per_candidate
+            chunk, rows = get_tiling(eng)
+            table.append({"chunk": chunk, "rows": rows, "prefetch": 1, "width": 32, "ms_per_step": ms})
         for chunk in CHUNKS:
-            if chunk > nx + 1:
+            if one_pass or chunk > nx + 1:
                 continue
             for rows in ROWS:
                 for pf in depths:
@@ -80,7 +98,7 @@ def tune(problem, precision: str, device: int = 0, steps_per_candidate: int = 64
                     ms = eng.run_timed(steps_per_candidate) / steps_per_candidate
                     table.append({"chunk": chunk, "rows": rows, "prefetch": pf, "width": 32, "ms_per_step": ms})
         best = min(table, key=lambda r: r["ms_per_step"])
-        for rows in NARROW_ROWS:
+        for rows in () if one_pass else NARROW_ROWS:
             set_tiling(eng, best["chunk"], rows, best["prefetch"], 16)
             eng.run_timed(steps_per_candidate)
             ms = eng.run_timed(steps_per_candidate) / steps_per_candidate
@@ -88,11 +106,9 @@ def tune(problem, precision: str, device: int = 0, steps_per_candidate: int = 64
                           "ms_per_step": ms})
     best = min(table, key=lambda r: r["ms_per_step"])
     out = {"chunk": best["chunk"], "rows": best["rows"], "prefetch": best["prefetch"], "width": best["width"],
-           "ms_per_step": best["ms_per_step"], "table": table}
+           "ms_per_step": best["ms_per_step"], "table": table, "one_pass": one_pass}
     cache[key] = out
-    os.makedirs(os.path.dirname(CACHE), exist_ok=True)
-    with open(CACHE, "w") as f:
-        json.dump(cache, f, indent=1)
+    _store(cache)
     return out
 
 
@@ -126,14 +142,15 @@ def batch_steps_needed(steps_per_candidate: int, precision: str = "f32-table") -
 
 def tune_batch(batch, steps_per_candidate: int = 16, use_cache: bool = True) -> dict:
     """Tunes a batch's launch shape on the batch itself (every shape computes
-    the same values, so tuning only advances the members by
-    batch_steps_needed(steps_per_candidate) steps).  Tile-list mode: x planes
-    per thread, block rows and prefetch depth with one block per tile, then
-    the tile group of the persistent grid.  Grouped mode: the members per
-    launch at the best tile-list shape, then block shapes and prefetch depths
-    at the best count.  Member-kernel mode: the worker
-    stream count at the first member shape, then the member shapes at the best
-    count (whole graphs of MEMBER_STEPS steps, since a member-mode step is
+    the same values, so tuning only advances the members, by at most
+    batch_steps_needed(steps_per_candidate) steps).  The members' one-pass chains,
+    where they serve the batch, have no shape and are timed once (the row with
+    "chains" set).  Tile-list mode otherwise: x planes per thread, block rows and
+    prefetch depth with one block per tile.  Then the tile group of the persistent
+    grid.  Grouped mode: the members per launch at the best shape so far, then
+    block shapes and prefetch depths at the best count.  Member-kernel mode: the
+    worker stream count at the first member shape, then the member shapes at the
+    best count (whole graphs of MEMBER_STEPS steps, since a member-mode step is
     many launches).  Sets and returns the fastest."""
     key = batch_key(batch)
     cache = _load()
@@ -144,21 +161,27 @@ def tune_batch(batch, steps_per_candidate: int = 16, use_cache: bool = True) -> 
         return r
     max_x = max(e.problem.grid.nx for e in batch.engines) + 1
     table = []
+    batch.set_tiling(min(MEMBER_SHAPES[0][0], max_x), *MEMBER_SHAPES[0][1:], 0, 0, 32, 0)
+    chains = batch.profile_kernels(1)["e"] == 0
 
     def trial(chunk, rows, pf, group, streams=0, steps=steps_per_candidate, width=32, per_launch=0):
         batch.set_tiling(chunk, rows, pf, group, streams, width, per_launch)
         batch.run_timed(steps)              # capture and warm the graph
         ms = batch.run_timed(steps) / steps
         table.append({"chunk": chunk, "rows": rows, "prefetch": pf, "group": group, "streams": streams,
-                      "width": width, "per_launch": per_launch, "ms_per_step": ms})
+                      "width": width, "per_launch": per_launch, "ms_per_step": ms,
+                      "chains": chains and not (group or streams or per_launch)})
 
-    for chunk in BATCH_CHUNKS:
-        for rows in ROWS:
-            for pf in prefetch_depths(batch.engines[0].precision):
-                trial(min(chunk, max_x), rows, pf, 0)
-    best = min(table, key=lambda r: r["ms_per_step"])
-    for rows in NARROW_ROWS:
-        trial(best["chunk"], rows, best["prefetch"], 0, width=16)
+    if chains:
+        trial(min(MEMBER_SHAPES[0][0], max_x), *MEMBER_SHAPES[0][1:], 0)
+    else:
+        for chunk in BATCH_CHUNKS:
+            for rows in ROWS:
+                for pf in prefetch_depths(batch.engines[0].precision):
+                    trial(min(chunk, max_x), rows, pf, 0)
+        best = min(table, key=lambda r: r["ms_per_step"])
+        for rows in NARROW_ROWS:
+            trial(best["chunk"], rows, best["prefetch"], 0, width=16)
     best = min(table, key=lambda r: r["ms_per_step"])
     for group in BATCH_GROUPS[1:]:
         trial(best["chunk"], best["rows"], best["prefetch"], group, width=best["width"])
@@ -180,9 +203,7 @@ def tune_batch(batch, steps_per_candidate: int = 16, use_cache: bool = True) -> 
     batch.set_tiling(best["chunk"], best["rows"], best["prefetch"], best["group"], best["streams"], best["width"],
                      best["per_launch"])
     cache[key] = out
-    os.makedirs(os.path.dirname(CACHE), exist_ok=True)
-    with open(CACHE, "w") as f:
-        json.dump(cache, f, indent=1)
+    _store(cache)
     return out
 
 

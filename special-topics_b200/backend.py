@@ -30,7 +30,8 @@ class Engine:
     """One problem resident on one GPU."""
 
     def __init__(self, problem: Problem, precision: str = "f64", device: int = 0, host_tables: bool = False,
-                 dft_accumulator: str = "f64", dft_block: int = 0, x_wall: bool | None = None):
+                 dft_accumulator: str = "f64", dft_block: int = 0, x_wall: bool | None = None,
+                 half_steps: bool = False):
         """host_tables=True builds an FP32-table problem's ids with numpy
         (tables.build_tables, needs per-cell material arrays) instead of on the
         device (fdtd_ctx_build_material).  dft_accumulator "kahan-f32" keeps an
@@ -38,7 +39,9 @@ class Engine:
         > 0 accumulates the surface DFT once per that many steps (FP32).
         x_wall: None keeps the precision's default (FP64: the reference's reads
         past Hz/Hy at i = nx; FP32: Ey, Ez at i = nx held at zero), True / False
-        forces the wall / the reference's reads (fdtd_ctx_set_x_wall)."""
+        forces the wall / the reference's reads (fdtd_ctx_set_x_wall).
+        half_steps=True runs the half-step kernels also where the one-pass step
+        serves (fdtd_ctx_set_step_path)."""
         if dft_accumulator not in ("f64", "kahan-f32"):
             raise ValueError("dft_accumulator must be 'f64' or 'kahan-f32'")
         if precision not in PRECISIONS:
@@ -61,6 +64,8 @@ class Engine:
                 N.check(L.fdtd_ctx_set_dft_block(h, int(dft_block)))
             if x_wall is not None:
                 N.check(L.fdtd_ctx_set_x_wall(h, int(bool(x_wall))))
+            if half_steps:
+                self.half_steps = True
         except Exception:
             self.close()
             raise
@@ -139,6 +144,16 @@ class Engine:
     @x_wall.setter
     def x_wall(self, wall: bool) -> None:
         N.check(N.lib().fdtd_ctx_set_x_wall(self._h, int(bool(wall))))
+
+    @property
+    def half_steps(self) -> bool:
+        w = C.c_int()
+        N.check(N.lib().fdtd_ctx_get_step_path(self._h, C.byref(w)))
+        return bool(w.value)
+
+    @half_steps.setter
+    def half_steps(self, half: bool) -> None:
+        N.check(N.lib().fdtd_ctx_set_step_path(self._h, int(bool(half))))
 
     def material(self, comp: str) -> tuple[np.ndarray, np.ndarray]:
         """(ids, FP64 table rows x 3) of a table problem's component."""
@@ -262,11 +277,12 @@ class Engine:
 
 class Batch:
     """Engines of one precision on one device advanced together
-    (fdtd_batch_* in include/fdtd_b200.h).  streams = 0: each engine's one-pass
-    steps as a chain of their own, side by side; where an engine cannot run
-    them, or the DFT blocks differ in length, every step is four launches for the whole batch over a tile list, or, with per_launch = P > 0,
+    (fdtd_batch_* in include/fdtd_b200.h).  By default each engine's one-pass
+    steps are a chain of their own, side by side.  Where an engine cannot run
+    them, the DFT blocks differ in length, or a tile group is set, every step is
+    four launches for the whole batch over a tile list; with per_launch = P > 0,
     H and E launches that each carry P members' parameter blocks as their
-    kernel parameter (grouped mode); streams = S > 0: each member's own step
+    kernel parameter (grouped mode).  streams = S > 0: each member's own step
     kernels on S worker streams in one graph.  The engines stay usable for
     readback and must outlive the batch."""
 

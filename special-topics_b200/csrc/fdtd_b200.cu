@@ -167,6 +167,7 @@ struct fdtd_ctx {
   int acc_kahan = 0;          // FP32 problems: compensated FP32 accumulator pairs instead of FP64
   int dft_block = 0;          // FP32 problems: steps per time block of the surface DFT (0: every step)
   int x_wall = 0;             // 1: Ey, Ez at i = nx stay zero (see fdtd_ctx_set_x_wall)
+  bool half_steps = false;    // see fdtd_ctx_set_step_path
   float* dft_samples = nullptr;
   int* d_dft_done = nullptr;
   long long ffsz[3] = {};
@@ -936,6 +937,7 @@ int fused_build(fdtd_ctx* c) {
 int fused_usable(fdtd_ctx* c, bool* use) {
   FusedState& fs = c->fs;
   *use = false;
+  if (c->half_steps) return FDTD_OK;
   if (c->wanted) return fused_drop(c);  // this run takes the half-step path, a later one builds again
   if (!fs.tried) {
     int rc = fused_build(c);
@@ -2347,6 +2349,24 @@ int fdtd_ctx_set_x_wall(fdtd_ctx* c, int wall) {
   return FDTD_OK;
 }
 
+int fdtd_ctx_set_step_path(fdtd_ctx* c, int path) {
+  if (!c) return fail(FDTD_ERR_BADARG, "NULL handle");
+  Using use(c->mu);
+  if (path != 0 && path != 1) return fail(FDTD_ERR_BADARG, "step path %d not in {0,1}", path);
+  CK(cudaSetDevice(c->device));
+  if (path == 1)
+    if (int rc = fused_drop(c)) return rc;
+  c->half_steps = path == 1;
+  invalidate(c);
+  return FDTD_OK;
+}
+
+int fdtd_ctx_get_step_path(const fdtd_ctx* c, int* path) {
+  if (!c || !path) return fail(FDTD_ERR_BADARG, "NULL argument");
+  *path = c->half_steps;
+  return FDTD_OK;
+}
+
 int fdtd_ctx_get_x_wall(const fdtd_ctx* c, int* wall) {
   if (!c || !wall) return fail(FDTD_ERR_BADARG, "NULL argument");
   *wall = c->x_wall;
@@ -3016,11 +3036,13 @@ int batch_chain_enqueue(fdtd_batch* b, int at, int count) {
   return rc;
 }
 
-// Whether every member can run the one-pass step (their DFT blocks closing
-// together); then makes them hold the current state in that form.
+// Whether no other mode was chosen and every member can run the one-pass step
+// (their DFT blocks closing together); then makes them hold the current state in
+// that form.
 int batch_chain_ready(fdtd_batch* b, bool* use) {
-  *use = b->streams == 0;
-  for (const fdtd_ctx* c : b->m) *use = *use && c->dft_block == b->m[0]->dft_block && (c->fs.ok || !c->fs.tried);
+  *use = b->streams == 0 && b->group == 0 && b->members_per_launch == 0;
+  for (const fdtd_ctx* c : b->m)
+    *use = *use && !c->half_steps && c->dft_block == b->m[0]->dft_block && (c->fs.ok || !c->fs.tried);
   std::vector<fdtd_ctx*> built;
   for (size_t q = 0; q < b->m.size() && *use; q++) {
     const bool had = b->m[q]->fs.ok;
