@@ -679,49 +679,61 @@ int fused_alloc(fdtd_ctx* c, void** p, size_t bytes) {
   return FDTD_OK;
 }
 
-// Every field and present Psi slot between the dense arrays and copy `cur`.
+// Field q between its dense array and copy `cur`.
 template <typename T>
-int fused_copy(fdtd_ctx* c, int to_pad) {
+int fused_copy_field(fdtd_ctx* c, int q, int to_pad) {
+  const int nx = c->nx, ny = c->ny, nz = c->nz;
+  const int ni = (q == 1 || q == 2 || q == 3) ? nx : nx + 1, nj = (q == 0 || q == 2 || q == 4) ? ny : ny + 1,
+            nk = (q == 0 || q == 1 || q == 5) ? nz : nz + 1;
+  CK(fused_repack<T>((T*)c->fs.f[c->fs.cur][q], fused_plane(c), fused_pitch(c), (T*)field_ptr(c, q), ni, nj, nk, to_pad,
+                     c->stream));
+  return FDTD_OK;
+}
+
+// Psi slot s of face f.
+template <typename T>
+int fused_copy_psi(fdtd_ctx* c, int f, int s, int to_pad) {
   FusedState& fs = c->fs;
+  const HostFace& h = c->face[f];
   const int nx = c->nx, ny = c->ny, nz = c->nz, P = fused_pitch(c);
   const long long S = fused_plane(c);
-  for (int q = 0; q < 6; q++) {
-    const int ni = (q == 1 || q == 2 || q == 3) ? nx : nx + 1, nj = (q == 0 || q == 2 || q == 4) ? ny : ny + 1,
-              nk = (q == 0 || q == 1 || q == 5) ? nz : nz + 1;
-    CK(fused_repack<T>((T*)fs.f[fs.cur][q], S, P, (T*)field_ptr(c, q), ni, nj, nk, to_pad, c->stream));
+  const int ax = f / 2, el = s >= 2, nb = fs.layout.row.n[ax];
+  const int c0 = ax == 2 ? (f % 2 ? fs.layout.zw[el][0] : 0) + (el ? h.e_start : h.m_start) - fs.layout.z0[el][f % 2]
+                         : (f % 2 ? c->face[2 * ax].nc : 0);
+  T* pad = (T*)(s < 2 ? fs.ph[ax][fs.cur][s] : fs.pe[ax][s - 2]);
+  // extents of the slot's component, the band along the face axis (cpml.js:147-448)
+  const bool first = s == 0 || s == 3;
+  int n[3] = {nx, ny, nz};
+  if (f / 2 == 0) n[first ? 1 : 2]++;
+  if (f / 2 == 1) n[s % 2 == 0 ? 0 : 2]++;
+  if (f / 2 == 2) n[first ? 0 : 1]++;
+  n[f / 2] = h.nc;
+  long long si, sj;
+  if (ax == 0) {
+    si = S;
+    sj = P;
+    pad += c0 * S;
+  } else if (ax == 1) {
+    si = (long long)nb * P;
+    sj = P;
+    pad += (long long)c0 * P;
+  } else {
+    si = (long long)(ny + 1) * nb;
+    sj = nb;
+    pad += c0;
   }
-  for (int f = 0; f < 6; f++) {
-    const HostFace& h = c->face[f];
-    if (!h.present) continue;
-    for (int s = 0; s < 4; s++) {
-      const int ax = f / 2, el = s >= 2, nb = fs.layout.row.n[ax];
-      const int c0 = ax == 2 ? (f % 2 ? fs.layout.zw[el][0] : 0) + (el ? h.e_start : h.m_start) - fs.layout.z0[el][f % 2]
-                             : (f % 2 ? c->face[2 * ax].nc : 0);
-      T* pad = (T*)(s < 2 ? fs.ph[ax][fs.cur][s] : fs.pe[ax][s - 2]);
-      // extents of the slot's component, the band along the face axis (cpml.js:147-448)
-      const bool first = s == 0 || s == 3;
-      int n[3] = {nx, ny, nz};
-      if (f / 2 == 0) n[first ? 1 : 2]++;
-      if (f / 2 == 1) n[s % 2 == 0 ? 0 : 2]++;
-      if (f / 2 == 2) n[first ? 0 : 1]++;
-      n[f / 2] = h.nc;
-      long long si, sj;
-      if (ax == 0) {
-        si = S;
-        sj = P;
-        pad += c0 * S;
-      } else if (ax == 1) {
-        si = (long long)nb * P;
-        sj = P;
-        pad += (long long)c0 * P;
-      } else {
-        si = (long long)(ny + 1) * nb;
-        sj = nb;
-        pad += c0;
-      }
-      CK(fused_repack<T>(pad, si, sj, (T*)h.psi[s], n[0], n[1], n[2], to_pad, c->stream));
-    }
-  }
+  CK(fused_repack<T>(pad, si, sj, (T*)h.psi[s], n[0], n[1], n[2], to_pad, c->stream));
+  return FDTD_OK;
+}
+
+// Every field and present Psi slot.
+template <typename T>
+int fused_copy(fdtd_ctx* c, int to_pad) {
+  for (int q = 0; q < 6; q++)
+    if (int rc = fused_copy_field<T>(c, q, to_pad)) return rc;
+  for (int f = 0; f < 6; f++)
+    for (int s = 0; s < 4 && c->face[f].present; s++)
+      if (int rc = fused_copy_psi<T>(c, f, s, to_pad)) return rc;
   return FDTD_OK;
 }
 
@@ -2157,7 +2169,8 @@ int fdtd_ctx_read_field(fdtd_ctx* c, int which, double* host, long n) {
   if (n != c->ncomp[which]) return fail(FDTD_ERR_BADARG, "field %d: buffer of %ld, need %lld", which, n, c->ncomp[which]);
   CK(cudaSetDevice(c->device));
   Using use(c->mu);
-  if (int rc = to_dense(c)) return rc;
+  if (!c->dense_valid)  // this array alone
+    if (int rc = c->esz == 8 ? fused_copy_field<double>(c, which, 0) : fused_copy_field<float>(c, which, 0)) return rc;
   return read_real(c, field_ptr(c, which), host, n);
 }
 
@@ -2167,7 +2180,8 @@ int fdtd_ctx_read_psi(fdtd_ctx* c, int f, int slot, double* host, long n) {
   if (n != c->face[f].n[slot]) return fail(FDTD_ERR_BADARG, "Psi buffer of %ld, need %lld", n, c->face[f].n[slot]);
   CK(cudaSetDevice(c->device));
   Using use(c->mu);
-  if (int rc = to_dense(c)) return rc;
+  if (!c->dense_valid)
+    if (int rc = c->esz == 8 ? fused_copy_psi<double>(c, f, slot, 0) : fused_copy_psi<float>(c, f, slot, 0)) return rc;
   return read_real(c, c->face[f].psi[slot], host, n);
 }
 
