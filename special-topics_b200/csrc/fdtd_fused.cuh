@@ -451,7 +451,7 @@ __device__ __forceinline__ void fused_e(const FusedParams<T>& p, const FusedCell
     const Row<T> x = c.x(q);
     ex.v[q] = A::lin3(x.c0, ex.v[q], x.c1, dhz_y.v[q], c.z0(q), dhy_z.v[q]);
   }
-  const bool wall_j = t.j == 0 || t.j == p.ny;
+  const bool wall_j = (unsigned)(t.j - 1) >= (unsigned)(p.ny - 1);
   fused_hold<true>(t.k, p.nz, wall_j, oex, ex);
   if (yz) {
     T cx0 = T(0), cx1 = T(0);
