@@ -11,6 +11,7 @@
 #include <cstdarg>
 #include <cstddef>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <functional>
 #include <initializer_list>
@@ -112,6 +113,7 @@ struct RunGraphs {
 // first run that can use it, dropped when the set-up changes.
 struct FusedState {
   bool tried = false, ok = false;  // built (or found unusable) for the present set-up
+  int no_room_at = -1;             // unusable for want of memory alone, found at this step
   bool valid = false;              // holds the current fields and Psi, in copy `cur`
   int cur = 0;
   int ts_at = -1;                  // step index in d_ts[cur]
@@ -665,14 +667,18 @@ int fused_pitch(const fdtd_ctx* c) {
 }
 long long fused_plane(const fdtd_ctx* c) { return (long long)(c->ny + 1) * fused_pitch(c); }
 
+// Memory for the padded state: no other handle's is taken for it.
+int fused_malloc(fdtd_ctx* c, void** p, size_t bytes) {
+  if (cudaMalloc(p, bytes) == cudaSuccess) return FDTD_OK;
+  cudaGetLastError();  // no room: the caller takes the half-step path
+  *p = nullptr;
+  c->fs.no_room_at = c->ts;
+  return FDTD_ERR_OOM;
+}
+
 // One zeroed allocation of the padded state.
 int fused_alloc(fdtd_ctx* c, void** p, size_t bytes) {
-  const cudaError_t e = cudaMalloc(p, bytes);
-  if (e != cudaSuccess) {
-    cudaGetLastError();  // no room: the caller takes the half-step path
-    *p = nullptr;
-    return FDTD_ERR_OOM;
-  }
+  if (int rc = fused_malloc(c, p, bytes)) return rc;
   c->fs.owned.push_back(*p);
   c->padded = true;
   CK(cudaMemsetAsync(*p, 0, bytes, c->stream));
@@ -816,10 +822,7 @@ int fused_classes(fdtd_ctx* c, const C& coef, bool* ok) {
   ClassTable tb{};
   void* scratch = nullptr;
   const size_t kb = kClassSlots * sizeof(unsigned long long), ib = kClassSlots * sizeof(unsigned);
-  if (cudaMalloc(&scratch, kb + ib + 16) != cudaSuccess) {
-    cudaGetLastError();
-    return FDTD_OK;  // no room: not usable
-  }
+  if (fused_malloc(c, &scratch, kb + ib + 16)) return FDTD_OK;  // not usable
   tb.key = (unsigned long long*)scratch;
   tb.id = (unsigned*)((char*)scratch + kb);
   tb.count = (int*)(tb.id + kClassSlots);
@@ -902,7 +905,10 @@ int fused_build(fdtd_ctx* c) {
   }
   size_t free_b = 0, total_b = 0;
   CK(cudaMemGetInfo(&free_b, &total_b));
-  if (need > free_b / 2) return FDTD_OK;
+  if (need > free_b / 2) {
+    fs.no_room_at = c->ts;
+    return FDTD_OK;
+  }
   Arena ar;
   for (int w = 0; w < 2; w++)
     for (int q = 0; q < 6; q++) ar.add(&fs.f[w][q], comp);
@@ -945,16 +951,26 @@ int fused_build(fdtd_ctx* c) {
   return rc;
 }
 
+// A padded state that was refused for want of memory is tried again after so many
+// steps: memory may be free by then, and a question costs little over them.
+constexpr int kRetrySteps = 512;
+bool fused_retry(const fdtd_ctx* c) {
+  return c->fs.tried && !c->fs.ok && c->fs.no_room_at >= 0 && std::abs(c->ts - c->fs.no_room_at) >= kRetrySteps;
+}
+
 // Builds the padded state where there is none; *use = false: half-step path.
 int fused_usable(fdtd_ctx* c, bool* use) {
   FusedState& fs = c->fs;
   *use = false;
   if (c->half_steps) return FDTD_OK;
+  if (fused_retry(c)) fs = FusedState();
   if (c->wanted) return fused_drop(c);  // this run takes the half-step path, a later one builds again
   if (!fs.tried) {
     int rc = fused_build(c);
     if (rc || !fs.ok) {
+      const int no_room_at = fs.no_room_at;
       fused_free(c);
+      fs.no_room_at = no_room_at;
       fs.tried = rc == FDTD_OK;
       if (rc) return rc;
     } else {
@@ -3056,13 +3072,14 @@ int batch_chain_enqueue(fdtd_batch* b, int at, int count) {
 int batch_chain_ready(fdtd_batch* b, bool* use) {
   *use = b->streams == 0 && b->group == 0 && b->members_per_launch == 0;
   for (const fdtd_ctx* c : b->m)
-    *use = *use && !c->half_steps && c->dft_block == b->m[0]->dft_block && (c->fs.ok || !c->fs.tried);
-  std::vector<fdtd_ctx*> built;
-  for (size_t q = 0; q < b->m.size() && *use; q++) {
-    const bool had = b->m[q]->fs.ok;
-    int rc = fused_usable(b->m[q], use);
+    *use = *use && !c->half_steps && c->dft_block == b->m[0]->dft_block && (c->fs.ok || !c->fs.tried || fused_retry(c));
+  std::vector<fdtd_ctx*> order = b->m, built;  // those refused before first: they may be again
+  std::stable_partition(order.begin(), order.end(), fused_retry);
+  for (size_t q = 0; q < order.size() && *use; q++) {
+    const bool had = order[q]->fs.ok;
+    int rc = fused_usable(order[q], use);
     if (rc) return rc;
-    if (!had && *use) built.push_back(b->m[q]);
+    if (!had && *use) built.push_back(order[q]);
   }
   if (!*use)  // built in vain
     for (fdtd_ctx* c : built)
