@@ -218,6 +218,9 @@ __device__ __forceinline__ constexpr bool in_band(double) { return true; }
 // Programmatic launches: waits for the launch before this one (at once where
 // this is an ordinary launch), and lets the one after it start its blocks.
 __device__ __forceinline__ void launch_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Orders what this thread sees of global memory ahead of its tensor copies, which
+// read it by another path (the launch before wrote it with ordinary stores).
+__device__ __forceinline__ void fence_proxy_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 __device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // One (k, j, i) tile from the padded array of `map` into shared memory,
@@ -451,7 +454,9 @@ __device__ __forceinline__ void fused_e(const FusedParams<T>& p, const FusedCell
     const Row<T> x = c.x(q);
     ex.v[q] = A::lin3(x.c0, ex.v[q], x.c1, dhz_y.v[q], c.z0(q), dhy_z.v[q]);
   }
-  const bool wall_j = (unsigned)(t.j - 1) >= (unsigned)(p.ny - 1);
+  // the row of a wall: as one compare it makes the table kernel spill 8 bytes, as two
+  // it costs FP64 0.7% of a step (256^3: 555 us for 551)
+  const bool wall_j = V > 1 ? t.j == 0 || t.j == p.ny : (unsigned)(t.j - 1) >= (unsigned)(p.ny - 1);
   fused_hold<true>(t.k, p.nz, wall_j, oex, ex);
   if (yz) {
     T cx0 = T(0), cx1 = T(0);
@@ -562,7 +567,7 @@ __device__ __forceinline__ void fused_tile(const FusedParams<T>& p, int bx, int 
   launch_next();
   if (tid == 0) {
     if (bx + by + bz == 0) *p.ts_next = *p.ts + 1;
-    fence_proxy_async();
+    fence_proxy_global();
     for (int m = 0; m <= min(NS - 1, last); m++) issue(m);
   }
   // H where the grid has none is read into differences that nothing uses
@@ -842,7 +847,14 @@ __global__ void __launch_bounds__(256)
                      const __grid_constant__ Probes pr, int late) {
   if (!late) launch_wait();
   launch_next();
-  if (late) __threadfence();  // nothing older than the step's start is read
+  // `late`: this launch starts when every block of the running step has passed its
+  // launch_next, which stands after its launch_wait.  So the launch before that step
+  // had ended, and it had waited, at its own end at the latest, for the step whose
+  // copy is read here: that copy was written and flushed before any block of this
+  // launch was there to read it, and its next writer is queued behind this launch.
+  // No block has read the copy before it was written, but a multiprocessor's cache
+  // may hold lines of an earlier epilogue's: the fence drops them.
+  if (late) __threadfence();
   const T* f[6];
 #pragma unroll
   for (int c = 0; c < 6; c++) f[c] = late ? p.fi[c] : p.fo[c];
