@@ -148,12 +148,12 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(sm)}
 
 
-def ncu_traffic(workload: str):
-    """dram bytes per launch of the dominant kernel from the committed ncu summary, if any."""
+def ncu_traffic(workload: str, kernel: str):
+    """dram bytes per launch of `kernel` from the committed ncu summary, if it has any."""
     path = os.path.join(ROOT, "profiles", f"traffic_{workload}.txt")
     try:
         for line in open(path):
-            if line.startswith("traffic_bytes_per_launch:"):
+            if line.startswith(f"traffic_bytes_per_launch {kernel}:"):
                 return float(line.split(":")[1])
     except OSError:
         pass
@@ -385,7 +385,7 @@ def main():
     dom, dom_bytes, dom_ms = dominant(kern, byts)
     peak, peak_kind = hbm_peak()
     achieved = dom_bytes / (dom_ms / 1e3) / 1e9
-    traffic = ncu_traffic(workload)
+    traffic = ncu_traffic(workload, dom)
     line = {
         "metric": METRIC, "value": value, "unit": "Gcell-updates/s", "n_gpus": world, "steps": K, "warmup": W,
         "ms_per_step": ms / K, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
