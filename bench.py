@@ -82,6 +82,13 @@ def one_pass(kern: dict) -> bool:
     return kern["e"] == 0.0
 
 
+def shape_ran(kern: dict, tiling: dict | None, keys=("chunk", "rows", "prefetch", "width")):
+    """The launch shape of a profiled leg: the one-pass step picks its own."""
+    if one_pass(kern):
+        return "the one-pass step's own"
+    return {k: tiling.get(k, 32 if k == "width" else None) for k in keys} if tiling else "default"
+
+
 def dominant(kern: dict, byts: dict) -> tuple:
     """(name, algorithmic bytes, ms) of the step's longest launch."""
     if one_pass(kern):
@@ -402,9 +409,7 @@ def main():
                      "algorithmic_bytes_per_launch": dom_bytes, "launch_ms": dom_ms,
                      "traffic": traffic},
         "kernel_ms": kern,
-        "tiling": "the one-pass step's own" if one_pass(kern) else
-                  {k: tuning.get(k, 32 if k == "width" else None) for k in ("chunk", "rows", "prefetch", "width", "ms_per_step")}
-                  if tuning else "default",
+        "tiling": shape_ran(kern, tuning, ("chunk", "rows", "prefetch", "width", "ms_per_step")),
         "clocks": clk.summary(),
         # H, mid, E, epilogue (+ the DFT flush); one-pass: the step, its epilogue, the wall where the reference's
         # reads are kept, and a flush per block
@@ -442,7 +447,8 @@ def main():
             t64 = None
             if not args.no_fp64:
                 line["fp64_plain"] = fp64_side(pkg)
-                t64 = line["fp64_plain"]["tiling"]
+                if isinstance(line["fp64_plain"]["tiling"], dict):
+                    t64 = line["fp64_plain"]["tiling"]
             line["scaling_sweep"] = scaling_sweep_side(tuning, t64, device=local, dft_block=dft_block)
         except Exception as e:
             line["scaling_sweep"] = {"error": str(e)}
@@ -735,7 +741,7 @@ def scaling_sweep_side(tiling32: dict | None, tiling64: dict | None, device: int
             work = algorithmic_bytes(p, prec)
             leg.update({"grid": list(n), "cells": cells,
                         "l2_resident": bool(work["e"] < L2_BYTES),
-                        "tiling": {k: tiling.get(k) for k in ("chunk", "rows", "prefetch", "width")} if tiling else "default"})
+                        "tiling": shape_ran(leg["kernel_ms"], tiling)})
             out.append(leg)
         del p
     return out
@@ -813,7 +819,7 @@ def fp64_side(pkg, n=(256, 256, 256), K: int = 300, W: int = 8) -> dict:
     ach = dom_bytes / (dom_ms / 1e3) / 1e9
     return {"workload": f"scaling-box-{n[0]}x{n[1]}x{n[2]}", "value": p.grid.cells * K / (ms / 1e3) / 1e9,
             "unit": "Gcell-updates/s", "ms_per_step": ms / K,
-            "tiling": "the one-pass step's own" if one_pass(kern) else {k: tuning[k] for k in ("chunk", "rows", "prefetch")},
+            "tiling": shape_ran(kern, tuning, ("chunk", "rows", "prefetch")),
             "roofline": {"kernel": dom, "achieved": ach, "peak": peak, "frac": ach / peak}}
 
 
